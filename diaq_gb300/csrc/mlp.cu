@@ -4,8 +4,9 @@
 // (src/spME.cpp:256-262) and m by a Frobenius stop test.
 //
 // Parameters live in one flat float buffer: W1[16][64] b1[64] W2[64][64] b2[64] W3[64][51] b3[51]
-// (W[i][j] maps input i to output j).  Every reduction over the batch runs in a fixed order in one
-// thread, so gradients are deterministic.
+// (W[i][j] maps input i to output j).  Every reduction over the batch runs in an order fixed by the
+// batch size, so gradients are deterministic.
+#include <algorithm>
 #include <cmath>
 #include <random>
 #include <vector>
@@ -19,8 +20,8 @@ constexpr int oW1 = 0, oB1 = oW1 + kIn * kH1, oW2 = oB1 + kH1, oB2 = oW2 + kH1 *
               oB3 = oW3 + kH2 * kOut, kParams = oB3 + kOut;
 
 struct Mlp {
-    float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;  // params, grads, Adam moments
-    float *work = nullptr;                                          // activations for `cap` rows
+    float *p = nullptr, *m = nullptr, *v = nullptr;  // params, Adam moments
+    float *work = nullptr;                           // weight gradients of `cap` blocks' rows
     int cap = 0;
     int64_t t = 0;  // Adam step
     ~Mlp() {
@@ -29,152 +30,264 @@ struct Mlp {
     }
 };
 
-// out[b][j] = act(sum_i in[b][i] W[i][j] + bias[j]); also keeps the pre-activation z.
-__global__ void dense_fwd(const float *__restrict__ in, int B, int din, const float *__restrict__ W,
-                          const float *__restrict__ bias, int dout, int relu, float *__restrict__ z,
-                          float *__restrict__ out) {
-    const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)B * dout) return;
-    const int b = (int)(idx / dout), j = (int)(idx % dout);
-    float s = bias[j];
-    for (int i = 0; i < din; ++i) s = fmaf(in[(int64_t)b * din + i], W[i * dout + j], s);
-    if (z) z[idx] = s;
-    out[idx] = relu ? fmaxf(s, 0.f) : s;
+// One pass over the batch.  The network is small (8,563 parameters, 34 KB) and a row's forward and
+// backward pass touches nothing but the weights, so a block keeps the weights in shared memory and
+// takes kRows rows at a time through the forward pass, the softmax, the backward pass and the
+// products that make up the weight gradient; every activation stays in shared memory.  The weight
+// gradient of the block's rows is held in registers (37 values per thread: a 4 x 4 tile of W2, one
+// of W3, a strip of W1, a bias) and written once per block; mlp_reduce_kernel then sums the blocks'
+// parts.  The sum over the batch is split over up to 2 blocks per SM this way: one thread per weight
+// walking the whole batch left a chain of B dependent loads on 34 blocks: a training step of 1,024
+// rows took 544 us that way (450 of them in those launches) and takes 26 us now.  What bounds it now
+// is latency: two dependent launches with one round of 8 rows per block.
+constexpr int kRows = 8;                       // rows per block and round: one per warp in the softmax
+constexpr int kMlpThreads = 256;
+constexpr int kLd2 = kH2 + 1;                  // W2 rows padded: read along both indices, conflict-free
+constexpr int kOutPad = 52;                    // logits rows padded to whole float4s
+
+struct MlpShared {  // 45 KB
+    float w1[kIn * kH1], b1[kH1], w2[kH1 * kLd2], b2[kH2], w3[kH2 * kOut], b3[kOut];
+    alignas(16) float x[kRows][kIn], a1[kRows][kH1], a2[kRows][kH2], lg[kRows][kOutPad], d2[kRows][kH2], d1[kRows][kH1];
+};
+
+__device__ __forceinline__ void mlp_load_weights(MlpShared &S, const float *__restrict__ p) {
+    const int t = threadIdx.x;
+    for (int i = t; i < kIn * kH1; i += kMlpThreads) S.w1[i] = p[oW1 + i];
+    for (int i = t; i < kH1 * kH2; i += kMlpThreads) S.w2[(i / kH2) * kLd2 + i % kH2] = p[oW2 + i];
+    for (int i = t; i < kH2 * kOut; i += kMlpThreads) S.w3[i] = p[oW3 + i];
+    if (t < kH1) S.b1[t] = p[oB1 + t];
+    if (t < kH2) S.b2[t] = p[oB2 + t];
+    if (t < kOut) S.b3[t] = p[oB3 + t];
 }
 
-// Per row: loss = CE(softmax(logits[0:21]), s) + CE(softmax(logits[21:51]), m-1); dlogits =
-// (softmax - onehot) / B.  Labels outside range give loss 0 and no gradient for that head.
-__global__ void softmax_ce(const float *__restrict__ logits, const int32_t *__restrict__ ys,
-                           const int32_t *__restrict__ ym, int B, float *__restrict__ dlog,
-                           float *__restrict__ loss) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const float *l = logits + (int64_t)b * kOut;
-    float *d = dlog + (int64_t)b * kOut;
-    float total = 0.f;
-    for (int head = 0; head < 2; ++head) {
-        const int o0 = head == 0 ? 0 : kOutS, n = head == 0 ? kOutS : kOutM;
-        const int lab = head == 0 ? ys[b] : ym[b] - 1;
-        float mx = l[o0];
-        for (int j = 1; j < n; ++j) mx = fmaxf(mx, l[o0 + j]);
-        float se = 0.f;
-        for (int j = 0; j < n; ++j) se += expf(l[o0 + j] - mx);
-        const bool ok = lab >= 0 && lab < n;
-        for (int j = 0; j < n; ++j) {
-            const float pj = expf(l[o0 + j] - mx) / se;
-            d[o0 + j] = ok ? (pj - (j == lab ? 1.f : 0.f)) / (float)B : 0.f;
+// Logits of rows row0 .. row0 + kRows - 1 into S.lg (rows past B read as zeros).  Thread t works on
+// unit t % 64 of rows t / 64 and t / 64 + 4; each unit's sum runs over its inputs in order.
+__device__ __forceinline__ void mlp_forward_rows(MlpShared &S, const float *__restrict__ X, int64_t row0, int B) {
+    const int t = threadIdx.x, j = t & 63, q = t >> 6;
+    if (t < kRows * kIn) {
+        const int64_t b = row0 + t / kIn;
+        S.x[t / kIn][t % kIn] = b < B ? X[row0 * kIn + t] : 0.f;
+    }
+    __syncthreads();
+    float s0 = S.b1[j], s1 = s0;
+#pragma unroll
+    for (int i = 0; i < kIn; ++i) {
+        const float w = S.w1[i * kH1 + j];
+        s0 = fmaf(S.x[q][i], w, s0);
+        s1 = fmaf(S.x[q + 4][i], w, s1);
+    }
+    S.a1[q][j] = fmaxf(s0, 0.f);
+    S.a1[q + 4][j] = fmaxf(s1, 0.f);
+    __syncthreads();
+    s0 = s1 = S.b2[j];
+#pragma unroll 16
+    for (int i = 0; i < kH1; ++i) {
+        const float w = S.w2[i * kLd2 + j];
+        s0 = fmaf(S.a1[q][i], w, s0);
+        s1 = fmaf(S.a1[q + 4][i], w, s1);
+    }
+    S.a2[q][j] = fmaxf(s0, 0.f);
+    S.a2[q + 4][j] = fmaxf(s1, 0.f);
+    __syncthreads();
+    if (j < kOut) {
+        s0 = s1 = S.b3[j];
+#pragma unroll 16
+        for (int i = 0; i < kH2; ++i) {
+            const float w = S.w3[i * kOut + j];
+            s0 = fmaf(S.a2[q][i], w, s0);
+            s1 = fmaf(S.a2[q + 4][i], w, s1);
         }
-        if (ok) total += -(l[o0 + lab] - mx - logf(se));
+        S.lg[q][j] = s0;
+        S.lg[q + 4][j] = s1;
+    } else if (j == kOut) {
+        S.lg[q][j] = S.lg[q + 4][j] = 0.f;
     }
-    loss[b] = total;
+    __syncthreads();
 }
 
-// dW[i][j] = sum_b in[b][i] dout[b][j]; db[j] = sum_b dout[b][j] (thread per weight, batch in order).
-__global__ void dense_bwd_w(const float *__restrict__ in, const float *__restrict__ dout, int B, int din, int dn,
-                            float *__restrict__ dW, float *__restrict__ db) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < din * dn) {
-        const int i = idx / dn, j = idx % dn;
-        float s = 0.f;
-        for (int b = 0; b < B; ++b) s = fmaf(in[(int64_t)b * din + i], dout[(int64_t)b * dn + j], s);
-        dW[idx] = s;
-    } else if (idx < din * dn + dn) {
-        const int j = idx - din * dn;
-        float s = 0.f;
-        for (int b = 0; b < B; ++b) s += dout[(int64_t)b * dn + j];
-        db[j] = s;
+// Logits[B][51], or the argmax of each head (s_out, m_out), for every row.
+__global__ void __launch_bounds__(kMlpThreads)
+    mlp_forward_kernel(const float *__restrict__ p, const float *__restrict__ X, int B, float *__restrict__ logits,
+                       int32_t *__restrict__ s_out, int32_t *__restrict__ m_out) {
+    __shared__ MlpShared S;
+    mlp_load_weights(S, p);
+    for (int64_t row0 = (int64_t)blockIdx.x * kRows; row0 < B; row0 += (int64_t)gridDim.x * kRows) {
+        __syncthreads();
+        mlp_forward_rows(S, X, row0, B);
+        const int n = (int)min((int64_t)kRows, B - row0);
+        if (logits)
+            for (int i = threadIdx.x; i < n * kOut; i += kMlpThreads)
+                logits[row0 * kOut + i] = S.lg[i / kOut][i % kOut];
+        if (s_out && threadIdx.x < n) {
+            const float *l = S.lg[threadIdx.x];
+            int bs = 0, bm = 0;
+            for (int j = 1; j < kOutS; ++j)
+                if (l[j] > l[bs]) bs = j;
+            for (int j = 1; j < kOutM; ++j)
+                if (l[kOutS + j] > l[kOutS + bm]) bm = j;
+            s_out[row0 + threadIdx.x] = bs;
+            m_out[row0 + threadIdx.x] = bm + 1;
+        }
     }
 }
 
-// dIn[b][i] = (sum_j dout[b][j] W[i][j]) * (z[b][i] > 0)
-__global__ void dense_bwd_x(const float *__restrict__ dout, const float *__restrict__ W, const float *__restrict__ z,
-                            int B, int din, int dn, float *__restrict__ dIn) {
-    const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)B * din) return;
-    const int b = (int)(idx / din), i = (int)(idx % din);
+// One head of one row, a lane per logit: CE(softmax(l), lab) to every lane, and l replaced by
+// (softmax - onehot) / B.  A label outside the head gives loss 0 and no gradient.
+__device__ __forceinline__ float softmax_ce_head(float *l, int n, int lab, int lane, float B) {
+    const float v = lane < n ? l[lane] : 0.f;
+    float mx = lane < n ? v : -INFINITY;
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float e = lane < n ? expf(v - mx) : 0.f;
+    float se = e;
+    for (int o = 16; o > 0; o >>= 1) se += __shfl_xor_sync(0xffffffffu, se, o);
+    const bool ok = lab >= 0 && lab < n;
+    const float vl = __shfl_sync(0xffffffffu, v, ok ? lab : 0);
+    if (lane < n) l[lane] = ok ? (e / se - (lane == lab ? 1.f : 0.f)) / B : 0.f;
+    return ok ? -(vl - mx - logf(se)) : 0.f;
+}
+
+// acc[4][4] += u (4 values) x v (4 values)
+__device__ __forceinline__ void outer4(float (&acc)[4][4], const float4 &u, const float4 &v) {
+    const float a[4] = {u.x, u.y, u.z, u.w}, b[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+}
+
+// Per-row losses (loss may be NULL) and, per block, the gradient of the mean loss over the block's
+// rows: part[block][kParams].
+__global__ void __launch_bounds__(kMlpThreads)
+    mlp_grad_kernel(const float *__restrict__ p, const float *__restrict__ X, const int32_t *__restrict__ ys,
+                    const int32_t *__restrict__ ym, int B, float *__restrict__ loss, float *__restrict__ part) {
+    __shared__ MlpShared S;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    mlp_load_weights(S, p);
+    const int i4 = (t >> 4) * 4, j4 = (t & 15) * 4;       // tile of W2 (and of W3, j4 < 52); column strip of W1
+    float g1[4] = {0.f, 0.f, 0.f, 0.f}, g2[4][4], g3[4][4], gb = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) g2[i][j] = g3[i][j] = 0.f;
+    for (int64_t row0 = (int64_t)blockIdx.x * kRows; row0 < B; row0 += (int64_t)gridDim.x * kRows) {
+        __syncthreads();
+        mlp_forward_rows(S, X, row0, B);
+        const int64_t b = row0 + wid;
+        const bool live = b < B;
+        const float l = softmax_ce_head(S.lg[wid], kOutS, live ? ys[b] : -1, lane, (float)B) +
+                        softmax_ce_head(S.lg[wid] + kOutS, kOutM, live ? ym[b] - 1 : -1, lane, (float)B);
+        if (loss && live && lane == 0) loss[b] = l;
+        __syncthreads();
+        {   // dL/da2, dL/da1 (masked by the ReLUs): thread t on unit t % 64 of two rows
+            const int i = t & 63, q = t >> 6;
+            float s0 = 0.f, s1 = 0.f;
+#pragma unroll 17
+            for (int j = 0; j < kOut; ++j) {
+                const float w = S.w3[i * kOut + j];
+                s0 = fmaf(S.lg[q][j], w, s0);
+                s1 = fmaf(S.lg[q + 4][j], w, s1);
+            }
+            S.d2[q][i] = S.a2[q][i] > 0.f ? s0 : 0.f;
+            S.d2[q + 4][i] = S.a2[q + 4][i] > 0.f ? s1 : 0.f;
+            __syncthreads();
+            s0 = s1 = 0.f;
+#pragma unroll 16
+            for (int j = 0; j < kH2; ++j) {
+                const float w = S.w2[i * kLd2 + j];
+                s0 = fmaf(S.d2[q][j], w, s0);
+                s1 = fmaf(S.d2[q + 4][j], w, s1);
+            }
+            S.d1[q][i] = S.a1[q][i] > 0.f ? s0 : 0.f;
+            S.d1[q + 4][i] = S.a1[q + 4][i] > 0.f ? s1 : 0.f;
+            __syncthreads();
+        }
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const float4 d1 = *reinterpret_cast<const float4 *>(&S.d1[r][j4]);
+            const float x = S.x[r][i4 >> 2];
+            g1[0] = fmaf(x, d1.x, g1[0]);
+            g1[1] = fmaf(x, d1.y, g1[1]);
+            g1[2] = fmaf(x, d1.z, g1[2]);
+            g1[3] = fmaf(x, d1.w, g1[3]);
+            outer4(g2, *reinterpret_cast<const float4 *>(&S.a1[r][i4]), *reinterpret_cast<const float4 *>(&S.d2[r][j4]));
+            if (j4 < kOutPad)
+                outer4(g3, *reinterpret_cast<const float4 *>(&S.a2[r][i4]), *reinterpret_cast<const float4 *>(&S.lg[r][j4]));
+            gb += t < kH1 ? S.d1[r][t] : t < kH1 + kH2 ? S.d2[r][t - kH1] : t < kH1 + kH2 + kOut ? S.lg[r][t - kH1 - kH2] : 0.f;
+        }
+    }
+    float *o = part + (int64_t)blockIdx.x * kParams;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[oW1 + (i4 >> 2) * kH1 + j4 + j] = g1[j];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            o[oW2 + (i4 + i) * kH2 + j4 + j] = g2[i][j];
+            if (j4 + j < kOut) o[oW3 + (i4 + i) * kOut + j4 + j] = g3[i][j];
+        }
+    if (t < kH1) o[oB1 + t] = gb;
+    else if (t < kH1 + kH2) o[oB2 + t - kH1] = gb;
+    else if (t < kH1 + kH2 + kOut) o[oB3 + t - kH1 - kH2] = gb;
+}
+
+// Sums the blocks' parts per parameter in a fixed order (8 slices of the blocks, then the slices),
+// into g (may be NULL) and, with adam, straight into the Adam step of p, m, v.
+struct AdamStep {
+    float *p, *m, *v;
+    float lr, b1, b2, eps, bc1, bc2;
+};
+constexpr int kSlices = 8;
+__global__ void __launch_bounds__(32 * kSlices)
+    mlp_reduce_kernel(const float *__restrict__ part, int nblk, float *__restrict__ g, int adam, AdamStep A) {
+    __shared__ float red[kSlices][32];
+    const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int j = 0; j < dn; ++j) s = fmaf(dout[(int64_t)b * dn + j], W[i * dn + j], s);
-    dIn[idx] = z[idx] > 0.f ? s : 0.f;
+    if (i < kParams) {
+#pragma unroll 8
+        for (int b = sl; b < nblk; b += kSlices) s += part[(int64_t)b * kParams + i];
+    }
+    red[sl][lane] = s;
+    __syncthreads();
+    if (sl != 0 || i >= kParams) return;
+    float gi = red[0][lane];
+#pragma unroll
+    for (int k = 1; k < kSlices; ++k) gi += red[k][lane];
+    if (g) g[i] = gi;
+    if (!adam) return;
+    const float mi = A.b1 * A.m[i] + (1.f - A.b1) * gi;
+    const float vi = A.b2 * A.v[i] + (1.f - A.b2) * gi * gi;
+    A.m[i] = mi;
+    A.v[i] = vi;
+    A.p[i] -= A.lr * (mi / A.bc1) / (sqrtf(vi / A.bc2) + A.eps);
 }
 
-__global__ void adam_kernel(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                            float *__restrict__ v, int n, float lr, float b1, float b2, float eps, float bc1,
-                            float bc2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi;
-    const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-}
+// Blocks of a pass over B rows: at most two per SM (the shared memory would hold four).
+static int grad_blocks(int B) { return (int)std::min<int64_t>(((int64_t)B + kRows - 1) / kRows, 2 * num_sms()); }
 
-__global__ void argmax_heads(const float *__restrict__ logits, int B, int32_t *__restrict__ s_out,
-                             int32_t *__restrict__ m_out) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const float *l = logits + (int64_t)b * kOut;
-    int bs = 0, bm = 0;
-    for (int j = 1; j < kOutS; ++j)
-        if (l[j] > l[bs]) bs = j;
-    for (int j = 1; j < kOutM; ++j)
-        if (l[kOutS + j] > l[kOutS + bm]) bm = j;
-    s_out[b] = bs;
-    m_out[b] = bm + 1;
-}
-
-// Activations for B rows: z1 a1 (B x 64) z2 a2 (B x 64) logits dlog (B x 51) d2 d1 (B x 64) loss (B)
-static int ensure_work(Mlp &M, int B) {
-    if (B <= M.cap) return DIAQ_OK;
+static int ensure_work(Mlp &M, int nblk) {
+    if (nblk <= M.cap) return DIAQ_OK;
     if (M.work) cudaFree(M.work);
     M.work = nullptr;
     M.cap = 0;
-    const size_t per = 6 * kH1 + 2 * kOut + 1;
-    DQ_CUDA(dev_malloc(&M.work, sizeof(float) * per * (size_t)B));
-    M.cap = B;
+    DQ_CUDA(dev_malloc(&M.work, sizeof(float) * kParams * (size_t)nblk));
+    M.cap = nblk;
     return DIAQ_OK;
 }
 
-struct Acts {
-    float *z1, *a1, *z2, *a2, *lg, *dl, *d2, *d1, *loss;
-};
-static Acts acts(const Mlp &M) {
-    const int64_t B = M.cap;
-    float *w = M.work;
-    Acts a;
-    a.z1 = w;
-    a.a1 = w + B * kH1;
-    a.z2 = w + 2 * B * kH1;
-    a.a2 = w + 3 * B * kH1;
-    a.lg = w + 4 * B * kH1;
-    a.dl = a.lg + B * kOut;
-    a.d2 = a.dl + B * kOut;
-    a.d1 = a.d2 + B * kH2;
-    a.loss = a.d1 + B * kH1;
-    return a;
-}
-
-static inline unsigned nb(int64_t n) { return (unsigned)((n + 255) / 256); }
-
-static int forward(Mlp &M, const float *X, int B, cudaStream_t s) {
-    const Acts a = acts(M);
-    dense_fwd<<<nb((int64_t)B * kH1), 256, 0, s>>>(X, B, kIn, M.p + oW1, M.p + oB1, kH1, 1, a.z1, a.a1);
-    dense_fwd<<<nb((int64_t)B * kH2), 256, 0, s>>>(a.a1, B, kH1, M.p + oW2, M.p + oB2, kH2, 1, a.z2, a.a2);
-    dense_fwd<<<nb((int64_t)B * kOut), 256, 0, s>>>(a.a2, B, kH2, M.p + oW3, M.p + oB3, kOut, 0, nullptr, a.lg);
+static int forward(Mlp &M, const float *X, int B, float *logits, int32_t *s_out, int32_t *m_out, cudaStream_t s) {
+    mlp_forward_kernel<<<grad_blocks(B), kMlpThreads, 0, s>>>(M.p, X, B, logits, s_out, m_out);
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
 
-static int gradient(Mlp &M, const float *X, const int32_t *ys, const int32_t *ym, int B, cudaStream_t s) {
-    DQ_TRY(forward(M, X, B, s));
-    const Acts a = acts(M);
-    softmax_ce<<<nb(B), 256, 0, s>>>(a.lg, ys, ym, B, a.dl, a.loss);
-    dense_bwd_w<<<nb(kH2 * kOut + kOut), 256, 0, s>>>(a.a2, a.dl, B, kH2, kOut, M.g + oW3, M.g + oB3);
-    dense_bwd_x<<<nb((int64_t)B * kH2), 256, 0, s>>>(a.dl, M.p + oW3, a.z2, B, kH2, kOut, a.d2);
-    dense_bwd_w<<<nb(kH1 * kH2 + kH2), 256, 0, s>>>(a.a1, a.d2, B, kH1, kH2, M.g + oW2, M.g + oB2);
-    dense_bwd_x<<<nb((int64_t)B * kH1), 256, 0, s>>>(a.d2, M.p + oW2, a.z1, B, kH1, kH2, a.d1);
-    dense_bwd_w<<<nb(kIn * kH1 + kH1), 256, 0, s>>>(X, a.d1, B, kIn, kH1, M.g + oW1, M.g + oB1);
+// The batch's gradient into g (may be NULL) and, with adam, into an Adam step.
+static int gradient(Mlp &M, const float *X, const int32_t *ys, const int32_t *ym, int B, float *loss, float *g,
+                    const AdamStep *adam, cudaStream_t s) {
+    const int nblk = grad_blocks(B);
+    DQ_TRY(ensure_work(M, nblk));
+    mlp_grad_kernel<<<nblk, kMlpThreads, 0, s>>>(M.p, X, ys, ym, B, loss, M.work);
+    mlp_reduce_kernel<<<(kParams + 31) / 32, 32 * kSlices, 0, s>>>(M.work, nblk, g, adam ? 1 : 0, adam ? *adam : AdamStep{});
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
@@ -201,12 +314,11 @@ int diaq_mlp_create(uint64_t seed, diaq_mlp_t *out) {
     init(oW2, kH1, kH1 * kH2);
     init(oW3, kH2, kH2 * kOut);
     diaq_mlp_s *M = new diaq_mlp_s();
-    cudaError_t e = dev_malloc(&M->p, sizeof(float) * 4 * kParams);
+    cudaError_t e = dev_malloc(&M->p, sizeof(float) * 3 * kParams);
     if (e == cudaSuccess) {
-        M->g = M->p + kParams;
-        M->m = M->p + 2 * kParams;
-        M->v = M->p + 3 * kParams;
-        e = cudaMemset(M->p, 0, sizeof(float) * 4 * kParams);
+        M->m = M->p + kParams;
+        M->v = M->p + 2 * kParams;
+        e = cudaMemset(M->p, 0, sizeof(float) * 3 * kParams);
     }
     if (e == cudaSuccess) e = cudaMemcpy(M->p, h.data(), sizeof(float) * kParams, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -239,46 +351,31 @@ int diaq_mlp_set_params(diaq_mlp_t M, const float *host_in) {
 int diaq_mlp_forward(diaq_mlp_t M, const float *X, int B, float *logits, void *stream) {
     if (!M || !X || !logits || B < 0) return set_error(DIAQ_ERR_INVALID, "mlp forward: bad argument");
     if (B == 0) return DIAQ_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    DQ_TRY(ensure_work(*M, B));
-    DQ_TRY(forward(*M, X, B, s));
-    DQ_CUDA(cudaMemcpyAsync(logits, acts(*M).lg, sizeof(float) * kOut * (size_t)B, cudaMemcpyDeviceToDevice, s));
-    return DIAQ_OK;
+    return forward(*M, X, B, logits, nullptr, nullptr, (cudaStream_t)stream);
 }
 
 int diaq_mlp_gradient(diaq_mlp_t M, const float *X, const int32_t *s_label, const int32_t *m_label, int B,
                       float *grad_out, float *loss_out, void *stream) {
     if (!M || !X || !s_label || !m_label || B <= 0) return set_error(DIAQ_ERR_INVALID, "mlp gradient: bad argument");
-    cudaStream_t s = (cudaStream_t)stream;
-    DQ_TRY(ensure_work(*M, B));
-    DQ_TRY(gradient(*M, X, s_label, m_label, B, s));
-    if (grad_out) DQ_CUDA(cudaMemcpyAsync(grad_out, M->g, sizeof(float) * kParams, cudaMemcpyDeviceToDevice, s));
-    if (loss_out) DQ_CUDA(cudaMemcpyAsync(loss_out, acts(*M).loss, sizeof(float) * B, cudaMemcpyDeviceToDevice, s));
-    return DIAQ_OK;
+    return gradient(*M, X, s_label, m_label, B, loss_out, grad_out, nullptr, (cudaStream_t)stream);
 }
 
 int diaq_mlp_train_step(diaq_mlp_t M, const float *X, const int32_t *s_label, const int32_t *m_label, int B,
                         float lr, float *loss_out, void *stream) {
-    DQ_TRY(diaq_mlp_gradient(M, X, s_label, m_label, B, nullptr, loss_out, stream));
-    cudaStream_t s = (cudaStream_t)stream;
-    M->t += 1;
+    if (!M || !X || !s_label || !m_label || B <= 0) return set_error(DIAQ_ERR_INVALID, "mlp gradient: bad argument");
     const float b1 = 0.9f, b2 = 0.999f;
-    const float bc1 = 1.f - (float)std::pow((double)b1, (double)M->t);
-    const float bc2 = 1.f - (float)std::pow((double)b2, (double)M->t);
-    adam_kernel<<<nb(kParams), 256, 0, s>>>(M->p, M->g, M->m, M->v, kParams, lr, b1, b2, 1e-8f, bc1, bc2);
-    DQ_CUDA(cudaGetLastError());
+    const int64_t t = M->t + 1;
+    const AdamStep A{M->p, M->m, M->v, lr, b1, b2, 1e-8f, 1.f - (float)std::pow((double)b1, (double)t),
+                     1.f - (float)std::pow((double)b2, (double)t)};
+    DQ_TRY(gradient(*M, X, s_label, m_label, B, loss_out, nullptr, &A, (cudaStream_t)stream));
+    M->t = t;
     return DIAQ_OK;
 }
 
 int diaq_mlp_propose(diaq_mlp_t M, const float *X, int B, int32_t *s_out, int32_t *m_out, void *stream) {
     if (!M || !X || !s_out || !m_out || B < 0) return set_error(DIAQ_ERR_INVALID, "mlp propose: bad argument");
     if (B == 0) return DIAQ_OK;
-    cudaStream_t s = (cudaStream_t)stream;
-    DQ_TRY(ensure_work(*M, B));
-    DQ_TRY(forward(*M, X, B, s));
-    argmax_heads<<<nb(B), 256, 0, s>>>(acts(*M).lg, B, s_out, m_out);
-    DQ_CUDA(cudaGetLastError());
-    return DIAQ_OK;
+    return forward(*M, X, B, nullptr, s_out, m_out, (cudaStream_t)stream);
 }
 
 }  // extern "C"
