@@ -743,7 +743,7 @@ int diaq_batch_create(int n_inst, const diaq_matrix_t *H, const int *nrhs, doubl
     cudaError_t e = cudaStreamCreateWithFlags(&B->s, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = dev_malloc(&B->work, work_bytes + 256);
     size_t mask_words = 0;
-    for (int i = 0; i < n_inst; ++i) mask_words += (size_t)H[i]->nd * (size_t)tile_mask_words(H[i]->rows);
+    for (int i = 0; i < n_inst; ++i) mask_words += tile_mask_bytes(H[i]->nd, H[i]->rows) / sizeof(uint32_t);
     if (e == cudaSuccess) e = dev_malloc(&B->masks, sizeof(uint32_t) * std::max<size_t>(mask_words, 1));
     if (e == cudaSuccess) e = dev_malloc(&B->d_inst, sizeof(BatchInst) * n_inst);
     if (e != cudaSuccess) {
@@ -765,7 +765,7 @@ int diaq_batch_create(int n_inst, const diaq_matrix_t *H, const int *nrhs, doubl
         I.il_ok = il_shape(i, I.sp, I.n_pad) ? 1 : 0;
         I.tmask = B->masks + mask_off;
         I.mw = tile_mask_words(H[i]->rows);
-        mask_off += (size_t)H[i]->nd * (size_t)I.mw;
+        mask_off += tile_mask_bytes(H[i]->nd, H[i]->rows) / sizeof(uint32_t);
         B->mats.push_back(H[i]);
         const size_t vb = vec_bytes(i);
         void **slots[8] = {&I.var, &I.vai, &I.vbr, &I.vbi, &I.hr, &I.hi, &I.lr, &I.li};

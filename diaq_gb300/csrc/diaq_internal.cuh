@@ -55,6 +55,12 @@ struct Matrix {
     size_t elem() const { return prec == DIAQ_C64 ? sizeof(float) : sizeof(double); }
 };
 
+// Zero-tile masks (described in spmv_kernel.cuh): words per diagonal, and bytes of the three planes.
+inline int64_t tile_mask_words(int64_t rows) { return (rows + 1023) / 1024; }
+inline size_t tile_mask_bytes(int64_t nd, int64_t rows) {
+    return 3 * sizeof(uint32_t) * (size_t)nd * (size_t)tile_mask_words(rows);
+}
+
 // ---- error state -------------------------------------------------------------------------
 int set_error(int status, const std::string &msg);
 int cuda_status(cudaError_t e, const char *what, const char *file, int line);

@@ -117,9 +117,11 @@ int allocate(Matrix &M, cudaStream_t s, bool zero) {
         DQ_CUDA(cudaMemsetAsync(M.im, 0, bytes, s));
     }
     if (M.nd > 0) {
-        // the zero-tile mask's storage, so that SpMV calls never allocate (it is filled on first use)
-        DQ_CUDA(dev_malloc(&M.tmask, sizeof(uint32_t) * (size_t)M.nd * (size_t)((M.rows + 1023) / 1024)));
-        DQ_CUDA(dev_malloc(&M.d_meta, sizeof(DiagMeta) * M.nd));
+        // metadata and, behind it, the zero-tile mask's storage, so that SpMV calls never allocate (it
+        // is filled on first use)
+        const size_t mb = (sizeof(DiagMeta) * (size_t)M.nd + 255) / 256 * 256;
+        DQ_CUDA(dev_malloc(&M.d_meta, mb + tile_mask_bytes(M.nd, M.rows)));
+        M.tmask = (uint32_t *)((uint8_t *)M.d_meta + mb);
         DQ_CUDA(cudaMemcpyAsync(M.d_meta, M.meta.data(), sizeof(DiagMeta) * M.nd,
                                 cudaMemcpyHostToDevice, s));
         // the host vector may be reallocated later; finish the copy before returning
@@ -132,7 +134,6 @@ void release(Matrix &M) {
     if (M.re) cudaFree(M.re);
     if (M.im) cudaFree(M.im);
     if (M.d_meta) cudaFree(M.d_meta);
-    if (M.tmask) cudaFree(M.tmask);
     M.re = M.im = nullptr;
     M.d_meta = nullptr;
     M.tmask = nullptr;

@@ -23,13 +23,13 @@ int spmv_launch(const Matrix &A, const void *xr, const void *xi, int64_t ldx, vo
         e.yr = (double *)yr;
         e.yi = (double *)yi;
         e.ldy = ldy;
-        return launch_dia_spmv_rhs<double>(A, (const double *)xr, (const double *)xi, ldx, nrhs, e, s);
+        return launch_dia_spmv_rhs<double>(A, (const double *)xr, (const double *)xi, ldx, nrhs, e, s, cached_tile_mask(A, s));
     }
     EpiStoreRhs<float> e;
     e.yr = (float *)yr;
     e.yi = (float *)yi;
     e.ldy = ldy;
-    return launch_dia_spmv_rhs<float>(A, (const float *)xr, (const float *)xi, ldx, nrhs, e, s);
+    return launch_dia_spmv_rhs<float>(A, (const float *)xr, (const float *)xi, ldx, nrhs, e, s, cached_tile_mask(A, s));
 }
 
 int taylor_term_launch(const Matrix &A, const void *tin_r, const void *tin_i, void *tout_r,
@@ -46,8 +46,7 @@ int taylor_term_launch(const Matrix &A, const void *tin_r, const void *tin_i, vo
         e.initi = (const double *)init_i;
         e.ld = ld;
         e.scale = scale;
-        return launch_dia_spmv_rhs_cfg<double, EpiTaylorRhs<double>, VecOf<double>::V>(
-            A, (const double *)tin_r, (const double *)tin_i, ld, nrhs, e, s, SpmvCfg{}, tmask);
+        return launch_dia_spmv_rhs<double>(A, (const double *)tin_r, (const double *)tin_i, ld, nrhs, e, s, tmask);
     }
     EpiTaylorRhs<float> e;
     e.tr = (float *)tout_r;
@@ -58,8 +57,7 @@ int taylor_term_launch(const Matrix &A, const void *tin_r, const void *tin_i, vo
     e.initi = (const float *)init_i;
     e.ld = ld;
     e.scale = (float)scale;
-    return launch_dia_spmv_rhs_cfg<float, EpiTaylorRhs<float>, VecOf<float>::V>(
-        A, (const float *)tin_r, (const float *)tin_i, ld, nrhs, e, s, SpmvCfg{}, tmask);
+    return launch_dia_spmv_rhs<float>(A, (const float *)tin_r, (const float *)tin_i, ld, nrhs, e, s, tmask);
 }
 
 }  // namespace diaq_gb300

@@ -23,13 +23,21 @@ constexpr int kMetaChunk = 256;
 // ---- zero-tile mask --------------------------------------------------------------------------------
 // One bit per diagonal and 32-row tile: bit t of word w of diagonal j is set when rows
 // 32 (32 w + t) .. 32 (32 w + t) + 31 of diagonal j hold a nonzero value (real or imaginary part),
-// word (j, w) at mask[j * tile_mask_words(rows) + w].  Kernels whose warps cover aligned 32-row
+// word (j, w) at mask[j * tile_mask_words(rows) + w]; two further planes of nd * tile_mask_words(rows)
+// words follow, the same for the real parts alone and for the imaginary parts alone.  Kernels whose warps cover aligned 32-row
 // tiles skip a clear tile whole -- no matrix load, no state window, no multiply-adds.  In
 // Pauli-sum Hamiltonians most off-diagonal tiles are zero: the hopping term of qubits k, k+1
 // fills a quarter of the rows of its diagonal, in runs of 2^k rows.  Leaving out terms a * x
 // with a == 0 changes no finite sum (up to the sign of a zero result).
-inline int64_t tile_mask_words(int64_t rows) { return (rows + 1023) / 1024; }
-// Fill the mask of A (tile_mask_words(A.rows) * A.nd words) on stream s.
+//
+// The plane words let a kernel go further in the tiles it visits: where one plane of the matrix is
+// all zero (the Hamiltonians of real spin chains, and each Pauli string's diagonal, hold one plane
+// only) it loads the other plane alone and runs two of the four multiply-adds of a complex product.
+// What is left out, 0 * x, matters only for an infinite or NaN x -- and such an x also reaches one of
+// the two sums through the plane that is used, since every value of a visited tile is multiplied.  So
+// a row whose sums come out non-finite (from x, from stored values, or by overflow) is summed again
+// with both planes: the results are those of the full product in every case.
+// Fill the mask of A (tile_mask_bytes(A.nd, A.rows)) on stream s.
 int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s);
 // A's own mask, built (and waited for) on first use after its values were last written; NULL when
 // it cannot be had now (s is being captured into a graph, or allocation failed): visit every tile.
@@ -141,6 +149,66 @@ __device__ __forceinline__ uint32_t block_tile_bits(uint32_t w, int64_t row0, in
     return tiles >= 32 ? w : (w >> ((row0 >> 5) & 31)) & ((1u << tiles) - 1u);
 }
 
+// Whether any of the sums is infinite or NaN, from their bit patterns.
+__device__ __forceinline__ uint32_t abs_hi(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t abs_hi(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+template <typename T>
+__device__ __forceinline__ bool any_nonfinite(uint32_t largest) {
+    return largest >= (sizeof(T) == 4 ? 0x7f800000u : 0x7ff00000u);
+}
+
+// One diagonal's value base and the word of its imaginary plane's mask for the block's rows.
+struct BaseIm {
+    int64_t base;
+    uint32_t im;
+    uint32_t pad;
+};
+
+// One diagonal's (q = offset, lo, hi) products with rows r0 .. r0 + V - 1 of up to K states, the real
+// (RE) and the imaginary (IM) plane of the matrix each taken or left out.
+template <typename T, int K, int V, bool RE, bool IM>
+__device__ __forceinline__ void dia_mac(const int4 &q, int64_t base, int64_t r0, const T *__restrict__ are,
+                                        const T *__restrict__ aim, const T *__restrict__ xr, const T *__restrict__ xi,
+                                        int64_t ldx, int kq, T (&accr)[K][V], T (&acci)[K][V]) {
+    constexpr int VB = V * (int)sizeof(T);
+    const int64_t lo = q.y, hi = q.z;
+    const bool full = (r0 >= lo) && (r0 + V <= hi);
+    T ar[V], ai[V];
+    if constexpr (RE) load_vec_stream<T, V>(ar, are + base + r0);
+    if constexpr (IM) load_vec_stream<T, V>(ai, aim + base + r0);
+    if (!full) {
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (r0 + v < lo || r0 + v >= hi) ar[v] = ai[v] = (T)0;
+    }
+    const int64_t c = r0 + q.x;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        if (k >= kq) break;
+        const T *pxr = xr + k * ldx + c;
+        const T *pxi = xi + k * ldx + c;
+        T xrv[V], xiv[V];
+        if (full && aligned_to<VB>(pxr) && aligned_to<VB>(pxi)) {
+            load_vec<T, V>(xrv, pxr);
+            load_vec<T, V>(xiv, pxi);
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const bool ok = (r0 + v >= lo) && (r0 + v < hi);
+                xrv[v] = ok ? __ldg(pxr + v) : (T)0;
+                xiv[v] = ok ? __ldg(pxi + v) : (T)0;
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            if constexpr (RE) accr[k][v] = fma(ar[v], xrv[v], accr[k][v]);
+            if constexpr (IM) accr[k][v] = fma(-ai[v], xiv[v], accr[k][v]);
+            if constexpr (RE) acci[k][v] = fma(ar[v], xiv[v], acci[k][v]);
+            if constexpr (IM) acci[k][v] = fma(ai[v], xrv[v], acci[k][v]);
+        }
+    }
+}
+
 // nrhs states in nchunk chunks of up to K, VR rows per thread.  Block b works on chunk
 // b % nchunk of row tile b / nchunk: the blocks of one row tile are neighbours in launch order and
 // run at the same time, so the matrix tile they all read comes from HBM once and from L2 for the
@@ -152,11 +220,10 @@ __global__ void __launch_bounds__(kSpmvThreads)
                     const T *__restrict__ xi, int64_t ldx, int nrhs, int nchunk, const uint32_t *__restrict__ tmask,
                     int64_t mw, Epi epi0) {
     constexpr int V = VR;
-    constexpr int VB = VR * (int)sizeof(T);
-    // per diagonal: offset, row range and the zero-tile mask word of the block's rows in one
-    // 16-byte record (rows < 2^31), the value base beside it
+    // per diagonal: offset, row range and the real plane's mask word of the block's rows in one
+    // 16-byte record (rows < 2^31), the value base and the imaginary plane's word in another
     __shared__ int4 sq[kMetaChunk];
-    __shared__ int64_t sb[kMetaChunk];
+    __shared__ BaseIm sb[kMetaChunk];
     const int chunk = (int)(blockIdx.x % (unsigned)nchunk);
     const int64_t tile = blockIdx.x / (unsigned)nchunk;
     const int q0 = chunk * K;
@@ -169,67 +236,225 @@ __global__ void __launch_bounds__(kSpmvThreads)
     const int64_t mword = (tile * kSpmvThreads * V) >> 10;
     const int tbit = (int)((r0 >> 5) & 31);
     T accr[K][V], acci[K][V];
-#pragma unroll
-    for (int q = 0; q < K; ++q)
-#pragma unroll
-        for (int v = 0; v < V; ++v) accr[q][v] = acci[q][v] = (T)0;
 
-    for (int c0 = 0; c0 < nd; c0 += kMetaChunk) {
-        const int cn = min(kMetaChunk, nd - c0);
-        __syncthreads();
-        for (int i = threadIdx.x; i < cn; i += kSpmvThreads) {
-            const DiagMeta m = meta[c0 + i];
-            const uint32_t w = tmask ? tmask[(int64_t)(c0 + i) * mw + mword] : 0xffffffffu;
-            sq[i] = make_int4(m.off, (int)m.lo, (int)m.hi, (int)w);
-            sb[i] = m.base;
-        }
-        __syncthreads();
-        if (r0 >= rows) continue;
+    for (int pass = 0;; ++pass) {  // a second pass, with both planes, for rows that are not finite
+#pragma unroll
+        for (int q = 0; q < K; ++q)
+#pragma unroll
+            for (int v = 0; v < V; ++v) accr[q][v] = acci[q][v] = (T)0;
+        for (int c0 = 0; c0 < nd; c0 += kMetaChunk) {
+            const int cn = min(kMetaChunk, nd - c0);
+            if (pass == 0 || nd > kMetaChunk) {
+                __syncthreads();
+                for (int i = threadIdx.x; i < cn; i += kSpmvThreads) {
+                    const DiagMeta m = meta[c0 + i];
+                    const int64_t w = (int64_t)(c0 + i) * mw + mword;
+                    const uint32_t wr = tmask ? tmask[nd * mw + w] : 0xffffffffu;
+                    const uint32_t wi = tmask ? tmask[2 * nd * mw + w] : 0xffffffffu;
+                    sq[i] = make_int4(m.off, (int)m.lo, (int)m.hi, (int)wr);
+                    sb[i] = BaseIm{m.base, wi, 0u};
+                }
+                __syncthreads();
+            }
+            if (r0 >= rows) continue;
 #pragma unroll 2
-        for (int k = 0; k < cn; ++k) {
-            const int4 q = sq[k];
-            const int64_t lo = q.y, hi = q.z;
-            if (r0 + V <= lo || r0 >= hi || !(((uint32_t)q.w >> tbit) & 1u)) continue;
-            const int64_t base = sb[k];
-            const int64_t d = q.x;
-            T ar[V], ai[V];
-            load_vec_stream<T, V>(ar, are + base + r0);
-            load_vec_stream<T, V>(ai, aim + base + r0);
-            const bool full = (r0 >= lo) && (r0 + V <= hi);
-            if (!full) {
-#pragma unroll
-                for (int v = 0; v < V; ++v)
-                    if (r0 + v < lo || r0 + v >= hi) ar[v] = ai[v] = (T)0;
-            }
-            const int64_t c = r0 + d;
-#pragma unroll
-            for (int q = 0; q < K; ++q) {
-                if (q >= kq) break;
-                const T *pxr = xr + q * ldx + c;
-                const T *pxi = xi + q * ldx + c;
-                T xrv[V], xiv[V];
-                if (full && aligned_to<VB>(pxr) && aligned_to<VB>(pxi)) {
-                    load_vec<T, V>(xrv, pxr);
-                    load_vec<T, V>(xiv, pxi);
-                } else {
-#pragma unroll
-                    for (int v = 0; v < V; ++v) {
-                        const bool ok = (r0 + v >= lo) && (r0 + v < hi);
-                        xrv[v] = ok ? __ldg(pxr + v) : (T)0;
-                        xiv[v] = ok ? __ldg(pxi + v) : (T)0;
-                    }
-                }
-#pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    accr[q][v] = fma(ar[v], xrv[v], accr[q][v]);
-                    accr[q][v] = fma(-ai[v], xiv[v], accr[q][v]);
-                    acci[q][v] = fma(ar[v], xiv[v], acci[q][v]);
-                    acci[q][v] = fma(ai[v], xrv[v], acci[q][v]);
-                }
+            for (int k = 0; k < cn; ++k) {
+                const int4 q = sq[k];
+                const BaseIm b = sb[k];
+                const int64_t lo = q.y, hi = q.z;
+                bool re = ((uint32_t)q.w >> tbit) & 1u, im = (b.im >> tbit) & 1u;
+                if (r0 + V <= lo || r0 >= hi || !(re || im)) continue;
+                if (pass) re = im = true;
+                // whole bodies rather than conditions around the multiply-adds: those become
+                // predicates, and a predicated-off FP64 multiply-add takes its issue slots all the same
+                // (165 us per c128 product on the 20-qubit chain).  float32 takes imaginary-only tiles
+                // as complex ones: a third body cost its complex tiles 4 %
+                if (!im)
+                    dia_mac<T, K, V, true, false>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
+                else if (re || sizeof(T) == 4)
+                    dia_mac<T, K, V, true, true>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
+                else
+                    dia_mac<T, K, V, false, true>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
             }
         }
+        if (pass || !tmask) break;
+        uint32_t big = 0u;
+#pragma unroll
+        for (int q = 0; q < K; ++q)
+#pragma unroll
+            for (int v = 0; v < V; ++v) big = max(big, max(abs_hi(accr[q][v]), abs_hi(acci[q][v])));
+        // with several chunks the staging barriers make the second pass the whole block's
+        const bool again = any_nonfinite<T>(big);
+        if (!(nd > kMetaChunk ? __syncthreads_or(again) : again)) break;
     }
     if (r0 < rows) epi.template apply<T, K, V>(r0, rows, kq, accr, acci);
+}
+
+// One row per thread in blocks of NT threads, for matrices of few rows.  With only a few warps per SM
+// nothing hides the chain of one diagonal after the other, so each warp finds the diagonals that hold
+// a nonzero in its 32 rows 32 at a time (one per lane, ballots for the two planes) and issues the loads
+// of U of them before the multiply-adds of the first; small blocks spread the rows over more SMs.  The
+// sums are those of dia_spmv_kernel, in its order.
+//
+// 12-qubit chain, 25 diagonals, one state: c128 6.4 us against 10.3 for dia_spmv_kernel with one row
+// per thread (16.4 with two), c64 6.3 against 10.3.  The line to dia_spmv_kernel (rows x state chunks):
+// float64 is bound by FP64 issue sooner and loses from there on (131,072 rows: 16.6 against 14.5 us on
+// the XXZ chain, 43.8 against 38.7 on a Pauli sum; 32,768 rows: 8.3 against 10.4); float32, against 4
+// rows per thread, holds to twice that (250,007 rows, 37 random diagonals: 18.6 against 21.5 us).
+template <typename T>
+constexpr int64_t kRowKernelMax = sizeof(T) == 8 ? 65536 : 262144;
+
+template <typename T, int K, int NT, int U, class Epi>
+__global__ void __launch_bounds__(NT)
+    dia_spmv_row_kernel(const DiagMeta *__restrict__ meta, int nd, const T *__restrict__ are,
+                        const T *__restrict__ aim, int rows, const T *__restrict__ xr, const T *__restrict__ xi,
+                        int64_t ldx, int nrhs, int nchunk, const uint32_t *__restrict__ tmask, int64_t mw, Epi epi0) {
+    __shared__ int4 sq[kMetaChunk];
+    __shared__ BaseIm sb[kMetaChunk];
+    const int chunk = (int)(blockIdx.x % (unsigned)nchunk);
+    const int tile = blockIdx.x / (unsigned)nchunk;
+    const int q0 = chunk * K;
+    const int kq = min(K, nrhs - q0);
+    xr += q0 * ldx;
+    xi += q0 * ldx;
+    const Epi epi = epi0.shifted(q0);
+    const int lane = (int)threadIdx.x & 31;
+    const int r = tile * NT + (int)threadIdx.x, w0 = r - lane;
+    const int64_t mword = ((int64_t)tile * NT) >> 10;
+    const uint32_t mine = 1u << ((r >> 5) & 31);
+    T accr[K][1], acci[K][1];
+    xr += r;
+    xi += r;
+    are += r;
+    aim += r;
+    for (int pass = 0;; ++pass) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) accr[k][0] = acci[k][0] = (T)0;
+        for (int c0 = 0; c0 < nd; c0 += kMetaChunk) {
+            const int cn = min(kMetaChunk, nd - c0);
+            if (pass == 0 || nd > kMetaChunk) {
+                __syncthreads();
+                for (int i = threadIdx.x; i < cn; i += NT) {
+                    const DiagMeta m = meta[c0 + i];
+                    const int64_t w = (int64_t)(c0 + i) * mw + mword;
+                    const uint32_t wr = tmask ? tmask[nd * mw + w] : 0xffffffffu;
+                    const uint32_t wi = tmask ? tmask[2 * nd * mw + w] : 0xffffffffu;
+                    sq[i] = make_int4(m.off, (int)m.lo, (int)m.hi, (int)wr);
+                    sb[i] = BaseIm{m.base, wi, 0u};
+                }
+                __syncthreads();
+            }
+            for (int i0 = 0; i0 < cn; i0 += 32) {
+                bool re = false, im = false;
+                if (i0 + lane < cn) {
+                    const int4 q = sq[i0 + lane];
+                    if (w0 < q.z && w0 + 32 > q.y) {
+                        re = ((uint32_t)q.w & mine) != 0u;
+                        im = (sb[i0 + lane].im & mine) != 0u;
+                    }
+                }
+                uint32_t mr = __ballot_sync(0xffffffffu, re), mi = __ballot_sync(0xffffffffu, im), live = mr | mi;
+                if (pass) mr = mi = live;
+                struct D {
+                    T x[K], y[K];
+                };
+                auto load = [&](int j, bool &ok, int64_t &base, D &d) {
+                    const int4 q = sq[i0 + j];
+                    base = sb[i0 + j].base;
+                    ok = r >= q.y && r < q.z;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        if (k >= kq) break;
+                        d.x[k] = ok ? __ldg(xr + k * ldx + q.x) : (T)0;
+                        d.y[k] = ok ? __ldg(xi + k * ldx + q.x) : (T)0;
+                    }
+                };
+                auto mac_re = [&](T a, const D &d) {
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        if (k >= kq) break;
+                        accr[k][0] = fma(a, d.x[k], accr[k][0]);
+                        acci[k][0] = fma(a, d.y[k], acci[k][0]);
+                    }
+                };
+                auto mac_im = [&](T b, const D &d) {
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        if (k >= kq) break;
+                        accr[k][0] = fma(-b, d.y[k], accr[k][0]);
+                        acci[k][0] = fma(b, d.x[k], acci[k][0]);
+                    }
+                };
+                if (!mi || !mr) {  // one plane in all of these diagonals
+                    const T *pl = mi ? aim : are;
+                    while (live) {
+                        D d[U];
+                        T a[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            if (!live) {
+                                a[u] = (T)0;
+                                for (int k = 0; k < K; ++k) d[u].x[k] = d[u].y[k] = (T)0;
+                                continue;
+                            }
+                            const int j = __ffs(live) - 1;
+                            live &= live - 1u;
+                            bool ok;
+                            int64_t base;
+                            load(j, ok, base, d[u]);
+                            a[u] = ok ? __ldcs(pl + base) : (T)0;
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+                            if (mi) mac_im(a[u], d[u]);
+                            else mac_re(a[u], d[u]);
+                    }
+                } else {
+                    while (live) {
+                        D d[U];
+                        T a[U], b[U];
+                        uint32_t bit[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            bit[u] = live & (0u - live);
+                            if (!live) continue;
+                            const int j = __ffs(live) - 1;
+                            live &= live - 1u;
+                            bool ok;
+                            int64_t base;
+                            load(j, ok, base, d[u]);
+                            a[u] = ok && (mr & bit[u]) ? __ldcs(are + base) : (T)0;
+                            b[u] = ok && (mi & bit[u]) ? __ldcs(aim + base) : (T)0;
+                        }
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            if (!(mi & bit[u])) {
+                                if (bit[u]) mac_re(a[u], d[u]);
+                            } else if (!(mr & bit[u])) {
+                                mac_im(b[u], d[u]);
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < K; ++k) {
+                                    if (k >= kq) break;
+                                    accr[k][0] = fma(a[u], d[u].x[k], accr[k][0]);
+                                    accr[k][0] = fma(-b[u], d[u].y[k], accr[k][0]);
+                                    acci[k][0] = fma(a[u], d[u].y[k], acci[k][0]);
+                                    acci[k][0] = fma(b[u], d[u].x[k], acci[k][0]);
+                                }
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        if (pass || !tmask) break;
+        uint32_t big = 0u;
+#pragma unroll
+        for (int k = 0; k < K; ++k) big = max(big, max(abs_hi(accr[k][0]), abs_hi(acci[k][0])));
+        const bool again = any_nonfinite<T>(big);
+        if (!(nd > kMetaChunk ? __syncthreads_or(again) : __any_sync(0xffffffffu, again))) break;
+    }
+    if (r < rows) epi.template apply<T, K, 1>(r, rows, kq, accr, acci);
 }
 
 // ---- float variant with L2 prefetch of the matrix and shuffled state windows ----------------------
@@ -494,6 +719,16 @@ void launch_vr(int vr, const Matrix &A, const T *xr, const T *xi, int64_t ldx, i
             return;
         }
     }
+    if constexpr (VR == 1 && K <= 2) {
+        constexpr int NT = 64, U = K == 1 ? 4 : 2;
+        const int64_t blocks = (A.rows + NT - 1) / NT * nchunk;
+        if (A.rows * nchunk <= kRowKernelMax<T>) {
+            dia_spmv_row_kernel<T, K, NT, U, Epi><<<(unsigned)blocks, NT, 0, s>>>(
+                A.d_meta, A.nd, (const T *)A.re, (const T *)A.im, (int)A.rows, xr, xi, ldx, nrhs, nchunk, tmask,
+                tile_mask_words(A.rows), e);
+            return;
+        }
+    }
     dia_spmv_kernel<T, K, VR, Epi><<<spmv_blocks(A.rows, VR) * (unsigned)nchunk, kSpmvThreads, 0, s>>>(
         A.d_meta, A.nd, (const T *)A.re, (const T *)A.im, A.rows, xr, xi, ldx, nrhs, nchunk, tmask,
         tile_mask_words(A.rows), e);
@@ -573,12 +808,26 @@ int launch_dia_spmv_pf(const Matrix &A, const float *xr, const float *xi, int64_
     return DIAQ_OK;
 }
 
-// The default shape: 8 states per launch, 16-byte rows per thread.
+// The default shape, two states per block.  One row per thread for float64 (bound by FP64 issue or by
+// latency: 76 us against 83 with two rows on the 20-qubit chain, 43 against 53 on a 250,007-row
+// band, where unaligned windows fall apart into single loads) and for few rows (the row kernel);
+// 16-byte vectors of 4 rows for float32 above that (35 us against 62 on the 20-qubit chain).  Two
+// states per block rather than eight: 38 against 79 us for 11 float32 states of 65,536 rows, 40 against
+// 46 for 5 of 250,007.
+template <typename T>
+SpmvCfg default_cfg(int64_t rows, int nrhs) {
+    const int k = nrhs == 1 ? 1 : 2;
+    const bool few = rows * ((nrhs + k - 1) / k) <= kRowKernelMax<T>;
+    return SpmvCfg{k, sizeof(T) == 8 || few ? 1 : 4, 0};
+}
 template <typename T, class Epi>
 int launch_dia_spmv_rhs(const Matrix &A, const T *xr, const T *xi, int64_t ldx, int nrhs, Epi epi,
-                        cudaStream_t s) {
-    return launch_dia_spmv_rhs_cfg<T, Epi, VecOf<T>::V>(A, xr, xi, ldx, nrhs, epi, s, SpmvCfg{},
-                                                         cached_tile_mask(A, s));
+                        cudaStream_t s, const uint32_t *tmask) {
+    const SpmvCfg cfg = default_cfg<T>(A.rows, nrhs);
+    if constexpr (sizeof(T) == 4)
+        return launch_dia_spmv_rhs_cfg<T, Epi, 4, 1>(A, xr, xi, ldx, nrhs, epi, s, cfg, tmask);
+    else
+        return launch_dia_spmv_rhs_cfg<T, Epi, 1>(A, xr, xi, ldx, nrhs, epi, s, cfg, tmask);
 }
 
 template <typename T>

@@ -1,0 +1,128 @@
+"""Tiles that hold one plane of the matrix only (real or imaginary): the kernels leave the other
+plane out, and the results are those of the full complex product -- also for infinite and NaN
+values, which the products left out would have spread to the other plane."""
+import numpy as np
+import pytest
+
+from conftest import maxrel
+from oracle import oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+def planes(rows, cols, offsets, seed, scale=0.3):
+    """Packed values whose 32-row tiles are, at random, zero, real, imaginary or complex."""
+    rng = np.random.default_rng(seed)
+    re, im = [], []
+    for d in offsets:
+        lo, L = max(0, -d), min(rows, cols - d) - max(0, -d)
+        t = (lo + np.arange(L)) // 32
+        kind = rng.integers(0, 4, (rows + 31) // 32)[t]
+        re.append(np.where(kind & 1, rng.standard_normal(L) * scale, 0.0))
+        im.append(np.where(kind & 2, rng.standard_normal(L) * scale, 0.0))
+    return np.array(offsets, dtype=np.int32), np.concatenate(re), np.concatenate(im)
+
+
+def full_product(rows, cols, off, re, im, X):
+    """A x row by row with all four products of every value in a tile that holds a nonzero."""
+    yr, yi = np.zeros((len(X), rows)), np.zeros((len(X), rows))
+    p = 0
+    with np.errstate(all="ignore"):
+        for d in off:
+            lo, L = max(0, -d), min(rows, cols - d) - max(0, -d)
+            a, b, p = re[p:p + L], im[p:p + L], p + L
+            t = (lo + np.arange(L)) // 32
+            live = np.zeros((rows + 31) // 32, dtype=bool)
+            np.logical_or.at(live, t, (a != 0) | (b != 0))
+            keep = live[t]
+            r, a, b = (lo + np.arange(L))[keep], a[keep], b[keep]
+            xr, xi = X.real[:, r + d], X.imag[:, r + d]
+            yr[:, r] += a * xr
+            yr[:, r] -= b * xi
+            yi[:, r] += a * xi
+            yi[:, r] += b * xr
+    return yr, yi
+
+
+def vectors(k, n, seed, special):
+    rng = np.random.default_rng(seed)
+    X = rng.standard_normal((k, n)) + 1j * rng.standard_normal((k, n))
+    if special:
+        at = rng.choice(n, size=12, replace=False)
+        for q in range(k):
+            X.real[q, at[:3]] = [np.inf, np.nan, -np.inf]
+            X.imag[q, at[3:6]] = [np.nan, np.inf, -np.inf]
+            X[q, at[6]] = complex(np.inf, np.nan)
+    return X
+
+
+MANY = list(range(-140, 150))  # more than one chunk of staged metadata
+
+
+@pytest.mark.parametrize("rows,cols,offs", [(3001, 2990, [0, 1, -1, 36, -37, 700, -701, 1501, 64]), (33, 40, [0, 2, -3]),
+                                            (1100, 1100, MANY)])
+@pytest.mark.parametrize("prec,k", [(0, 1), (0, 3), (1, 1), (1, 9)])
+@pytest.mark.parametrize("special", [False, True])
+def test_products_are_the_full_products(native, rows, cols, offs, prec, k, special):
+    import torch
+
+    capi, _ = native
+    off, re, im = planes(rows, cols, offs, 7)
+    dt = torch.float64 if prec != 1 else torch.float32
+    if prec == 1:
+        re, im = re.astype(np.float32).astype(float), im.astype(np.float32).astype(float)
+    M = capi.Matrix.create(rows, cols, off, re, im, precision=prec)
+    X = vectors(k, cols, 3, special)
+    if prec == 1:
+        X = X.astype(np.complex64).astype(complex)
+    xr, xi = (torch.from_numpy(np.ascontiguousarray(v)).to("cuda", dt) for v in (X.real, X.imag))
+    yr, yi = torch.empty(k, rows, device="cuda", dtype=dt), torch.empty(k, rows, device="cuda", dtype=dt)
+    capi.check(capi.lib().diaq_spmm(M.h, k, xr.data_ptr(), xi.data_ptr(), cols, yr.data_ptr(), yi.data_ptr(), rows, None))
+    want = full_product(rows, cols, off, re, im, X)
+    tol = 1e-13 if prec == 0 else 1e-5  # sums of up to 290 products of order 1, in the vectors' precision
+    for got, w in zip((yr, yi), want):
+        got = got.double().cpu().numpy()
+        assert np.array_equal(np.isnan(got), np.isnan(w))
+        assert np.array_equal(got[np.isinf(w)], w[np.isinf(w)])
+        ok = np.isfinite(w)
+        assert maxrel(got[ok], w[ok]) < tol
+        if special:
+            assert not ok.all()
+
+
+def _evolve(capi, H, N, X, mode, cfg):
+    import torch
+
+    E = capi.Evolve(H, len(X), mode)
+    E.set_config(*cfg)
+    pr, pi = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (X.real, X.imag))
+    E.run(pr, pi, N, 0.05, 1, 0, 3)
+    return np.stack([pr.cpu().numpy(), pi.cpu().numpy()])
+
+
+@pytest.mark.parametrize("k", [1, 4, 9])
+@pytest.mark.parametrize("mode", ["c128", "mixed", "horner"])
+def test_plans_are_the_full_products(native, k, mode):
+    """The plan kernels that look at the planes against the ones that always take both (the c128
+    plan: against the oracle), also with infinite and NaN states."""
+    capi, _ = native
+    N = 2100
+    off, re, im = planes(N, N, [0, 1, -1, 37, -37, 700, -700, 64, 5], 9)
+    H = capi.Matrix.create(N, N, off, re, im)
+    X = vectors(k, N, 4, False)
+    X /= np.linalg.norm(X, axis=1, keepdims=True)
+    bad = vectors(k, N, 4, True)
+    if mode == "c128":
+        A = orc.OMatrix(N, N, off, re, im)
+        for cfg in ((8, 1, 0), (4, 2, 0), (1, 2, 0)):
+            got = _evolve(capi, H, N, X, capi.EVOLVE_C128, cfg)
+            for q in range(k):
+                assert maxrel(got[0, q] + 1j * got[1, q], orc.ham_sim(A, X[q], 0.05, 1, 3)) < 1e-12
+        return
+    md = capi.EVOLVE_MIXED if mode == "mixed" else capi.EVOLVE_HORNER
+    for P in (X, bad):
+        want = _evolve(capi, H, N, P, md, (4, 1, 9))
+        assert np.isfinite(want).all() == (P is X)
+        for cfg in ((8, 1, 0), (4, 2, 0), (8, 4, 0), (4, 1, 12)):
+            got = _evolve(capi, H, N, P, md, cfg)
+            assert np.array_equal(got, want, equal_nan=True), cfg
