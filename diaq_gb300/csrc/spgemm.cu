@@ -7,12 +7,11 @@
 // compaction yields them ascending and distinct -- a counting sort, exact by construction, the
 // set the reference collects in a std::map (src/spGEMM.cpp:346-369).
 //
-// Numeric pass: the grid is (row tiles of C, diagonals of C).  In row-indexed form
-// C[r, dC] = sum_a A[r, dA_a] * B[r + dA_a, dC - dA_a]; the thread owning rows r0..r0+V-1 of
-// one C diagonal walks A's slots in order (metadata staged in shared memory), finds B's slot
-// for dC - dA through a dense offset->slot map, and accumulates the shifted products -- the
-// SpMV access pattern with B's diagonal in place of x.  Pairs of one C diagonal are summed in
-// A-slot order, as src/spGEMM_gpu.cu:55-77 and src/spGEMM.cpp:425-493 do.
+// Numeric pass: in row-indexed form C[r, dC] = sum_a A[r, dA_a] * B[r + dA_a, dC - dA_a].  The (A, B)
+// slot pairs of every C diagonal are listed once on the device; a warp owns a strip of rows, walks the
+// pairs of a run of C diagonals and accumulates the shifted products -- the SpMV access pattern with
+// B's diagonal in place of x.  Pairs of one C diagonal are summed in A-slot order, as
+// src/spGEMM_gpu.cu:55-77 and src/spGEMM.cpp:425-493 do.
 #include <algorithm>
 
 #include "spmv_kernel.cuh"
@@ -154,7 +153,8 @@ int spgemm_symbolic(const Matrix &A, const Matrix &B, std::vector<int32_t> &offC
 // ---- numeric pass -------------------------------------------------------------------------------
 // Pair lists first: for every C diagonal c, the (A slot, B slot) pairs with dA + dB = dC whose
 // rows can overlap C's, in A-slot order (the reference's summation order, src/spGEMM.cpp:346-378).
-// One thread per C diagonal counts them, the host scans the counts, the same thread writes them.
+// One warp per C diagonal counts them, the host scans the counts, the same warp writes them (one thread
+// per diagonal took 745 us for the 2,047 x 2,047 pairs of a full 1,024-row square, a warp 35 us).
 // The numeric kernel then walks only the pairs of its C diagonal -- an earlier version scanned
 // every A diagonal for every C diagonal and row tile (41 candidates for ~2.3 pairs on the
 // 20-qubit XXZ H H) and spent half its instructions on that.
@@ -167,99 +167,249 @@ __device__ __forceinline__ bool pair_rows(const DiagMeta &ma, const DiagMeta &mb
     return lo < hi;
 }
 
-// fill == nullptr: count the pairs of each C diagonal into cnt; else write them at start[c].
+// One warp per C diagonal, 32 A slots at a time (a ballot keeps the slot order).  fill == nullptr: count
+// the pairs of each C diagonal into cnt; else write them at start[c].
 __global__ void spgemm_pairs_kernel(const DiagMeta *__restrict__ mA, int ndA, const DiagMeta *__restrict__ mB,
                                     const int32_t *__restrict__ bslot, int64_t bmin, int64_t bmax,
                                     const DiagMeta *__restrict__ mC, int ndC, int32_t *__restrict__ cnt,
                                     const int64_t *__restrict__ start, int2 *__restrict__ fill) {
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ndC; c += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < ndC; c += warps) {
         const DiagMeta mc = mC[c];
         int64_t w = fill ? start[c] : 0;
         int32_t n = 0;
-        for (int a = 0; a < ndA; ++a) {
-            const DiagMeta ma = mA[a];
-            const int64_t db = (int64_t)mc.off - ma.off;
-            if (db < bmin || db > bmax) continue;
-            const int32_t b = bslot[db - bmin];
-            if (b < 0) continue;
-            int64_t lo, hi;
-            if (!pair_rows(ma, mB[b], mc, lo, hi)) continue;
-            if (fill) fill[w++] = make_int2(a, b);
-            ++n;
+        for (int a0 = 0; a0 < ndA; a0 += 32) {
+            const int a = a0 + lane;
+            int32_t b = -1;
+            if (a < ndA) {
+                const DiagMeta ma = mA[a];
+                const int64_t db = (int64_t)mc.off - ma.off;
+                if (db >= bmin && db <= bmax) b = bslot[db - bmin];
+                int64_t lo, hi;
+                if (b >= 0 && !pair_rows(ma, mB[b], mc, lo, hi)) b = -1;
+            }
+            const uint32_t in = __ballot_sync(0xffffffffu, b >= 0);
+            if (fill && b >= 0) fill[w + __popc(in & ((1u << lane) - 1u))] = make_int2(a, b);
+            w += __popc(in);
+            n += __popc(in);
         }
-        if (!fill) cnt[c] = n;
+        if (!fill && lane == 0) cnt[c] = n;
     }
 }
 
-// bit of row r's 32-row tile in diagonal slot j of a zero-tile mask (mw words per diagonal)
-__device__ __forceinline__ bool tile_live(const uint32_t *__restrict__ mask, int64_t mw, int j, int64_t r) {
-    return (__ldg(mask + (int64_t)j * mw + (r >> 10)) >> ((r >> 5) & 31)) & 1u;
+// Bits t0 .. t0 + n - 1 (n <= 8) of a mask row of mw words, bits outside it zero; all ones without a mask.
+__device__ __forceinline__ uint32_t mask_bits(const uint32_t *__restrict__ row, int64_t mw, int t0, int n) {
+    if (!row) return (1u << n) - 1u;
+    const int w = t0 >> 5;
+    const uint32_t lo = w >= 0 && w < mw ? __ldg(row + w) : 0u, hi = w + 1 >= 0 && w + 1 < mw ? __ldg(row + w + 1) : 0u;
+    return __funnelshift_r(lo, hi, t0 & 31) & ((1u << n) - 1u);
 }
 
-// Block (x, y): row tile x of the C diagonals y, y + gridDim.y, ...; thread t owns V rows.  With
-// the operands' zero-tile masks (maskA, maskB) a pair is skipped where A's tile or both B tiles
-// that its rows read are zero: a product with a zero factor adds nothing.
+// A pair that has a nonzero product in a warp's strip of rows: values of row r at A[a + r] and
+// B[b + r], rows [lo, hi); the live tiles of the strip (A: V bits per plane) and of the strip's B rows,
+// which start `s` rows into a tile (V + 1 bits per plane); its C diagonal, counted from the group's first.
+struct __align__(16) LivePair {
+    int64_t a, b;
+    int32_t lo, hi;
+    uint32_t s_c, bits;   // s | C diagonal << 8; bits: A re, A im, B re, B im, a byte each
+};
+// A C diagonal of the group: value base, rows, first pair.
+struct __align__(16) CDiag {
+    int64_t base, pstart;
+    int32_t lo, hi, pad[2];
+};
+
+template <typename T, int V>
+__device__ __forceinline__ void store_rows(T *__restrict__ p, int64_t lo, int64_t hi, int64_t r0, const T (&v)[V]) {
+    if (r0 >= lo && r0 + V <= hi) {
+        using VT = typename Vec<T, V>::type;
+        if constexpr (V == 2)
+            *reinterpret_cast<VT *>(p + r0) = VT{v[0], v[1]};
+        else
+            *reinterpret_cast<VT *>(p + r0) = VT{v[0], v[1], v[2], v[3]};
+    } else {
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+            if (r0 + i >= lo && r0 + i < hi) p[r0 + i] = v[i];
+    }
+}
+
+// Adds the pair's products to the sums of this thread's rows r0 .. r0 + V - 1; all: take both planes
+// of both operands whatever the masks say.
+template <typename T, int V>
+__device__ __forceinline__ void pair_mac(const LivePair &q, bool all, int64_t r0, int lane, const T *__restrict__ Are,
+                                         const T *__restrict__ Aim, const T *__restrict__ Bre,
+                                         const T *__restrict__ Bim, T (&accr)[V], T (&acci)[V]) {
+    // this thread's rows of the pair, if their own tiles are live
+    const uint32_t ta = q.bits | q.bits >> 8, tb = (q.bits >> 16) | (q.bits >> 24);
+    const int s = (int)(q.s_c & 0xffu) + lane * V;
+    if (r0 >= q.hi || r0 + V <= q.lo || !((ta >> (lane * V >> 5)) & 1u) || !(((tb >> (s >> 5)) | (tb >> ((s + V - 1) >> 5))) & 1u))
+        return;
+    const bool full = r0 >= q.lo && r0 + V <= q.hi;
+    auto load = [&](const T *base, bool vec, T(&out)[V]) {
+        if (full && vec) {
+            load_vec<T, V>(out, base + r0);
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; ++v) out[v] = r0 + v >= q.lo && r0 + v < q.hi ? __ldg(base + r0 + v) : (T)0;
+        }
+    };
+    const bool vb = ((q.b + r0) & (V - 1)) == 0;
+    const T *pa = Are + q.a, *pai = Aim + q.a, *pb = Bre + q.b, *pbi = Bim + q.b;
+    const uint32_t cls = all ? 0xffffffffu : q.bits;
+    const bool ar = cls & 0xffu, ai = cls & 0xff00u, br = cls & 0xff0000u, bi = cls & 0xff000000u;
+    if (ar != ai && br != bi) {   // one plane each
+        T a[V], b[V];
+        load(ar ? pa : pai, true, a);
+        load(br ? pb : pbi, vb, b);
+        if (ar == br) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) accr[v] = fma(ar ? a[v] : -a[v], b[v], accr[v]);
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; ++v) acci[v] = fma(a[v], b[v], acci[v]);
+        }
+    } else if (ar != ai) {        // one plane of A, both of B
+        T a[V], b[V], d[V];
+        load(ar ? pa : pai, true, a);
+        load(ar ? pb : pbi, vb, b);
+        load(ar ? pbi : pb, vb, d);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            accr[v] = fma(ar ? a[v] : -a[v], b[v], accr[v]);
+            acci[v] = fma(a[v], d[v], acci[v]);
+        }
+    } else if (br != bi) {        // both planes of A, one of B
+        T a[V], d[V], b[V];
+        load(br ? pa : pai, true, a);
+        load(br ? pai : pa, true, d);
+        load(br ? pb : pbi, vb, b);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            accr[v] = fma(br ? a[v] : -a[v], b[v], accr[v]);
+            acci[v] = fma(d[v], b[v], acci[v]);
+        }
+    } else {
+        T xr[V], xi[V], yr[V], yi[V];
+        load(pa, true, xr);
+        load(pai, true, xi);
+        load(pb, vb, yr);
+        load(pbi, vb, yi);
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            accr[v] = fma(xr[v], yr[v], accr[v]);
+            accr[v] = fma(-xi[v], yi[v], accr[v]);
+            acci[v] = fma(xr[v], yi[v], acci[v]);
+            acci[v] = fma(xi[v], yr[v], acci[v]);
+        }
+    }
+}
+
+// Block (x, y): row strips of x (one per warp, 32 V rows), a run of `chunk` C diagonals of y.  A warp
+// takes up to 32 of its C diagonals at a time, and their pairs -- 2.3 per diagonal on the XXZ chain's
+// H H, hundreds in a full square -- 32 at a time across the diagonals, a lane per pair: the lane reads
+// the pair's metadata and the operands' zero-tile masks of the strip (maskA, maskB: the plane of real
+// parts, the plane of imaginary parts psA / psB words behind it) and stages the pair in shared memory
+// if its product can hold a nonzero there, so that the chain of dependent reads is paid once for many
+// pairs.  The warp then walks the staged pairs, in order, and writes each C diagonal when its pairs
+// are done.  A product with a zero factor adds nothing, so a plane that is zero in the strip takes
+// part in no product: 1, 2 or 4 multiply-adds per row, each case a body of its own (see
+// dia_spmv_kernel).  A diagonal whose sums are not finite is summed again with all four products.
+//
+// H H of the 18-qubit chain (2.4 GB written, real values): 1,075 -> 677 us, 3.6 TB/s of stores; bound by
+// instruction issue (one thread reading its pair's metadata for itself, all four products: 1,075; the
+// products by plane alone: 965).  A full complex square of 1,024 rows, 2,047 diagonals: 19.9 -> 8.8 ms,
+// 82 % of the FP64 rate (4.3 G multiply-adds).
 template <typename T>
-__global__ void __launch_bounds__(kSpmvThreads)
+__global__ void __launch_bounds__(kSpmvThreads, 4)
     spgemm_numeric_kernel(const DiagMeta *__restrict__ mA, const T *__restrict__ Are, const T *__restrict__ Aim,
                           const DiagMeta *__restrict__ mB, const T *__restrict__ Bre, const T *__restrict__ Bim,
-                          const DiagMeta *__restrict__ mC, int ndC, const int64_t *__restrict__ pstart,
+                          const DiagMeta *__restrict__ mC, int ndC, int chunk, const int64_t *__restrict__ pstart,
                           const int2 *__restrict__ pairs, T *__restrict__ Cre, T *__restrict__ Cim,
-                          const uint32_t *__restrict__ maskA, int64_t mwA, const uint32_t *__restrict__ maskB,
-                          int64_t mwB) {
+                          const uint32_t *__restrict__ maskA, int64_t mwA, int64_t psA,
+                          const uint32_t *__restrict__ maskB, int64_t mwB, int64_t psB) {
     constexpr int V = VecOf<T>::V;
-    const int64_t r0 = ((int64_t)blockIdx.x * kSpmvThreads + threadIdx.x) * V;
-    for (int c = blockIdx.y; c < ndC; c += gridDim.y) {
-        const DiagMeta mc = mC[c];
-        if (r0 >= mc.hi || r0 + V <= mc.lo) continue;
+    __shared__ LivePair sp[kSpmvThreads / 32][32];
+    __shared__ CDiag sc[kSpmvThreads / 32][33];
+    const int lane = threadIdx.x & 31;
+    LivePair *mine = sp[threadIdx.x >> 5];
+    CDiag *cd = sc[threadIdx.x >> 5];
+    const int64_t w0 = ((int64_t)blockIdx.x * (kSpmvThreads / 32) + (threadIdx.x >> 5)) * 32 * V, r0 = w0 + lane * V;
+    const int cend = min(ndC, ((int)blockIdx.y + 1) * chunk);
+
+    // the pair at list position p, staged into L; whether it is live in the strip
+    auto stage = [&](int64_t p, int c, int64_t clo, int64_t chi, LivePair &L) {
+        const int2 ab = pairs[p];
+        const DiagMeta ma = mA[ab.x], mb = mB[ab.y];
+        const int64_t lo = max(max(ma.lo, mb.lo - (int64_t)ma.off), clo), hi = min(min(ma.hi, mb.hi - (int64_t)ma.off), chi);
+        const int bt = (int)(w0 + ma.off);   // first B row of the strip
+        const uint32_t *ka = maskA ? maskA + ab.x * mwA : nullptr, *kb = maskB ? maskB + ab.y * mwB : nullptr;
+        const uint32_t ar = mask_bits(ka, mwA, (int)(w0 >> 5), V), ai = mask_bits(ka ? ka + psA : ka, mwA, (int)(w0 >> 5), V);
+        const uint32_t br = mask_bits(kb, mwB, bt >> 5, V + 1), bi = mask_bits(kb ? kb + psB : kb, mwB, bt >> 5, V + 1);
+        L = LivePair{ma.base, mb.base + ma.off, (int)lo, (int)hi, (uint32_t)(bt & 31) | (uint32_t)c << 8,
+                     ar | ai << 8 | br << 16 | bi << 24};
+        return w0 < hi && w0 + 32 * V > lo && (ar | ai) && (br | bi);
+    };
+
+    for (int c0 = (int)blockIdx.y * chunk; c0 < cend; c0 += 32) {
+        const int nc = min(32, cend - c0);
+        __syncwarp();
+        if (lane < nc) {
+            const DiagMeta m = mC[c0 + lane];
+            cd[lane] = CDiag{m.base, pstart[c0 + lane], (int)m.lo, (int)m.hi, {0, 0}};
+        }
+        if (lane == 0) cd[nc].pstart = pstart[c0 + nc];
+        __syncwarp();
         T accr[V], acci[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) accr[v] = acci[v] = (T)0;
-        const int64_t p1 = pstart[c + 1];
-        for (int64_t p = pstart[c]; p < p1; ++p) {
-            const int2 ab = pairs[p];
-            const DiagMeta ma = mA[ab.x], mb = mB[ab.y];
-            int64_t lo, hi;
-            pair_rows(ma, mb, mc, lo, hi);
-            if (r0 + V <= lo || r0 >= hi) continue;
-            if (maskA) {  // r0 .. r0 + V - 1 share one tile (V | 32); their B rows span at most two
-                if (!tile_live(maskA, mwA, ab.x, r0)) continue;
-                const int64_t b0 = max(r0, lo) + ma.off, b1 = min(r0 + V, hi) - 1 + ma.off;
-                if (!tile_live(maskB, mwB, ab.y, b0) && !tile_live(maskB, mwB, ab.y, b1)) continue;
-            }
-            T ar[V], ai[V], br[V], bi[V];
-            load_vec<T, V>(ar, Are + ma.base + r0);
-            load_vec<T, V>(ai, Aim + ma.base + r0);
-            const bool full = (r0 >= lo) && (r0 + V <= hi);
-            const T *pbr = Bre + mb.base + r0 + ma.off;
-            const T *pbi = Bim + mb.base + r0 + ma.off;
-            if (full && aligned16(pbr)) {
-                load_vec<T, V>(br, pbr);
-                load_vec<T, V>(bi, pbi);
-            } else {
+        int c = 0;   // the diagonal being summed
+        // write it and go on to the next
+        auto finish = [&]() {
+            const CDiag q = cd[c];
+            if (w0 < q.hi && w0 + 32 * V > q.lo) {
+                uint32_t big = 0u;
 #pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    const bool ok = (r0 + v >= lo) && (r0 + v < hi);
-                    br[v] = ok ? __ldg(pbr + v) : (T)0;
-                    bi[v] = ok ? __ldg(pbi + v) : (T)0;
-                    if (!ok) ar[v] = ai[v] = (T)0;
+                for (int v = 0; v < V; ++v) big = max(big, max(abs_hi(accr[v]), abs_hi(acci[v])));
+                if (maskA && __any_sync(0xffffffffu, any_nonfinite<T>(big))) {
+#pragma unroll
+                    for (int v = 0; v < V; ++v) accr[v] = acci[v] = (T)0;
+                    const int64_t p1 = cd[c + 1].pstart;
+                    for (int64_t p = q.pstart; p < p1; ++p) {
+                        LivePair L;
+                        if (stage(p, c, q.lo, q.hi, L)) pair_mac<T, V>(L, true, r0, lane, Are, Aim, Bre, Bim, accr, acci);
+                    }
                 }
+                store_rows<T, V>(Cre + q.base, q.lo, q.hi, r0, accr);
+                store_rows<T, V>(Cim + q.base, q.lo, q.hi, r0, acci);
             }
 #pragma unroll
-            for (int v = 0; v < V; ++v) {
-                accr[v] = fma(ar[v], br[v], accr[v]);
-                accr[v] = fma(-ai[v], bi[v], accr[v]);
-                acci[v] = fma(ar[v], bi[v], acci[v]);
-                acci[v] = fma(ai[v], br[v], acci[v]);
-            }
-        }
+            for (int v = 0; v < V; ++v) accr[v] = acci[v] = (T)0;
+            ++c;
+        };
+        const int64_t p1 = cd[nc].pstart;
+        for (int64_t p = cd[0].pstart;; p += 32) {
+            bool live = false;
+            LivePair L;
+            if (p + lane < p1) {
+                int k = 0;   // the diagonal of pair p + lane: the last one whose list starts at or before it
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const int64_t r = r0 + v;
-            if (r >= mc.lo && r < mc.hi) {
-                Cre[mc.base + r] = accr[v];
-                Cim[mc.base + r] = acci[v];
+                for (int step = 16; step > 0; step >>= 1)
+                    if (k + step < nc && cd[k + step].pstart <= p + lane) k += step;
+                live = stage(p + lane, k, cd[k].lo, cd[k].hi, L);
             }
+            const uint32_t set = __ballot_sync(0xffffffffu, live);
+            if (live) mine[__popc(set & ((1u << lane) - 1u))] = L;
+            __syncwarp();
+            const int n = __popc(set), last = p + 32 >= p1;
+            for (int k = 0; k < n + last; ++k) {   // after the last pair, the diagonals left
+                const int to = k < n ? (int)(mine[k].s_c >> 8) : nc;
+                while (c < to) finish();
+                if (k < n) pair_mac<T, V>(mine[k], false, r0, lane, Are, Aim, Bre, Bim, accr, acci);
+                __syncwarp();
+            }
+            if (last) break;
+            __syncwarp();
         }
     }
 }
@@ -289,7 +439,7 @@ int spgemm_numeric(const Matrix &A, const Matrix &B, Matrix &C, cudaStream_t s) 
     int2 *dpairs = nullptr;
     std::vector<int32_t> cnt((size_t)C.nd);
     std::vector<int64_t> start((size_t)C.nd + 1, 0);
-    const int pg = (int)std::max<int64_t>(1, std::min<int64_t>((C.nd + 127) / 128, 4 * num_sms()));
+    const int pg = (int)std::max<int64_t>(1, std::min<int64_t>((C.nd + 3) / 4, 8 * num_sms()));
     cudaError_t e = cudaMemcpyAsync(dmap, map.data(), mbytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         spgemm_pairs_kernel<<<pg, 128, 0, s>>>(A.d_meta, A.nd, B.d_meta, dmap, bmin, bmax, C.d_meta, C.nd, dcnt,
@@ -310,20 +460,29 @@ int spgemm_numeric(const Matrix &A, const Matrix &B, Matrix &C, cudaStream_t s) 
         int64_t maxrows = 1;
         for (const auto &m : C.meta) maxrows = std::max(maxrows, m.hi);
         const int V = A.prec == DIAQ_C128 ? 2 : 4;
-        // up to 64 C diagonals per block row: each block walks several diagonals' pairs
-        const dim3 grid(spmv_blocks(maxrows, V), (unsigned)std::min<int64_t>(C.nd, 64));
+        // runs of C diagonals per block: 64 of them, or more where the rows are few -- some 32 blocks
+        // per SM, as the pairs per diagonal vary (1,024 rows, 2,047 diagonals squared: 8.8 ms; 9.4
+        // with half as many runs, 19.9 with 64)
+        const unsigned gx = spmv_blocks(maxrows, V);
+        const int64_t runs = std::min<int64_t>(C.nd, std::max<int64_t>(64, std::min<int64_t>(65535, 32 * (int64_t)num_sms() / gx)));
+        const int chunk = (int)((C.nd + runs - 1) / runs);
+        const dim3 grid(gx, (unsigned)((C.nd + chunk - 1) / chunk));
         // the operands' masks (both or neither); taken here, outside any graph capture
         const uint32_t *ka = cached_tile_mask(A, s), *kb = ka ? cached_tile_mask(B, s) : nullptr;
         if (!kb) ka = nullptr;
-        const int64_t wa = tile_mask_words(A.rows), wb = tile_mask_words(B.rows);
+        const int64_t wa = tile_mask_words(A.rows), wb = tile_mask_words(B.rows), pa = wa * A.nd, pb = wb * B.nd;
+        if (ka) {   // the planes of real parts; those of imaginary parts follow
+            ka += pa;
+            kb += pb;
+        }
         if (A.prec == DIAQ_C128)
             spgemm_numeric_kernel<double><<<grid, kSpmvThreads, 0, s>>>(
                 A.d_meta, (const double *)A.re, (const double *)A.im, B.d_meta, (const double *)B.re,
-                (const double *)B.im, C.d_meta, C.nd, dstart, dpairs, (double *)C.re, (double *)C.im, ka, wa, kb, wb);
+                (const double *)B.im, C.d_meta, C.nd, chunk, dstart, dpairs, (double *)C.re, (double *)C.im, ka, wa, pa, kb, wb, pb);
         else
             spgemm_numeric_kernel<float><<<grid, kSpmvThreads, 0, s>>>(
                 A.d_meta, (const float *)A.re, (const float *)A.im, B.d_meta, (const float *)B.re,
-                (const float *)B.im, C.d_meta, C.nd, dstart, dpairs, (float *)C.re, (float *)C.im, ka, wa, kb, wb);
+                (const float *)B.im, C.d_meta, C.nd, chunk, dstart, dpairs, (float *)C.re, (float *)C.im, ka, wa, pa, kb, wb, pb);
         e = cudaGetLastError();
     }
     // the host vectors must outlive the async copies

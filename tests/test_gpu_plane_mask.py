@@ -126,3 +126,77 @@ def test_plans_are_the_full_products(native, k, mode):
         for cfg in ((8, 1, 0), (4, 2, 0), (8, 4, 0), (4, 1, 12)):
             got = _evolve(capi, H, N, P, md, cfg)
             assert np.array_equal(got, want, equal_nan=True), cfg
+
+
+def _special(off, rows, cols, re, im, seed):
+    """The matrix with every tile holding a nonzero, and a few infinite and NaN values."""
+    rng = np.random.default_rng(seed)
+    p = 0
+    for d in off:
+        L = min(rows, cols - d) - max(0, -d)
+        t = (max(0, -d) + np.arange(L)) // 32
+        live = np.zeros((rows + 31) // 32, dtype=bool)
+        np.logical_or.at(live, t, (re[p:p + L] != 0) | (im[p:p + L] != 0))
+        re[p:p + L][~live[t]] = 0.25
+        p += L
+    at = rng.choice(len(re), size=6, replace=False)
+    re[at[:2]], im[at[2:4]] = [np.inf, np.nan], [np.nan, -np.inf]
+    return re, im
+
+
+@pytest.mark.parametrize("prec,tol", [(0, 1e-13), (1, 1e-5)])
+@pytest.mark.parametrize("rows,inner,cols,offa,offb", [(1030, 1001, 1100, [0, 1, -3, 33, -65, 200], [0, -1, 5, 31, -40, 130]),
+                                                       (70, 64, 33, [0, -37, 2], [0, 1, -1]),
+                                                       (300, 300, 300, list(range(-45, 45)), list(range(-50, 50)))])
+@pytest.mark.parametrize("special", [False, True])
+def test_matrix_products_are_the_full_products(native, prec, tol, rows, inner, cols, offa, offb, special):
+    """A B by planes: more pairs per result diagonal than a warp stages at once (the third shape),
+    odd offsets, rectangular shapes; sums of at most 90 products of order 0.1."""
+    import ctypes
+
+    capi, _ = native
+    oa, ra, ia = planes(rows, inner, offa, 11)
+    ob, rb, ib = planes(inner, cols, offb, 12)
+    if special:
+        ra, ia = _special(oa, rows, inner, ra, ia, 5)
+        rb, ib = _special(ob, inner, cols, rb, ib, 6)
+    if prec == 1:
+        ra, ia, rb, ib = (v.astype(np.float32).astype(float) for v in (ra, ia, rb, ib))
+    A = capi.Matrix.create(rows, inner, oa, ra, ia, precision=prec)
+    B = capi.Matrix.create(inner, cols, ob, rb, ib, precision=prec)
+    out = ctypes.c_void_p()
+    capi.check(capi.lib().diaq_spgemm(A.h, B.h, 0, None, ctypes.byref(out)))
+    off, re, im = capi.Matrix(out).download()
+    want = {}
+    pa = 0
+    with np.errstate(all="ignore"):
+        for da in oa:
+            lo, L = max(0, -da), min(rows, inner - da) - max(0, -da)
+            a, b, pa = ra[pa:pa + L], ia[pa:pa + L], pa + L
+            pb = 0
+            for db in ob:
+                lob, Lb = max(0, -db), min(inner, cols - db) - max(0, -db)
+                c, d, pb = rb[pb:pb + Lb], ib[pb:pb + Lb], pb + Lb
+                r0, r1 = max(lo, lob - da), min(lo + L, lob + Lb - da)
+                if r0 >= r1:
+                    continue
+                wr, wi = want.setdefault(da + db, (np.zeros(rows), np.zeros(rows)))
+                u, v, x, y = a[r0 - lo:r1 - lo], b[r0 - lo:r1 - lo], c[r0 + da - lob:r1 + da - lob], d[r0 + da - lob:r1 + da - lob]
+                wr[r0:r1] += u * x
+                wr[r0:r1] -= v * y
+                wi[r0:r1] += u * y
+                wi[r0:r1] += v * x
+    assert set(want) <= set(off.tolist())
+    p = 0
+    bad = 0
+    for dc in off.tolist():
+        lo, L = max(0, -dc), min(rows, cols - dc) - max(0, -dc)
+        for got, w in ((re, want.get(dc, (np.zeros(rows),) * 2)[0]), (im, want.get(dc, (np.zeros(rows),) * 2)[1])):
+            g, w = got[p:p + L], w[lo:lo + L]
+            assert np.array_equal(np.isnan(g), np.isnan(w)), dc
+            assert np.array_equal(g[np.isinf(w)], w[np.isinf(w)]), dc
+            ok = np.isfinite(w)
+            bad += int((~ok).sum())
+            assert np.abs(g[ok] - w[ok]).max(initial=0.0) < tol * 10, dc
+        p += L
+    assert (bad > 0) == special
