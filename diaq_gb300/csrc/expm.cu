@@ -13,7 +13,7 @@
 
 namespace diaq_gb300 {
 
-int spgemm(const Matrix &A, const Matrix &B, bool prune, cudaStream_t s, Matrix **out);
+int spgemm(const Matrix &A, const Matrix &B, bool prune, cudaStream_t s, Matrix **out, bool internal);
 
 // ---- norms ---------------------------------------------------------------------------------------
 // Column sums of |re|+|im| (one thread per column, diagonals in slot order), max over columns via
@@ -196,7 +196,7 @@ __global__ void union_add_kernel(const DiagMeta *__restrict__ mA, const T *__res
 
 // A + sign * B over the union of the offsets, ascending (diaQMatrix::combined,
 // src/diaQMatrix.hpp:867-916).
-int union_add(const Matrix &A, const Matrix &B, double sign, cudaStream_t s, Matrix **out) {
+int union_add(const Matrix &A, const Matrix &B, double sign, cudaStream_t s, Matrix **out, bool internal) {
     if (A.rows != B.rows || A.cols != B.cols) return set_error(DIAQ_ERR_INVALID, "diaQMatrix::add: shape mismatch");
     std::map<int32_t, int2> u;
     for (int32_t k = 0; k < A.nd; ++k) u[A.off[k]] = make_int2(k, -1);
@@ -212,7 +212,7 @@ int union_add(const Matrix &A, const Matrix &B, double sign, cudaStream_t s, Mat
         slots.push_back(kv.second);
     }
     Matrix *C = nullptr;
-    DQ_TRY(make_zero(A.rows, A.cols, (int32_t)off.size(), off.data(), A.prec, s, &C));
+    DQ_TRY(make_zero(A.rows, A.cols, (int32_t)off.size(), off.data(), A.prec, s, &C, true, internal));
     if (C->nd == 0) {
         *out = C;
         return DIAQ_OK;
@@ -255,10 +255,10 @@ __global__ void fill_diag_kernel(T *__restrict__ re, T *__restrict__ im, int64_t
 }
 
 // identityMatrix(n) (src/specialMatrices.hpp:9-24).
-int identity(int64_t n, int prec, cudaStream_t s, Matrix **out) {
+int identity(int64_t n, int prec, cudaStream_t s, Matrix **out, bool internal) {
     const int32_t zero = 0;
     Matrix *I = nullptr;
-    DQ_TRY(make_zero(n, n, n > 0 ? 1 : 0, &zero, prec, s, &I));
+    DQ_TRY(make_zero(n, n, n > 0 ? 1 : 0, &zero, prec, s, &I, true, internal));
     if (n > 0) {
         const DiagMeta &m = I->meta[0];
         const int grid = (int)std::min<int64_t>((n + 255) / 256, 4 * num_sms());
@@ -303,7 +303,7 @@ __global__ void single_diag_exp_kernel(const T *__restrict__ are, const T *__res
 
 int single_diag_exp(const Matrix &A, int negative, double t, cudaStream_t s, Matrix **out) {
     Matrix *R = nullptr;
-    DQ_TRY(identity(A.rows, A.prec, s, &R));
+    DQ_TRY(identity(A.rows, A.prec, s, &R, false));
     const DiagMeta &ma = A.meta[0];
     const int64_t len = ma.hi - ma.lo;
     const DiagMeta &mr = R->meta[0];
@@ -329,13 +329,14 @@ int single_diag_exp(const Matrix &A, int negative, double t, cudaStream_t s, Mat
 }
 
 // ---- pow ------------------------------------------------------------------------------------------
-int pow_matrix(const Matrix &A, int n, bool prune, cudaStream_t s, Matrix **out) {
+// The intermediate powers are internal matrices; the result becomes the caller's.
+static int pow_internal(const Matrix &A, int n, bool prune, cudaStream_t s, Matrix **out) {
     if (A.prec == DIAQ_C128F2) return set_error(DIAQ_ERR_UNSUPPORTED, "pow: convert a c128f2 matrix to c128 first");
     if (n < 0) return set_error(DIAQ_ERR_INVALID, "pow: negative exponent not supported");
     if (A.rows != A.cols) return set_error(DIAQ_ERR_INVALID, "pow: matrix must be square");
-    if (n == 0) return identity(A.rows, A.prec, s, out);
+    if (n == 0) return identity(A.rows, A.prec, s, out, true);
     Matrix *base = nullptr;
-    DQ_TRY(copy_as(A, A.prec, s, &base));
+    DQ_TRY(copy_as(A, A.prec, s, &base, true));
     if (n == 1) {
         *out = base;
         return DIAQ_OK;
@@ -344,7 +345,7 @@ int pow_matrix(const Matrix &A, int n, bool prune, cudaStream_t s, Matrix **out)
     if ((e0 & (e0 - 1)) == 0) {  // 2^s: s squarings
         for (uint64_t e = e0; e > 1; e >>= 1) {
             Matrix *sq = nullptr;
-            const int st = spgemm(*base, *base, prune, s, &sq);
+            const int st = spgemm(*base, *base, prune, s, &sq, true);
             destroy(base);
             if (st != DIAQ_OK) return st;
             base = sq;
@@ -360,17 +361,17 @@ int pow_matrix(const Matrix &A, int n, bool prune, cudaStream_t s, Matrix **out)
         if (e & 1ULL) {
             Matrix *r2 = nullptr;
             if (result) {
-                st = spgemm(*result, *base, prune, s, &r2);
+                st = spgemm(*result, *base, prune, s, &r2, true);
                 destroy(result);
             } else {
-                st = copy_as(*base, base->prec, s, &r2);
+                st = copy_as(*base, base->prec, s, &r2, true);
             }
             result = r2;
         }
         e >>= 1ULL;
         if (e && st == DIAQ_OK) {
             Matrix *b2 = nullptr;
-            st = spgemm(*base, *base, prune, s, &b2);
+            st = spgemm(*base, *base, prune, s, &b2, true);
             destroy(base);
             base = b2;
         }
@@ -384,28 +385,40 @@ int pow_matrix(const Matrix &A, int n, bool prune, cudaStream_t s, Matrix **out)
     return DIAQ_OK;
 }
 
+int pow_matrix(const Matrix &A, int n, bool prune, cudaStream_t s, Matrix **out) {
+    Matrix *P = nullptr;
+    DQ_TRY(pow_internal(A, n, prune, s, &P));
+    const int st = publish(*P);
+    if (st != DIAQ_OK) {
+        destroy(P);
+        return st;
+    }
+    *out = P;
+    return DIAQ_OK;
+}
+
 // ---- exponential -----------------------------------------------------------------------------------
 static int scaling_exponent(double norm, double t_abs, double cutoff) {
     const double scaled = t_abs * norm + 1e-12;  // src/spME.cpp:256-262
     return scaled > cutoff ? (int)std::ceil(std::log2(scaled / cutoff)) : 0;
 }
 
-// Taylor series of exp(X) with X prepared by the caller; term_k = term_{k-1} X / k.
+// Taylor series of exp(X) with X prepared by the caller; term_k = term_{k-1} X / k.  *out is internal.
 static int taylor(const Matrix &X, int max_it, double tol, bool prune, cudaStream_t s, Matrix **out, int *terms) {
     Matrix *result = nullptr, *term = nullptr;
-    DQ_TRY(identity(X.rows, X.prec, s, &result));
-    int st = identity(X.rows, X.prec, s, &term);
+    DQ_TRY(identity(X.rows, X.prec, s, &result, true));
+    int st = identity(X.rows, X.prec, s, &term, true);
     int k = 0;
     for (k = 1; k <= max_it && st == DIAQ_OK; ++k) {
         Matrix *t2 = nullptr;
-        st = spgemm(*term, X, prune, s, &t2);
+        st = spgemm(*term, X, prune, s, &t2, true);
         destroy(term);
         term = t2;
         if (st != DIAQ_OK) break;
         st = scale(*term, kDivInt, (double)k, s);
         if (st != DIAQ_OK) break;
         Matrix *r2 = nullptr;
-        st = union_add(*result, *term, 1.0, s, &r2);
+        st = union_add(*result, *term, 1.0, s, &r2, true);
         if (st != DIAQ_OK) break;
         destroy(result);
         result = r2;
@@ -437,7 +450,7 @@ int expm_negative(const Matrix &A, double t, int max_it, double cutoff, double t
     const double ts = std::ldexp(t, -sc);
     const double tol_s = std::max(1e-15, tol * std::ldexp(1.0, -sc));
     Matrix *X = nullptr;
-    DQ_TRY(copy_as(A, A.prec, s, &X));
+    DQ_TRY(copy_as(A, A.prec, s, &X, true));
     int st = scale(*X, kTimesI, -ts, s);  // X = -i t_s A
     Matrix *U = nullptr;
     int terms = 0;
@@ -464,7 +477,7 @@ int expm(const Matrix &A, int max_it, double cutoff, double tol, bool prune, cud
     const double inv = std::ldexp(1.0, -sc);
     const double tol_s = std::max(1e-15, tol * inv);
     Matrix *X = nullptr;
-    DQ_TRY(copy_as(A, A.prec, s, &X));
+    DQ_TRY(copy_as(A, A.prec, s, &X, true));
     int st = scale(*X, kTimesReal, inv, s);
     Matrix *U = nullptr;
     if (st == DIAQ_OK) st = taylor(*X, max_it, tol_s, prune, s, &U, nullptr);

@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <unordered_set>
 
@@ -38,6 +39,92 @@ size_t alloc_limit() {
     char *end = nullptr;
     const unsigned long long n = std::strtoull(v, &end, 10);
     return (end && *end == '\0') ? (size_t)n : SIZE_MAX;
+}
+
+// ---- memory pools ------------------------------------------------------------------------------
+// One per device, made on first use and kept until the process exits.  `s` is a stream of its own for
+// freeing memory that nothing uses any more: no order with anyone else's work is implied.
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t s = nullptr;
+    int64_t matrices = 0;   // alive on the device
+};
+constexpr int kMaxDevices = 64;
+static std::mutex g_pool_mu;
+static DevicePool g_pools[kMaxDevices];
+
+static cudaError_t pool_of(int dev, DevicePool **out) {   // g_pool_mu held, dev current
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    DevicePool &P = g_pools[dev];
+    *out = &P;
+    if (P.pool) return cudaSuccess;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kPoolKeep;
+    e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e == cudaSuccess && !P.s) e = cudaStreamCreateWithFlags(&P.s, cudaStreamNonBlocking);
+    if (e != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return e;
+    }
+    P.pool = pool;
+    return cudaSuccess;
+}
+
+cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        DevicePool *P = nullptr;
+        e = pool_of(dev, &P);
+        if (e != cudaSuccess) return e;
+        pool = P->pool;
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
+void pool_free_idle(void *p, int device) {
+    cudaStream_t s = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        if (device >= 0 && device < kMaxDevices) s = g_pools[device].s;
+    }
+    if (p) cudaFreeAsync(p, s);
+}
+
+bool alloc_failed(cudaError_t e) {
+    if (e != cudaErrorMemoryAllocation) return false;
+    cudaGetLastError();
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    bool any = false;
+    for (auto &P : g_pools)
+        if (P.pool) {
+            uint64_t kept = 0, used = 0;
+            cudaMemPoolGetAttribute(P.pool, cudaMemPoolAttrReservedMemCurrent, &kept);
+            cudaMemPoolGetAttribute(P.pool, cudaMemPoolAttrUsedMemCurrent, &used);
+            any = (cudaMemPoolTrimTo(P.pool, 0) == cudaSuccess && kept > used) || any;
+        }
+    return any;
+}
+
+// Counts the matrices alive on a device; the pool gives back what it keeps when the last one goes.
+static void count_matrix(int device, int by) {
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    DevicePool &P = g_pools[device];
+    P.matrices += by;
+    if (P.matrices == 0 && P.pool) {
+        cudaStreamSynchronize(P.s);   // the frees have landed
+        cudaMemPoolTrimTo(P.pool, 0);
+    }
 }
 
 int num_sms() {
@@ -107,33 +194,97 @@ int plan_layout(Matrix &M, int64_t rows, int64_t cols, int32_t nd, const int32_t
     return DIAQ_OK;
 }
 
+// The metadata block: DiagMeta records and, behind them, the zero-tile mask's storage, so that SpMV
+// calls never allocate (it is filled on first use).
+static size_t meta_bytes(const Matrix &M) { return (sizeof(DiagMeta) * (size_t)M.nd + 255) / 256 * 256; }
+
+// The planes come from the pool.  A caller's matrix has its metadata block from cudaMalloc: freeing
+// that waits for all work on the device (as freeing the planes so would), after which the planes may
+// go back to the pool whatever streams the matrix was used on.
 int allocate(Matrix &M, cudaStream_t s, bool zero) {
     cudaGetDevice(&M.device);
-    const size_t bytes = (size_t)M.capacity * M.elem();
-    DQ_CUDA(dev_malloc(&M.re, bytes));
-    DQ_CUDA(dev_malloc(&M.im, bytes));
+    const size_t bytes = (size_t)M.capacity * M.elem(), block = meta_bytes(M) + tile_mask_bytes(M.nd, M.rows);
+    if (M.nd == 0 && !M.internal) {   // no metadata block: plain allocations
+        DQ_CUDA(dev_malloc(&M.re, bytes));
+        DQ_CUDA(dev_malloc(&M.im, bytes));
+    } else {
+        DQ_CUDA(dev_malloc_async(&M.re, bytes, s));
+        DQ_CUDA(dev_malloc_async(&M.im, bytes, s));
+    }
     if (zero) {
         DQ_CUDA(cudaMemsetAsync(M.re, 0, bytes, s));
         DQ_CUDA(cudaMemsetAsync(M.im, 0, bytes, s));
     }
     if (M.nd > 0) {
-        // metadata and, behind it, the zero-tile mask's storage, so that SpMV calls never allocate (it
-        // is filled on first use)
-        const size_t mb = (sizeof(DiagMeta) * (size_t)M.nd + 255) / 256 * 256;
-        DQ_CUDA(dev_malloc(&M.d_meta, mb + tile_mask_bytes(M.nd, M.rows)));
-        M.tmask = (uint32_t *)((uint8_t *)M.d_meta + mb);
-        DQ_CUDA(cudaMemcpyAsync(M.d_meta, M.meta.data(), sizeof(DiagMeta) * M.nd,
-                                cudaMemcpyHostToDevice, s));
+        if (M.internal)
+            DQ_CUDA(dev_malloc_async(&M.d_meta, block, s));
+        else
+            DQ_CUDA(dev_malloc(&M.d_meta, block));
+        M.tmask = (uint32_t *)((uint8_t *)M.d_meta + meta_bytes(M));
+        DQ_CUDA(cudaMemcpyAsync(M.d_meta, M.meta.data(), sizeof(DiagMeta) * M.nd, cudaMemcpyHostToDevice, s));
         // the host vector may be reallocated later; finish the copy before returning
         DQ_CUDA(cudaStreamSynchronize(s));
     }
     return DIAQ_OK;
 }
 
+int publish(Matrix &M) {
+    if (!M.internal) return DIAQ_OK;
+    const size_t block = meta_bytes(M) + tile_mask_bytes(M.nd, M.rows);
+    DiagMeta *d = nullptr;
+    void *re = nullptr, *im = nullptr;
+    if (M.nd > 0) {
+        DQ_CUDA(dev_malloc(&d, block));
+    } else {   // as allocate() has it
+        const size_t bytes = (size_t)M.capacity * M.elem();
+        DQ_CUDA(dev_malloc(&re, bytes));
+        cudaError_t e = dev_malloc(&im, bytes);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(re, M.re, bytes, cudaMemcpyDeviceToDevice, M.stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(im, M.im, bytes, cudaMemcpyDeviceToDevice, M.stream);
+        if (e != cudaSuccess) {
+            cudaFree(re);
+            cudaFree(im);
+            return cuda_status(e, "publish", __FILE__, __LINE__);
+        }
+    }
+    cudaError_t e = cudaSuccess;
+    if (d) e = cudaMemcpyAsync(d, M.d_meta, block, cudaMemcpyDeviceToDevice, M.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(M.stream);
+    if (e != cudaSuccess) {
+        cudaFree(d);
+        cudaFree(re);
+        cudaFree(im);
+        return cuda_status(e, "publish", __FILE__, __LINE__);
+    }
+    if (d) {
+        cudaFreeAsync(M.d_meta, M.stream);
+        M.d_meta = d;
+        M.tmask = (uint32_t *)((uint8_t *)d + meta_bytes(M));
+    } else {
+        cudaFreeAsync(M.re, M.stream);
+        cudaFreeAsync(M.im, M.stream);
+        M.re = re;
+        M.im = im;
+    }
+    M.internal = false;
+    return DIAQ_OK;
+}
+
 void release(Matrix &M) {
-    if (M.re) cudaFree(M.re);
-    if (M.im) cudaFree(M.im);
-    if (M.d_meta) cudaFree(M.d_meta);
+    if (M.internal) {
+        if (M.re) cudaFreeAsync(M.re, M.stream);
+        if (M.im) cudaFreeAsync(M.im, M.stream);
+        if (M.d_meta) cudaFreeAsync(M.d_meta, M.stream);
+    } else if (M.nd > 0) {
+        // (a matrix whose allocation failed half-way was used by nothing but its own stream's fills)
+        if (M.d_meta) cudaFree(M.d_meta);
+        else cudaStreamSynchronize(M.stream);
+        pool_free_idle(M.re, M.device);
+        pool_free_idle(M.im, M.device);
+    } else {
+        cudaFree(M.re);
+        cudaFree(M.im);
+    }
     M.re = M.im = nullptr;
     M.d_meta = nullptr;
     M.tmask = nullptr;
@@ -141,11 +292,15 @@ void release(Matrix &M) {
 }
 
 int make_zero(int64_t rows, int64_t cols, int32_t nd, const int32_t *off, int prec,
-              cudaStream_t s, Matrix **out, bool zero) {
+              cudaStream_t s, Matrix **out, bool zero, bool internal) {
     if (prec != DIAQ_C128 && prec != DIAQ_C64 && prec != DIAQ_C128F2)
         return set_error(DIAQ_ERR_INVALID, "precision must be DIAQ_C128, DIAQ_C64 or DIAQ_C128F2");
     Matrix *M = new diaq_matrix_s();
+    cudaGetDevice(&M->device);
+    count_matrix(M->device, 1);
     M->prec = prec;
+    M->internal = internal;
+    M->stream = s;
     int st = plan_layout(*M, rows, cols, nd, off);
     if (st == DIAQ_OK) st = allocate(*M, s, zero);
     if (st != DIAQ_OK) {
@@ -184,6 +339,7 @@ int zero_gaps(const Matrix &M, cudaStream_t s) {
 void destroy(Matrix *M) {
     if (!M) return;
     release(*M);
+    count_matrix(M->device, -1);
     delete static_cast<diaq_matrix_s *>(M);
 }
 
@@ -308,9 +464,9 @@ static int remap(const Matrix &src, Matrix &dst, const int32_t *d_map, cudaStrea
     return DIAQ_OK;
 }
 
-int copy_as(const Matrix &A, int prec, cudaStream_t s, Matrix **out) {
+int copy_as(const Matrix &A, int prec, cudaStream_t s, Matrix **out, bool internal) {
     Matrix *C = nullptr;
-    DQ_TRY(make_zero(A.rows, A.cols, A.nd, A.off.data(), prec, s, &C));
+    DQ_TRY(make_zero(A.rows, A.cols, A.nd, A.off.data(), prec, s, &C, true, internal));
     int st = DIAQ_OK;
     if (A.prec == DIAQ_C128F2 && prec == DIAQ_C128F2) {
         cudaError_t e = cudaMemcpyAsync(C->re, A.re, A.capacity * A.elem(), cudaMemcpyDeviceToDevice, s);
@@ -321,7 +477,7 @@ int copy_as(const Matrix &A, int prec, cudaStream_t s, Matrix **out) {
     } else {
         st = remap(A, *C, nullptr, s);
     }
-    if (st == DIAQ_OK) {
+    if (st == DIAQ_OK && !internal) {
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) st = cuda_status(e, "cudaStreamSynchronize", __FILE__, __LINE__);
     }
@@ -333,12 +489,12 @@ int copy_as(const Matrix &A, int prec, cudaStream_t s, Matrix **out) {
     return DIAQ_OK;
 }
 
-int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out) {
+int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out, bool internal) {
     if (A.prec == DIAQ_C128F2) return set_error(DIAQ_ERR_UNSUPPORTED, "prune: convert a c128f2 matrix to c128 first");
     std::vector<int32_t> flag(A.nd, 1);
     if (A.nd > 0) {
         int32_t *d_flag = nullptr;
-        DQ_CUDA(dev_malloc(&d_flag, sizeof(int32_t) * A.nd));
+        DQ_CUDA(dev_malloc_async(&d_flag, sizeof(int32_t) * A.nd, s));
         const int grid = (int)std::min<int64_t>(A.nd, 65535);
         if (A.prec == DIAQ_C128)
             nonzero_kernel<double><<<grid, 256, 0, s>>>(A.d_meta, A.nd, (const double *)A.re, (const double *)A.im, d_flag);
@@ -347,7 +503,7 @@ int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out) {
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(flag.data(), d_flag, sizeof(int32_t) * A.nd, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        cudaFree(d_flag);
+        cudaFreeAsync(d_flag, s);
         if (e != cudaSuccess) return cuda_status(e, "prune flags", __FILE__, __LINE__);
     }
     std::vector<int32_t> keep_off, map;
@@ -357,16 +513,16 @@ int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out) {
             map.push_back(k);
         }
     Matrix *C = nullptr;
-    DQ_TRY(make_zero(A.rows, A.cols, (int32_t)keep_off.size(), keep_off.data(), A.prec, s, &C));
+    DQ_TRY(make_zero(A.rows, A.cols, (int32_t)keep_off.size(), keep_off.data(), A.prec, s, &C, true, internal));
     int st = DIAQ_OK;
     if (C->nd > 0) {
         int32_t *d_map = nullptr;
-        cudaError_t e = dev_malloc(&d_map, sizeof(int32_t) * C->nd);
+        cudaError_t e = dev_malloc_async(&d_map, sizeof(int32_t) * C->nd, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_map, map.data(), sizeof(int32_t) * C->nd, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) st = remap(A, *C, d_map, s);
         else st = cuda_status(e, "prune map", __FILE__, __LINE__);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (d_map) cudaFree(d_map);
+        if (d_map) cudaFreeAsync(d_map, s);
         if (st == DIAQ_OK && e != cudaSuccess) st = cuda_status(e, "prune copy", __FILE__, __LINE__);
     }
     if (st != DIAQ_OK) {

@@ -19,11 +19,11 @@
 namespace diaq_gb300 {
 
 // ---- dry-run -----------------------------------------------------------------------------------
-__global__ void mark_pairs_kernel(const int32_t *__restrict__ offA, int ndA, const int32_t *__restrict__ offB,
+__global__ void mark_pairs_kernel(const DiagMeta *__restrict__ mA, int ndA, const DiagMeta *__restrict__ mB,
                                   int ndB, int64_t lo, int64_t hi, uint8_t *__restrict__ flags) {
     const int64_t n = (int64_t)ndA * ndB;
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t dc = (int64_t)offA[p / ndB] + offB[p % ndB];
+        const int64_t dc = (int64_t)mA[p / ndB].off + mB[p % ndB].off;
         if (dc >= lo && dc <= hi) flags[dc - lo] = 1;  // benign race: every writer stores 1
     }
 }
@@ -51,8 +51,8 @@ __global__ void count_tiles_kernel(const uint8_t *__restrict__ flags, int64_t n,
     }
 }
 
-// Exclusive scan of the tile counts in one block (loops over chunks); total at [ntiles].
-__global__ void scan_tiles_kernel(int32_t *__restrict__ tile_count, int64_t ntiles) {
+// Exclusive scan of the tile counts in one block (loops over chunks); the total goes to *total.
+__global__ void scan_tiles_kernel(int32_t *__restrict__ tile_count, int64_t ntiles, int32_t *__restrict__ total) {
     __shared__ int32_t buf[1024];
     __shared__ int32_t carry;
     if (threadIdx.x == 0) carry = 0;
@@ -73,7 +73,7 @@ __global__ void scan_tiles_kernel(int32_t *__restrict__ tile_count, int64_t ntil
         if (threadIdx.x == 1023) carry += buf[1023];
         __syncthreads();
     }
-    if (threadIdx.x == 0) tile_count[ntiles] = carry;
+    if (threadIdx.x == 0) *total = carry;
 }
 
 // Write the offsets of the set flags, ascending.
@@ -109,41 +109,41 @@ int spgemm_symbolic(const Matrix &A, const Matrix &B, std::vector<int32_t> &offC
     const int64_t lo = -(A.rows - 1), hi = B.cols - 1;
     const int64_t range = hi - lo + 1;
     const int64_t ntiles = (range + kScanTile - 1) / kScanTile;
-    // one scratch allocation: flags | tile counts | offsets A | offsets B | output
+    // one scratch allocation: flags | tile counts | output (the count, then the offsets)
     const size_t fbytes = (size_t)((range + 15) / 16 * 16);
     const size_t tbytes = sizeof(int32_t) * (size_t)(ntiles + 1);
-    const size_t abytes = sizeof(int32_t) * A.nd, bbytes = sizeof(int32_t) * B.nd;
     const int64_t maxout = std::min<int64_t>((int64_t)A.nd * B.nd, range);
-    const size_t obytes = sizeof(int32_t) * (size_t)maxout;
+    const size_t obytes = sizeof(int32_t) * (size_t)(maxout + 1);
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t total = up(fbytes) + up(tbytes) + up(abytes) + up(bbytes) + up(obytes);
     uint8_t *scratch = nullptr;
-    DQ_CUDA(dev_malloc_async(&scratch, total, s));
+    DQ_CUDA(dev_malloc_async(&scratch, up(fbytes) + up(tbytes) + up(obytes), s));
     uint8_t *flags = scratch;
     int32_t *tiles = (int32_t *)(scratch + up(fbytes));
-    int32_t *dA = (int32_t *)((uint8_t *)tiles + up(tbytes));
-    int32_t *dB = (int32_t *)((uint8_t *)dA + up(abytes));
-    int32_t *dout = (int32_t *)((uint8_t *)dB + up(bbytes));
+    int32_t *dout = (int32_t *)((uint8_t *)tiles + up(tbytes));
     int st = DIAQ_OK;
     cudaError_t e = cudaMemsetAsync(flags, 0, fbytes, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dA, A.off.data(), abytes, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dB, B.off.data(), bbytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
         const int64_t pairs = (int64_t)A.nd * B.nd;
         const int grid = (int)std::min<int64_t>((pairs + 255) / 256, 8 * num_sms());
-        mark_pairs_kernel<<<grid, 256, 0, s>>>(dA, A.nd, dB, B.nd, lo, hi, flags);
+        mark_pairs_kernel<<<grid, 256, 0, s>>>(A.d_meta, A.nd, B.d_meta, B.nd, lo, hi, flags);
         count_tiles_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(flags, range, tiles);
-        scan_tiles_kernel<<<1, 1024, 0, s>>>(tiles, ntiles);
-        compact_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(flags, range, lo, tiles, dout);
+        scan_tiles_kernel<<<1, 1024, 0, s>>>(tiles, ntiles, dout);
+        compact_kernel<<<(unsigned)ntiles, kScanThreads, 0, s>>>(flags, range, lo, tiles, dout + 1);
         e = cudaGetLastError();
     }
-    int32_t count = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&count, tiles + ntiles, sizeof(int32_t), cudaMemcpyDeviceToHost, s);
+    // the count with every offset there can be in one copy, unless those are many
+    const int64_t first = maxout <= (1 << 18) ? maxout + 1 : 1;
+    std::vector<int32_t> got((size_t)first, 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(got.data(), dout, sizeof(int32_t) * (size_t)first, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess && count > 0) {
-        offC.resize(count);
-        e = cudaMemcpyAsync(offC.data(), dout, sizeof(int32_t) * count, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && got[0] > 0) {
+        if (first > 1) {
+            offC.assign(got.begin() + 1, got.begin() + 1 + got[0]);
+        } else {
+            offC.resize((size_t)got[0]);
+            e = cudaMemcpyAsync(offC.data(), dout + 1, sizeof(int32_t) * offC.size(), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        }
     }
     if (e != cudaSuccess) st = cuda_status(e, "spgemm dry-run", __FILE__, __LINE__);
     cudaFreeAsync(scratch, s);
@@ -195,6 +195,39 @@ __global__ void spgemm_pairs_kernel(const DiagMeta *__restrict__ mA, int ndA, co
         }
         if (!fill && lane == 0) cnt[c] = n;
     }
+}
+
+// Dense offset -> slot map (entries without a diagonal stay -1).
+__global__ void slot_map_kernel(const DiagMeta *__restrict__ meta, int nd, int64_t dmin, int32_t *__restrict__ map) {
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nd; k += gridDim.x * blockDim.x) map[meta[k].off - dmin] = k;
+}
+
+// start[c] = cnt[0] + ... + cnt[c - 1], c = 0 .. n, by one block.
+__global__ void __launch_bounds__(1024)
+    scan_counts_kernel(const int32_t *__restrict__ cnt, int n, int64_t *__restrict__ start) {
+    __shared__ int64_t part[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int64_t carry = 0;
+    for (int c0 = 0; c0 < n; c0 += 1024) {
+        const int c = c0 + (int)threadIdx.x;
+        const int64_t own = c < n ? cnt[c] : 0;
+        int64_t v = own;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        if (lane == 31) part[wid] = v;
+        __syncthreads();
+        int64_t before = 0, all = 0;
+        for (int w = 0; w < 32; ++w) {
+            if (w < wid) before += part[w];
+            all += part[w];
+        }
+        if (c < n) start[c] = carry + before + v - own;
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) start[n] = carry;
 }
 
 // Bits t0 .. t0 + n - 1 (n <= 8) of a mask row of mw words, bits outside it zero; all ones without a mask.
@@ -422,12 +455,9 @@ int spgemm_numeric(const Matrix &A, const Matrix &B, Matrix &C, cudaStream_t s) 
         return set_error(DIAQ_ERR_INVALID, "product: operands must have the same precision");
     C.tmask_ok = false;  // new values
     if (C.nd == 0 || C.rows == 0) return DIAQ_OK;
-    // dense offset -> slot map of B
     const int64_t bmin = -(B.rows - 1), bmax = B.cols - 1;
     const int64_t span = bmax - bmin + 1;
-    std::vector<int32_t> map((size_t)span, -1);
-    for (int32_t k = 0; k < B.nd; ++k) map[(size_t)(B.off[k] - bmin)] = k;
-    // scratch: B map, per-C counts, per-C starts
+    // scratch: dense offset -> slot map of B, per-C counts, per-C starts
     const size_t mbytes = sizeof(int32_t) * (size_t)span, cbytes = sizeof(int32_t) * (size_t)C.nd,
                  sbytes = sizeof(int64_t) * ((size_t)C.nd + 1);
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -437,23 +467,24 @@ int spgemm_numeric(const Matrix &A, const Matrix &B, Matrix &C, cudaStream_t s) 
     int32_t *dcnt = (int32_t *)(scratch + up(mbytes));
     int64_t *dstart = (int64_t *)(scratch + up(mbytes) + up(cbytes));
     int2 *dpairs = nullptr;
-    std::vector<int32_t> cnt((size_t)C.nd);
-    std::vector<int64_t> start((size_t)C.nd + 1, 0);
     const int pg = (int)std::max<int64_t>(1, std::min<int64_t>((C.nd + 3) / 4, 8 * num_sms()));
-    cudaError_t e = cudaMemcpyAsync(dmap, map.data(), mbytes, cudaMemcpyHostToDevice, s);
+    cudaError_t e = cudaMemsetAsync(dmap, 0xff, mbytes, s);
     if (e == cudaSuccess) {
+        slot_map_kernel<<<std::max(1, (B.nd + 255) / 256), 256, 0, s>>>(B.d_meta, B.nd, bmin, dmap);
         spgemm_pairs_kernel<<<pg, 128, 0, s>>>(A.d_meta, A.nd, B.d_meta, dmap, bmin, bmax, C.d_meta, C.nd, dcnt,
                                                nullptr, nullptr);
+        scan_counts_kernel<<<1, 1024, 0, s>>>(dcnt, C.nd, dstart);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), dcnt, cbytes, cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) {
-        for (int32_t c = 0; c < C.nd; ++c) start[(size_t)c + 1] = start[(size_t)c] + cnt[(size_t)c];
-        const int64_t npairs = start[(size_t)C.nd];
-        e = cudaMemcpyAsync(dstart, start.data(), sbytes, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = dev_malloc_async((void **)&dpairs, sizeof(int2) * (size_t)std::max<int64_t>(npairs, 1), s);
+    // room for every pair of slots, or -- where that is much -- for as many as there are
+    size_t pbytes = sizeof(int2) * (size_t)A.nd * (size_t)B.nd;
+    if (pbytes > std::min<size_t>((size_t)64 << 20, alloc_limit())) {
+        int64_t npairs = 0;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&npairs, dstart + C.nd, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        pbytes = sizeof(int2) * (size_t)npairs;
     }
+    if (e == cudaSuccess) e = dev_malloc_async((void **)&dpairs, std::max<size_t>(pbytes, sizeof(int2)), s);
     if (e == cudaSuccess) {
         spgemm_pairs_kernel<<<pg, 128, 0, s>>>(A.d_meta, A.nd, B.d_meta, dmap, bmin, bmax, C.d_meta, C.nd, nullptr,
                                                dstart, dpairs);
@@ -485,15 +516,14 @@ int spgemm_numeric(const Matrix &A, const Matrix &B, Matrix &C, cudaStream_t s) 
                 (const float *)B.im, C.d_meta, C.nd, chunk, dstart, dpairs, (float *)C.re, (float *)C.im, ka, wa, pa, kb, wb, pb);
         e = cudaGetLastError();
     }
-    // the host vectors must outlive the async copies
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (dpairs) cudaFreeAsync(dpairs, s);
     cudaFreeAsync(scratch, s);
     if (e != cudaSuccess) return cuda_status(e, "spgemm numeric", __FILE__, __LINE__);
     return DIAQ_OK;
 }
 
-int spgemm(const Matrix &A, const Matrix &B, bool prune, cudaStream_t s, Matrix **out) {
+// internal: see Matrix::internal; else the result is the caller's and complete on return.
+int spgemm(const Matrix &A, const Matrix &B, bool prune, cudaStream_t s, Matrix **out, bool internal) {
     if (A.prec == DIAQ_C128F2) return set_error(DIAQ_ERR_UNSUPPORTED, "product: convert a c128f2 matrix to c128 first");
     if (A.cols != B.rows) return set_error(DIAQ_ERR_INVALID, "diaQMatrix product_cuda: dimension mismatch.");
     if (A.prec != B.prec) return set_error(DIAQ_ERR_INVALID, "product: operands must have the same precision");
@@ -501,16 +531,20 @@ int spgemm(const Matrix &A, const Matrix &B, bool prune, cudaStream_t s, Matrix 
     DQ_TRY(spgemm_symbolic(A, B, offC, s));
     Matrix *C = nullptr;
     // the numeric pass writes every stored value of C: only the gaps around them need zeroing
-    DQ_TRY(make_zero(A.rows, B.cols, (int32_t)offC.size(), offC.data(), A.prec, s, &C, false));
+    DQ_TRY(make_zero(A.rows, B.cols, (int32_t)offC.size(), offC.data(), A.prec, s, &C, false, internal || prune));
     int st = spgemm_numeric(A, B, *C, s);
     if (st == DIAQ_OK) st = zero_gaps(*C, s);
     if (st == DIAQ_OK && prune) {
         Matrix *P = nullptr;
-        st = prune_matrix(*C, s, &P);
+        st = prune_matrix(*C, s, &P, internal);
         if (st == DIAQ_OK) {
             destroy(C);
             C = P;
         }
+    }
+    if (st == DIAQ_OK && !internal) {
+        const cudaError_t e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) st = cuda_status(e, "spgemm", __FILE__, __LINE__);
     }
     if (st != DIAQ_OK) {
         destroy(C);
@@ -539,13 +573,15 @@ int diaq_spgemm_symbolic(diaq_matrix_t A, diaq_matrix_t B, int32_t *offsets_out,
 
 int diaq_spgemm_numeric(diaq_matrix_t A, diaq_matrix_t B, diaq_matrix_t C, void *stream) {
     if (!A || !B || !C) return set_error(DIAQ_ERR_INVALID, "NULL argument");
-    return spgemm_numeric(*A, *B, *C, (cudaStream_t)stream);
+    DQ_TRY(spgemm_numeric(*A, *B, *C, (cudaStream_t)stream));
+    DQ_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    return DIAQ_OK;
 }
 
 int diaq_spgemm(diaq_matrix_t A, diaq_matrix_t B, int prune, void *stream, diaq_matrix_t *C) {
     if (!A || !B || !C) return set_error(DIAQ_ERR_INVALID, "NULL argument");
     Matrix *M = nullptr;
-    DQ_TRY(spgemm(*A, *B, prune != 0, (cudaStream_t)stream, &M));
+    DQ_TRY(spgemm(*A, *B, prune != 0, (cudaStream_t)stream, &M, false));
     *C = handle(M);
     return DIAQ_OK;
 }

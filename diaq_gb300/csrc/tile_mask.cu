@@ -97,7 +97,8 @@ const uint32_t *cached_tile_mask(const Matrix &A, cudaStream_t s) {
         return nullptr;
     }
     if (A.tmask_ok) return A.tmask;
-    if (build_tile_mask(A, A.tmask, s) != DIAQ_OK || cudaStreamSynchronize(s) != cudaSuccess) {
+    // (an internal matrix is used on its own stream only)
+    if (build_tile_mask(A, A.tmask, s) != DIAQ_OK || (!A.internal && cudaStreamSynchronize(s) != cudaSuccess)) {
         cudaGetLastError();
         return nullptr;
     }
