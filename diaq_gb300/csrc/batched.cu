@@ -58,6 +58,7 @@ struct BatchInst {
     int64_t n_pad;   // interleaved: rows padded to a multiple of 32
     const uint32_t *tmask;  // zero-tile mask of the matrix (rebuilt at every run), mw words per diagonal
     int64_t mw;
+    const int *has_im;      // whether the matrix holds an imaginary part (taken with the mask)
     double tau;      // dt / 2^s
     double *pr, *pi; // states, leading dimension rows
     void *var, *vai, *vbr, *vbi, *hr, *hi, *lr, *li;  // T work vectors, leading dimension rows
@@ -313,9 +314,11 @@ __device__ __forceinline__ void batched_il_item(const BatchInst &I, int4 *sq, in
     const int g = wid % groups;
     const int64_t r = r0 + (int64_t)(wid / groups) * 32 + lane;
     float accr[G], acci[G];
+    const float *are = (const float *)I.are, *aim = (const float *)I.aim;
+    // no imaginary part in the matrix: half the loads and multiply-adds (one chunk of metadata only)
+    const bool real = I.nd <= kMetaChunk && !*I.has_im;
 #pragma unroll
     for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;
-    const float *are = (const float *)I.are, *aim = (const float *)I.aim;
     for (int c0 = 0; c0 < I.nd; c0 += kMetaChunk) {
         const int cn = min(kMetaChunk, I.nd - c0);
         __syncthreads();
@@ -333,11 +336,17 @@ __device__ __forceinline__ void batched_il_item(const BatchInst &I, int4 *sq, in
             const int j = lane * 8 + wid;
             if (j < cn) {
                 const int4 q = sq[j];
-                prefetch_tiles_l2(are, aim, sb[j], (int64_t)q.y, (int64_t)q.z,
+                prefetch_tiles_l2(are, aim, real, sb[j], (int64_t)q.y, (int64_t)q.z,
                                   block_tile_bits((uint32_t)q.w, r0, 8 / groups), r0);
             }
         }
         if (r >= I.rows) continue;
+        if (real) {
+            il_accumulate32<G, false, true>(sq, sb, cn, (int)r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+            if (!il_nonfinite<G>(accr, acci)) continue;
+#pragma unroll
+            for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;   // not finite: sum again, in full
+        }
         il_accumulate32<G>(sq, sb, cn, (int)r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
     }
     if (r >= I.rows) return;
@@ -395,6 +404,7 @@ struct Batch {
     int items_il = -1;                // il_on of the current item lists
     void *work = nullptr;
     uint32_t *masks = nullptr;        // zero-tile masks of every instance's matrix
+    int *has_im = nullptr;            // ... and whether it holds an imaginary part
     std::vector<const Matrix *> mats;
     cudaStream_t s = nullptr;         // capture stream
     SpmvCfg cfg{8, 0};
@@ -744,7 +754,9 @@ int diaq_batch_create(int n_inst, const diaq_matrix_t *H, const int *nrhs, doubl
     if (e == cudaSuccess) e = dev_malloc(&B->work, work_bytes + 256);
     size_t mask_words = 0;
     for (int i = 0; i < n_inst; ++i) mask_words += tile_mask_bytes(H[i]->nd, H[i]->rows) / sizeof(uint32_t);
-    if (e == cudaSuccess) e = dev_malloc(&B->masks, sizeof(uint32_t) * std::max<size_t>(mask_words, 1));
+    // the masks and, behind them, one "has an imaginary part" flag per instance
+    if (e == cudaSuccess) e = dev_malloc(&B->masks, sizeof(uint32_t) * (mask_words + (size_t)n_inst));
+    B->has_im = (int *)B->masks + mask_words;
     if (e == cudaSuccess) e = dev_malloc(&B->d_inst, sizeof(BatchInst) * n_inst);
     if (e != cudaSuccess) {
         delete B;
@@ -765,6 +777,7 @@ int diaq_batch_create(int n_inst, const diaq_matrix_t *H, const int *nrhs, doubl
         I.il_ok = il_shape(i, I.sp, I.n_pad) ? 1 : 0;
         I.tmask = B->masks + mask_off;
         I.mw = tile_mask_words(H[i]->rows);
+        I.has_im = B->has_im + i;
         mask_off += tile_mask_bytes(H[i]->nd, H[i]->rows) / sizeof(uint32_t);
         B->mats.push_back(H[i]);
         const size_t vb = vec_bytes(i);
@@ -835,7 +848,9 @@ int diaq_batch_run(diaq_batch_t B, double dt, const int *substeps_log2, const in
     if (steps == 0) return DIAQ_OK;
     cudaStream_t user = (cudaStream_t)stream;
     // the matrices are the caller's: their zero-tile masks are taken afresh at every run
-    for (size_t i = 0; i < B->inst.size(); ++i) DQ_TRY(build_tile_mask(*B->mats[i], (uint32_t *)B->inst[i].tmask, user));
+    DQ_CUDA(cudaMemsetAsync(B->has_im, 0, sizeof(int) * B->inst.size(), user));
+    for (size_t i = 0; i < B->inst.size(); ++i)
+        DQ_TRY(build_tile_mask(*B->mats[i], (uint32_t *)B->inst[i].tmask, user, B->has_im + i));
     DQ_CUDA(cudaStreamSynchronize(user));
     std::vector<int> key(substeps_log2, substeps_log2 + B->inst.size());
     key.insert(key.end(), m, m + B->inst.size());

@@ -408,7 +408,11 @@ __global__ void __launch_bounds__(kSpmvThreads)
 //   instead of 67.5 M instructions per launch, 93.1 -> 91.1 us per 8-state term.
 // - The Horner epilogue's middle and last steps are separate instantiations (EpiHornerT<0> and
 //   <1>): the middle steps' kernel holds no float64 code.
-template <class Epi, int G, int MINB>
+// - REAL: the matrix has no imaginary part (spin chains without Y fields), so the loop loads one plane
+//   and runs half the multiply-adds: 95 -> 84 us per 8-state Horner term of a step on the 20-qubit chain,
+//   where issue is now at 50 %, L1 at 58 % and DRAM at 32 % of their peaks.  A row whose sums are
+//   not finite is summed again with both planes (one chunk of metadata: the launcher sees to it).
+template <class Epi, int G, int MINB, bool REAL>
 __global__ void __launch_bounds__(kSpmvThreads, MINB)
     dia_spmv_il32_kernel(const DiagMeta *__restrict__ meta, int nd, const float *__restrict__ are,
                          const float *__restrict__ aim, int rows, const float *__restrict__ xr,
@@ -426,8 +430,6 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
     const int row0 = bi * (8 / groups) * 32;
     const int r = row0 + (wid / groups) * 32 + lane;
     float accr[G], acci[G];
-#pragma unroll
-    for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;
     bool tile = false;
     if constexpr (kTile) {
         tile = epi.reads_psi() && r < rows;
@@ -456,6 +458,8 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
         prefetch_l2(xr + at, bytes);
         prefetch_l2(xi + at, bytes);
     }
+#pragma unroll
+    for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;
     for (int c0 = 0; c0 < nd; c0 += kMetaChunk) {
         const int cn = min(kMetaChunk, nd - c0);
         __syncthreads();
@@ -472,12 +476,19 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
             const int i = lane * 8 + wid;
             if (i < cn) {
                 const int4 q = sq[i];
-                prefetch_tiles_l2(are, aim, sb[i], (int64_t)q.y, (int64_t)q.z,
+                prefetch_tiles_l2(are, aim, REAL, sb[i], (int64_t)q.y, (int64_t)q.z,
                                   block_tile_bits((uint32_t)q.w, row0, 8 / groups), row0);
             }
         }
         if (r >= rows) continue;
-        il_accumulate32<G, true>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+        il_accumulate32<G, true, REAL>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+        if constexpr (REAL) {   // one chunk (the launcher sees to it): not finite -- sum again, in full
+            if (il_nonfinite<G>(accr, acci)) {
+#pragma unroll
+                for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;
+                il_accumulate32<G, true, false>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+            }
+        }
     }
     if constexpr (kTile) asm volatile("cp.async.wait_all;" ::: "memory");
     if (r >= rows) return;
@@ -524,6 +535,7 @@ struct EvolvePlan {
     bool renorm = false;  // rescale every state to norm 1 (float64) after each step
     double *part = nullptr;  // renormalisation partial sums, nrhs * kNormBlocks
     uint32_t *tmask = nullptr;  // zero-tile mask of the matrix the term kernels read (Hc, or H for C128)
+    bool real = false;          // Hc holds no imaginary part
     int *err = nullptr;           // bounded waits of the bulk-copy kernels (variants 10, 11) record here
     int *err_host = nullptr;      // pinned copy of *err taken after each run
     cudaEvent_t err_ev = nullptr; // ... and the event that says it has landed
@@ -588,12 +600,17 @@ int launch_il(const EvolvePlan &P, const float *xr, const float *xi, const Epi &
         const int64_t mw = tile_mask_words(P.n);
         // blocks per SM: 5 (48 registers) for 8 states per thread -- 107.7 us per 8-state term on
         // the 20-qubit chain, against 112.9 at 6 (40 registers and spills)
-        if (eight)
-            dia_spmv_il32_kernel<Epi, 8, 5><<<g, kSpmvThreads, 0, P.s>>>(P.Hc->d_meta, P.Hc->nd, are, aim, (int)P.n, xr,
-                                                                         xi, P.tmask, mw, e);
+        const DiagMeta *md = P.Hc->d_meta;
+        const int nd = P.Hc->nd, n = (int)P.n;
+        const bool real = P.real && nd <= kMetaChunk;
+        if (eight && real)
+            dia_spmv_il32_kernel<Epi, 8, 5, true><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
+        else if (eight)
+            dia_spmv_il32_kernel<Epi, 8, 5, false><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
+        else if (real)
+            dia_spmv_il32_kernel<Epi, 4, 6, true><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
         else
-            dia_spmv_il32_kernel<Epi, 4, 6><<<g, kSpmvThreads, 0, P.s>>>(P.Hc->d_meta, P.Hc->nd, are, aim, (int)P.n, xr,
-                                                                         xi, P.tmask, mw, e);
+            dia_spmv_il32_kernel<Epi, 4, 6, false><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
         DQ_CUDA(cudaGetLastError());
         return DIAQ_OK;
     }
@@ -683,6 +700,7 @@ static int plan_create(const Matrix &H, int nrhs, int mode, EvolvePlan **out, co
     if (borrow) {
         P->Hc = share->Hc;
         P->tmask = share->tmask;
+        P->real = share->real;
         P->owns_hc = false;
     }
     if (st == DIAQ_OK && mode != DIAQ_EVOLVE_C128 && !borrow) st = copy_as(H, DIAQ_C64, P->s, &P->Hc);
@@ -702,9 +720,16 @@ static int plan_create(const Matrix &H, int nrhs, int mode, EvolvePlan **out, co
         // again at every run (its values may have changed)
         e = dev_malloc(&P->tmask, tile_mask_bytes(H.nd, H.rows));
         if (e != cudaSuccess) st = cuda_status(e, "evolve plan mask", __FILE__, __LINE__);
-        if (st == DIAQ_OK) st = build_tile_mask(P->Hc ? *P->Hc : H, P->tmask, P->s);
-        if (st == DIAQ_OK && (e = cudaStreamSynchronize(P->s)) != cudaSuccess)
-            st = cuda_status(e, "evolve plan mask", __FILE__, __LINE__);
+        // (the error flag doubles as the mask's "has an imaginary part" until the plan runs)
+        if (st == DIAQ_OK) st = build_tile_mask(P->Hc ? *P->Hc : H, P->tmask, P->s, P->err);
+        if (st == DIAQ_OK) {
+            int has_im = 1;
+            e = cudaMemcpyAsync(&has_im, P->err, sizeof(int), cudaMemcpyDeviceToHost, P->s);
+            if (e == cudaSuccess) e = cudaMemsetAsync(P->err, 0, sizeof(int), P->s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(P->s);
+            if (e != cudaSuccess) st = cuda_status(e, "evolve plan mask", __FILE__, __LINE__);
+            P->real = P->Hc && has_im == 0;
+        }
     }
     if (st != DIAQ_OK) {
         delete static_cast<diaq_evolve_s *>(P);

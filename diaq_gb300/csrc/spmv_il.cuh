@@ -174,11 +174,12 @@ __device__ __forceinline__ void il_load(int64_t c, int g0, int quads, const floa
         w.y[h] = __ldg(reinterpret_cast<const float4 *>(xi + at));
     }
 }
-// acc += (a + i b) * window, per state.  PACKED: two states per instruction (__ffma2_rn: each
-// lane one fmaf, the same rounding, so the same bits) -- 93.1 -> 91.1 us per 8-state Horner term
-// of the evolution plans; in the register-bounded batched kernels (six blocks per SM) it cost
-// 10 % (7,955 -> 7,122 states x steps/s), so they keep one FMA per state.
-template <int G, bool PACKED = false>
+// acc += (a + i b) * window, per state; RE / IM: with the real and the imaginary part of the matrix
+// value, or one of them alone (the other plane of the tile is zero).  PACKED: two states per
+// instruction (__ffma2_rn: each lane one fmaf, the same rounding, so the same bits) -- 93.1 -> 91.1 us
+// per 8-state Horner term of the evolution plans; in the register-bounded batched kernels (six blocks
+// per SM) it cost 10 % (7,955 -> 7,122 states x steps/s), so they keep one FMA per state.
+template <int G, bool PACKED = false, bool RE = true, bool IM = true>
 __device__ __forceinline__ void il_fma(float a, float b, const IlWindow<G> &w, float (&accr)[G], float (&acci)[G]) {
     if constexpr (PACKED) {
         const float2 aa = make_float2(a, a), bb = make_float2(b, b), nb = make_float2(-b, -b);
@@ -188,14 +189,22 @@ __device__ __forceinline__ void il_fma(float a, float b, const IlWindow<G> &w, f
             const float2 y01 = make_float2(w.y[h].x, w.y[h].y), y23 = make_float2(w.y[h].z, w.y[h].w);
             float2 r01 = make_float2(accr[4 * h], accr[4 * h + 1]), r23 = make_float2(accr[4 * h + 2], accr[4 * h + 3]);
             float2 i01 = make_float2(acci[4 * h], acci[4 * h + 1]), i23 = make_float2(acci[4 * h + 2], acci[4 * h + 3]);
-            r01 = __ffma2_rn(aa, x01, r01);
-            r23 = __ffma2_rn(aa, x23, r23);
-            r01 = __ffma2_rn(nb, y01, r01);
-            r23 = __ffma2_rn(nb, y23, r23);
-            i01 = __ffma2_rn(aa, y01, i01);
-            i23 = __ffma2_rn(aa, y23, i23);
-            i01 = __ffma2_rn(bb, x01, i01);
-            i23 = __ffma2_rn(bb, x23, i23);
+            if constexpr (RE) {
+                r01 = __ffma2_rn(aa, x01, r01);
+                r23 = __ffma2_rn(aa, x23, r23);
+            }
+            if constexpr (IM) {
+                r01 = __ffma2_rn(nb, y01, r01);
+                r23 = __ffma2_rn(nb, y23, r23);
+            }
+            if constexpr (RE) {
+                i01 = __ffma2_rn(aa, y01, i01);
+                i23 = __ffma2_rn(aa, y23, i23);
+            }
+            if constexpr (IM) {
+                i01 = __ffma2_rn(bb, x01, i01);
+                i23 = __ffma2_rn(bb, x23, i23);
+            }
             accr[4 * h] = r01.x;
             accr[4 * h + 1] = r01.y;
             accr[4 * h + 2] = r23.x;
@@ -212,10 +221,10 @@ __device__ __forceinline__ void il_fma(float a, float b, const IlWindow<G> &w, f
             const float yv[4] = {w.y[h].x, w.y[h].y, w.y[h].z, w.y[h].w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                accr[4 * h + q] = fmaf(a, xv[q], accr[4 * h + q]);
-                accr[4 * h + q] = fmaf(-b, yv[q], accr[4 * h + q]);
-                acci[4 * h + q] = fmaf(a, yv[q], acci[4 * h + q]);
-                acci[4 * h + q] = fmaf(b, xv[q], acci[4 * h + q]);
+                if constexpr (RE) accr[4 * h + q] = fmaf(a, xv[q], accr[4 * h + q]);
+                if constexpr (IM) accr[4 * h + q] = fmaf(-b, yv[q], accr[4 * h + q]);
+                if constexpr (RE) acci[4 * h + q] = fmaf(a, yv[q], acci[4 * h + q]);
+                if constexpr (IM) acci[4 * h + q] = fmaf(b, xv[q], acci[4 * h + q]);
             }
         }
     }
@@ -233,8 +242,10 @@ __device__ __forceinline__ void il_term(int64_t c, int g0, int quads, float a, f
 // The diagonals k < cn of one metadata chunk for row r (32-bit row and window arithmetic: rows
 // and n_pad * sp below 2^31).  sq[k] = (offset, lo, hi, mask word of the block's rows), sb[k] =
 // value base: one 16-byte and one 8-byte shared-memory load per diagonal; a warp skips a dead
-// tile or a diagonal outside its rows together.
-template <int G, bool PACKED = false>
+// tile or a diagonal outside its rows together.  REAL: the matrix holds no imaginary part, so half the
+// matrix loads and multiply-adds are left out (choosing per tile, as the planar kernels do, put
+// branches between the loads of successive diagonals and made this loop 10 % slower, not faster).
+template <int G, bool PACKED = false, bool REAL = false>
 __device__ __forceinline__ void il_accumulate32(const int4 *sq, const int64_t *sb, int cn, int r, int g0, int quads,
                                                 const float *__restrict__ are, const float *__restrict__ aim,
                                                 const float *__restrict__ xr, const float *__restrict__ xi,
@@ -246,7 +257,7 @@ __device__ __forceinline__ void il_accumulate32(const int4 *sq, const int64_t *s
         const int4 q = sq[k];
         if (r < q.y || r >= q.z || !(((uint32_t)q.w >> tbit) & 1u)) continue;
         const int64_t vb = sb[k] + r;
-        const float a = __ldcs(are + vb), b = __ldcs(aim + vb);
+        const float a = __ldcs(are + vb), b = REAL ? 0.f : __ldcs(aim + vb);
         const int c = r + q.x;
         IlWindow<G> w;
 #pragma unroll
@@ -255,8 +266,17 @@ __device__ __forceinline__ void il_accumulate32(const int4 *sq, const int64_t *s
             w.x[h] = __ldg(reinterpret_cast<const float4 *>(xr + at));
             w.y[h] = __ldg(reinterpret_cast<const float4 *>(xi + at));
         }
-        il_fma<G, PACKED>(a, b, w, accr, acci);
+        il_fma<G, PACKED, true, !REAL>(a, b, w, accr, acci);
     }
+}
+
+// Whether any of a thread's sums is infinite or NaN.
+template <int G>
+__device__ __forceinline__ bool il_nonfinite(const float (&accr)[G], const float (&acci)[G]) {
+    uint32_t big = 0u;
+#pragma unroll
+    for (int q = 0; q < G; ++q) big = max(big, max(abs_hi(accr[q]), abs_hi(acci[q])));
+    return any_nonfinite<float>(big);
 }
 
 }  // namespace diaq_gb300

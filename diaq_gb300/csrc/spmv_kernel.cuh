@@ -37,8 +37,9 @@ constexpr int kMetaChunk = 256;
 // the two sums through the plane that is used, since every value of a visited tile is multiplied.  So
 // a row whose sums come out non-finite (from x, from stored values, or by overflow) is summed again
 // with both planes: the results are those of the full product in every case.
-// Fill the mask of A (tile_mask_bytes(A.nd, A.rows)) on stream s.
-int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s);
+// Fill the mask of A (tile_mask_bytes(A.nd, A.rows)) on stream s; *has_im (on the device, may be NULL)
+// is set to 1 if A holds a nonzero imaginary part and else left as it is.
+int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s, int *has_im = nullptr);
 // A's own mask, built (and waited for) on first use after its values were last written; NULL when
 // it cannot be had now (s is being captured into a graph, or allocation failed): visit every tile.
 const uint32_t *cached_tile_mask(const Matrix &A, cudaStream_t s);
@@ -114,7 +115,8 @@ __device__ __forceinline__ bool aligned16(const void *p) { return aligned_to<16>
 // run of live 32-row tiles among the block's tiles from row row0 (mask bits `bits`, bit j = tile
 // j), clipped to the stored rows [lo, hi) widened to whole tiles.  Tile starts are 128-byte
 // aligned in every plane (base is a multiple of 32 values), and the widened ends stay inside the
-// allocation (a guard of 32 values before the first diagonal and after the last).  The
+// allocation (a guard of 32 values before the first diagonal and after the last).  real: the real
+// plane only.  The
 // interleaved kernels (256 rows per block) use it; in the planar kernel below and the float-pair
 // SpMV (1,024 rows per block, up to 8 KB per diagonal and plane ahead) it measured slower on the
 // 20-qubit chain -- one-state Horner evolution 2,106 -> 1,693 states x steps/s, float-pair SpMV
@@ -135,12 +137,12 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 template <typename T>
-__device__ __forceinline__ void prefetch_tiles_l2(const T *are, const T *aim, int64_t base, int64_t lo, int64_t hi,
-                                                  uint32_t bits, int64_t row0) {
+__device__ __forceinline__ void prefetch_tiles_l2(const T *are, const T *aim, bool real, int64_t base, int64_t lo,
+                                                  int64_t hi, uint32_t bits, int64_t row0) {
     for_live_runs(bits, row0, lo, hi, [&](int64_t a, int64_t b) {
         const uint32_t bytes = (uint32_t)(b - a) * (uint32_t)sizeof(T);
         prefetch_l2(are + base + a, bytes);
-        prefetch_l2(aim + base + a, bytes);
+        if (!real) prefetch_l2(aim + base + a, bytes);
     });
 }
 

@@ -16,7 +16,7 @@ constexpr int kMaskRows = 256;   // rows per warp: 8 tiles
 template <typename T>
 __global__ void __launch_bounds__(kMaskWarps * 32)
     tile_mask_kernel(const DiagMeta *__restrict__ meta, int64_t words, const T *__restrict__ re,
-                     const T *__restrict__ im, int64_t W, uint32_t *__restrict__ mask) {
+                     const T *__restrict__ im, int64_t W, uint32_t *__restrict__ mask, int *__restrict__ has_im) {
     constexpr int V = VecOf<T>::V;            // rows per lane and load: a warp's load covers V tiles
     constexpr int N = kMaskRows / (32 * V);   // loads per plane
     constexpr int L = 32 / V;                 // lanes per tile
@@ -62,19 +62,20 @@ __global__ void __launch_bounds__(kMaskWarps * 32)
     }
     // byte `at & 3` of the word, in memory order (little-endian)
     if (lane < 3) reinterpret_cast<uint8_t *>(mask)[lane * 4 * words + at] = (uint8_t)(lane == 0 ? br | bi : lane == 1 ? br : bi);
+    if (has_im && bi && lane == 0) *has_im = 1;   // every writer stores 1
 }
 
-int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s) {
+int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s, int *has_im) {
     if (A.nd == 0 || A.rows == 0) return DIAQ_OK;
     const int64_t W = tile_mask_words(A.rows), words = W * A.nd, blocks = (4 * words + kMaskWarps - 1) / kMaskWarps;
     if (blocks > 0x7fffffffll) return set_error(DIAQ_ERR_UNSUPPORTED, "tile mask: too many rows");
     // float pairs: the hi planes (the first `capacity` floats); a zero hi part has a zero lo part
     if (A.prec == DIAQ_C64 || A.prec == DIAQ_C128F2)
         tile_mask_kernel<float><<<(unsigned)blocks, kMaskWarps * 32, 0, s>>>(A.d_meta, words, (const float *)A.re,
-                                                                             (const float *)A.im, W, mask);
+                                                                             (const float *)A.im, W, mask, has_im);
     else
         tile_mask_kernel<double><<<(unsigned)blocks, kMaskWarps * 32, 0, s>>>(A.d_meta, words, (const double *)A.re,
-                                                                              (const double *)A.im, W, mask);
+                                                                              (const double *)A.im, W, mask, has_im);
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }

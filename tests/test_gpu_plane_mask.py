@@ -200,3 +200,36 @@ def test_matrix_products_are_the_full_products(native, prec, tol, rows, inner, c
             assert np.abs(g[ok] - w[ok]).max(initial=0.0) < tol * 10, dc
         p += L
     assert (bad > 0) == special
+
+
+@pytest.mark.parametrize("offs", [[0, 1, -1, 37, -37, 700, 64, 5], list(range(-130, 140))])
+@pytest.mark.parametrize("k", [4, 9])
+@pytest.mark.parametrize("mode", ["mixed", "horner"])
+@pytest.mark.parametrize("special", [False, True])
+def test_real_matrices_in_the_interleaved_kernels(native, offs, k, mode, special):
+    """A matrix without an imaginary part: the interleaved plan kernel and the interleaved batched
+    kernel give the bits of the kernels that take both planes, also for infinite and NaN states."""
+    import torch
+
+    capi, _ = native
+    N = 1500
+    off, re, im = planes(N, N, offs, 21, scale=0.05)
+    im[:] = 0
+    H = capi.Matrix.create(N, N, off, re, im)
+    X = vectors(k, N, 5, special) * 0.1
+    md = capi.EVOLVE_MIXED if mode == "mixed" else capi.EVOLVE_HORNER
+    want = _evolve(capi, H, N, X, md, (4, 1, 9))
+    assert np.isfinite(want).all() != special
+    assert np.array_equal(_evolve(capi, H, N, X, md, (4, 1, 12)), want, equal_nan=True)
+    got = []
+    for il in (True, False):
+        pr, pi = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (X.real, X.imag))
+        B = capi.Batch([H.convert(capi.C64)], [pr], [pi])
+        B.set_horner(mode == "horner")
+        B.set_interleaved(il)
+        B.set_config(4, 1)
+        B.run(0.05, [0], [3], 1)
+        torch.cuda.synchronize()
+        got.append(np.stack([pr.cpu().numpy(), pi.cpu().numpy()]))
+    assert np.array_equal(got[0], got[1], equal_nan=True)
+    assert np.array_equal(got[0], want, equal_nan=True)
