@@ -390,7 +390,9 @@ struct Batch {
     void *work = nullptr;
     uint32_t *masks = nullptr;        // zero-tile masks of every instance's matrix
     int *has_im = nullptr;            // ... and whether it holds an imaginary part
-    std::vector<const Matrix *> mats;
+    MaskJob *d_jobs = nullptr;        // what fills them, one entry per instance with diagonals
+    int n_jobs = 0;
+    int64_t job_bytes = 0;
     cudaStream_t s = nullptr;         // capture stream
     cudaStream_t side[5] = {};        // ... and those of the chains recorded beside it
     cudaEvent_t fork = nullptr, join[5] = {};
@@ -410,6 +412,7 @@ struct Batch {
         cudaFree(d_il_items);
         cudaFree(work);
         cudaFree(masks);
+        cudaFree(d_jobs);
         if (s) cudaStreamDestroy(s);
         if (fork) cudaEventDestroy(fork);
         for (int c = 0; c < 5; ++c) {
@@ -791,6 +794,7 @@ int diaq_batch_create(int n_inst, const diaq_matrix_t *H, const int *nrhs, doubl
     }
     uint8_t *w = (uint8_t *)B->work;
     size_t mask_off = 0;
+    std::vector<MaskJob> jobs;
     for (int i = 0; i < n_inst; ++i) {
         BatchInst I{};
         I.meta = H[i]->d_meta;
@@ -805,8 +809,11 @@ int diaq_batch_create(int n_inst, const diaq_matrix_t *H, const int *nrhs, doubl
         I.tmask = B->masks + mask_off;
         I.mw = tile_mask_words(H[i]->rows);
         I.has_im = B->has_im + i;
+        if (H[i]->nd > 0 && H[i]->rows > 0) {
+            jobs.push_back(mask_job(*H[i], B->masks + mask_off, B->has_im + i, B->job_bytes));
+            B->job_bytes += mask_job_bytes(*H[i]);
+        }
         mask_off += tile_mask_bytes(H[i]->nd, H[i]->rows) / sizeof(uint32_t);
-        B->mats.push_back(H[i]);
         const size_t vb = vec_bytes(i);
         void **slots[8] = {&I.var, &I.vai, &I.vbr, &I.vbi, &I.hr, &I.hi, &I.lr, &I.li};
         for (int j = 0; j < 8; ++j) {
@@ -814,6 +821,13 @@ int diaq_batch_create(int n_inst, const diaq_matrix_t *H, const int *nrhs, doubl
             w += vb;
         }
         B->inst.push_back(I);
+    }
+    B->n_jobs = (int)jobs.size();
+    e = dev_malloc(&B->d_jobs, sizeof(MaskJob) * std::max<size_t>(jobs.size(), 1));
+    if (e == cudaSuccess) e = cudaMemcpy(B->d_jobs, jobs.data(), sizeof(MaskJob) * jobs.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        delete B;
+        return cuda_status(e, "batch create", __FILE__, __LINE__);
     }
     *out = B;
     return DIAQ_OK;
@@ -876,8 +890,7 @@ int diaq_batch_run(diaq_batch_t B, double dt, const int *substeps_log2, const in
     cudaStream_t user = (cudaStream_t)stream;
     // the matrices are the caller's: their zero-tile masks are taken afresh at every run
     DQ_CUDA(cudaMemsetAsync(B->has_im, 0, sizeof(int) * B->inst.size(), user));
-    for (size_t i = 0; i < B->inst.size(); ++i)
-        DQ_TRY(build_tile_mask(*B->mats[i], (uint32_t *)B->inst[i].tmask, user, B->has_im + i));
+    DQ_TRY(build_tile_masks(B->d_jobs, B->n_jobs, B->job_bytes, B->prec, user));
     DQ_CUDA(cudaStreamSynchronize(user));
     std::vector<int> key(substeps_log2, substeps_log2 + B->inst.size());
     key.insert(key.end(), m, m + B->inst.size());

@@ -40,6 +40,19 @@ constexpr int kMetaChunk = 256;
 // Fill the mask of A (tile_mask_bytes(A.nd, A.rows)) on stream s; *has_im (on the device, may be NULL)
 // is set to 1 if A holds a nonzero imaginary part and else left as it is.
 int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s, int *has_im = nullptr);
+// The masks of many matrices of one precision in one launch: jobs (on the device) in the order of
+// `first`, the running sum of their mask_job_bytes; bytes is the whole sum.
+struct MaskJob {
+    const DiagMeta *meta;
+    const void *re, *im;
+    int64_t W, words;    // words per diagonal and per plane
+    uint32_t *mask;
+    int *has_im;
+    int64_t first;
+};
+MaskJob mask_job(const Matrix &A, uint32_t *mask, int *has_im, int64_t first);
+inline int64_t mask_job_bytes(const Matrix &A) { return 4 * tile_mask_words(A.rows) * A.nd; }
+int build_tile_masks(const MaskJob *jobs, int n, int64_t bytes, int prec, cudaStream_t s);
 // A's own mask, built (and waited for) on first use after its values were last written; NULL when
 // it cannot be had now (s is being captured into a graph, or allocation failed): visit every tile.
 const uint32_t *cached_tile_mask(const Matrix &A, cudaStream_t s);

@@ -13,17 +13,16 @@ namespace diaq_gb300 {
 constexpr int kMaskWarps = 8;
 constexpr int kMaskRows = 256;   // rows per warp: 8 tiles
 
+// Byte `at` of each plane of the mask of one matrix (words = W * nd words per plane), by one warp.
 template <typename T>
-__global__ void __launch_bounds__(kMaskWarps * 32)
-    tile_mask_kernel(const DiagMeta *__restrict__ meta, int64_t words, const T *__restrict__ re,
-                     const T *__restrict__ im, int64_t W, uint32_t *__restrict__ mask, int *__restrict__ has_im) {
+__device__ __forceinline__ void tile_mask_byte(const DiagMeta *__restrict__ meta, int64_t words, const T *__restrict__ re,
+                                               const T *__restrict__ im, int64_t W, uint32_t *__restrict__ mask,
+                                               int *__restrict__ has_im, int64_t at) {
     constexpr int V = VecOf<T>::V;            // rows per lane and load: a warp's load covers V tiles
     constexpr int N = kMaskRows / (32 * V);   // loads per plane
     constexpr int L = 32 / V;                 // lanes per tile
     constexpr uint32_t G = (1u << L) - 1u;
     const int lane = (int)threadIdx.x & 31;
-    const int64_t at = (int64_t)blockIdx.x * kMaskWarps + (threadIdx.x >> 5);   // byte of a plane
-    if (at >= 4 * words) return;
     const int64_t j = (at >> 2) / W, r0 = ((at >> 2) - j * W) * 1024 + (at & 3) * kMaskRows;
     const DiagMeta m = meta[j];
     uint32_t br = 0u, bi = 0u;
@@ -65,6 +64,29 @@ __global__ void __launch_bounds__(kMaskWarps * 32)
     if (has_im && bi && lane == 0) *has_im = 1;   // every writer stores 1
 }
 
+template <typename T>
+__global__ void __launch_bounds__(kMaskWarps * 32)
+    tile_mask_kernel(const DiagMeta *__restrict__ meta, int64_t words, const T *__restrict__ re,
+                     const T *__restrict__ im, int64_t W, uint32_t *__restrict__ mask, int *__restrict__ has_im) {
+    const int64_t at = (int64_t)blockIdx.x * kMaskWarps + (threadIdx.x >> 5);
+    if (at < 4 * words) tile_mask_byte<T>(meta, words, re, im, W, mask, has_im, at);
+}
+
+// Many matrices at once: warp w works on byte w - first of the job whose bytes hold it.
+template <typename T>
+__global__ void __launch_bounds__(kMaskWarps * 32) tile_masks_kernel(const MaskJob *__restrict__ jobs, int n, int64_t bytes) {
+    const int64_t w = (int64_t)blockIdx.x * kMaskWarps + (threadIdx.x >> 5);
+    if (w >= bytes) return;
+    int a = 0, b = n - 1;   // the last job that starts at or before w
+    while (a < b) {
+        const int m = (a + b + 1) >> 1;
+        if (jobs[m].first <= w) a = m;
+        else b = m - 1;
+    }
+    const MaskJob J = jobs[a];
+    tile_mask_byte<T>(J.meta, J.words, (const T *)J.re, (const T *)J.im, J.W, J.mask, J.has_im, w - J.first);
+}
+
 int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s, int *has_im) {
     if (A.nd == 0 || A.rows == 0) return DIAQ_OK;
     const int64_t W = tile_mask_words(A.rows), words = W * A.nd, blocks = (4 * words + kMaskWarps - 1) / kMaskWarps;
@@ -76,6 +98,23 @@ int build_tile_mask(const Matrix &A, uint32_t *mask, cudaStream_t s, int *has_im
     else
         tile_mask_kernel<double><<<(unsigned)blocks, kMaskWarps * 32, 0, s>>>(A.d_meta, words, (const double *)A.re,
                                                                               (const double *)A.im, W, mask, has_im);
+    DQ_CUDA(cudaGetLastError());
+    return DIAQ_OK;
+}
+
+MaskJob mask_job(const Matrix &A, uint32_t *mask, int *has_im, int64_t first) {
+    const int64_t W = tile_mask_words(A.rows);
+    return MaskJob{A.d_meta, A.re, A.im, W, W * A.nd, mask, has_im, first};
+}
+
+int build_tile_masks(const MaskJob *jobs, int n, int64_t bytes, int prec, cudaStream_t s) {
+    if (n == 0 || bytes == 0) return DIAQ_OK;
+    const int64_t blocks = (bytes + kMaskWarps - 1) / kMaskWarps;
+    if (blocks > 0x7fffffffll) return set_error(DIAQ_ERR_UNSUPPORTED, "tile mask: too many rows");
+    if (prec == DIAQ_C64 || prec == DIAQ_C128F2)
+        tile_masks_kernel<float><<<(unsigned)blocks, kMaskWarps * 32, 0, s>>>(jobs, n, bytes);
+    else
+        tile_masks_kernel<double><<<(unsigned)blocks, kMaskWarps * 32, 0, s>>>(jobs, n, bytes);
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
