@@ -165,9 +165,9 @@ __global__ void __launch_bounds__(kSpmvThreads)
                     const int64_t lo = q.y, hi = q.z;
                     if (r0 + VR <= lo || r0 >= hi || !(((uint32_t)q.w >> tbit) & 1u)) continue;
                     if (real)
-                        dia_mac<T, K, VR, true, false>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
+                        dia_mac<T, K, VR, true, false, false>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
                     else
-                        dia_mac<T, K, VR, true, true>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
+                        dia_mac<T, K, VR, true, true, false>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
                 }
             }
             if (!real) break;

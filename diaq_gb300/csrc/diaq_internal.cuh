@@ -137,17 +137,43 @@ int zero_gaps(const Matrix &M, cudaStream_t s);
 int scatter_packed(Matrix &M, const double *re, const double *im, cudaStream_t s);
 int gather_packed(const Matrix &M, double *re, double *im, cudaStream_t s);
 
+// ---- dependent launches ----------------------------------------------------------------------------
+// A chain of short kernels on one stream (the Taylor terms of a step) spends much of its time between
+// kernels.  launch_chained starts a kernel while its predecessor drains: the kernel does what needs
+// none of the predecessor's results (metadata, masks, matrix prefetches), then dependency_wait(),
+// which returns when the predecessor has completed and its writes are visible.  Every thread calls
+// dependency_wait before it reads a vector and before it writes anything; dependents_go lets the
+// successor start -- called after the sums, so that waiting blocks take nothing from the ones at work
+// (called at the start: 291 -> 316 us for 16 terms of 16 states on a 15-qubit Pauli sum).  Launched the
+// ordinary way both do nothing.  10 steps of 12 terms, 12-qubit Ising chain: 990 -> 615 us.
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependents_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned grid, unsigned block, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ---- kernels used across units ------------------------------------------------------------
 int spmv_launch(const Matrix &A, const void *xr, const void *xi, int64_t ldx, void *yr, void *yi,
                 int64_t ldy, int nrhs, cudaStream_t s);
 
 // Taylor term of the time evolution: term_out = (-i * scale) * (A term_in); acc += term_out
 // (acc = init + term_out when init is given).  Vectors in the matrix's precision.  tmask: A's
-// zero-tile mask, or NULL.
+// zero-tile mask, or NULL.  chained: see launch_chained.
 int taylor_term_launch(const Matrix &A, const void *tin_r, const void *tin_i, void *tout_r,
                        void *tout_i, void *acc_r, void *acc_i, const void *init_r,
                        const void *init_i, double scale, int nrhs, int64_t ld, cudaStream_t s,
-                       const uint32_t *tmask);
+                       const uint32_t *tmask, bool chained);
 
 int num_sms();
 

@@ -33,7 +33,7 @@ int ham_sim_run(const Matrix &H, const double *p0r, const double *p0i, double t,
         double *tin_r = ar, *tin_i = ai, *tout_r = t0r, *tout_i = t0i;
         for (int k = 1; k <= m; ++k) {
             DQ_TRY(taylor_term_launch(H, tin_r, tin_i, tout_r, tout_i, br, bi, k == 1 ? ar : nullptr,
-                                      k == 1 ? ai : nullptr, dt / (double)k, 1, n, s, tmask));
+                                      k == 1 ? ai : nullptr, dt / (double)k, 1, n, s, tmask, step > 0 || k > 1));
             std::swap(tin_r, tout_r);
             std::swap(tin_i, tout_i);
         }

@@ -50,6 +50,7 @@ namespace diaq_gb300 {
 // ---- epilogues ---------------------------------------------------------------------------------------
 // Plain term: term = (-i*scale) * (A x); out = base + term, base = init (first term) or `in`.
 struct EpiPlain {
+    static constexpr bool kChained = true;
     double *tr, *ti;              // term out (NULL on a sub-step's last term: nobody reads it)
     const double *br, *bi;        // base of the sum
     double *outr, *outi;          // sum out
@@ -94,6 +95,7 @@ struct EpiPlain {
 //   k <  m:  vout = t;
 //   k == m:  psi += (double)hi + (double)lo;  vout = fp32(psi)  (next sub-step's input).
 struct EpiMixed {
+    static constexpr bool kChained = true;
     float *vr, *vi;                     // vout
     float *hr, *hi_, *lr, *li;          // compensated sum (hi, lo), re and im
     double *pr, *pi;                    // state
@@ -164,6 +166,7 @@ struct EpiMixed {
 // carry no float64 code); -1: the runtime field `last` decides.
 template <int LAST = -1>
 struct EpiHornerP {
+    static constexpr bool kChained = true;
     float *wr, *wi;                 // w out
     const float *fr, *fi;           // fp32(psi)
     double *pr, *pi;                // psi
@@ -412,11 +415,11 @@ __global__ void __launch_bounds__(kSpmvThreads)
 //   and runs half the multiply-adds: 95 -> 84 us per 8-state Horner term of a step on the 20-qubit chain,
 //   where issue is now at 50 %, L1 at 58 % and DRAM at 32 % of their peaks.  A row whose sums are
 //   not finite is summed again with both planes (one chunk of metadata: the launcher sees to it).
-template <class Epi, int G, int MINB, bool REAL>
+template <class Epi, int G, int MINB, bool REAL, bool CHAINED>
 __global__ void __launch_bounds__(kSpmvThreads, MINB)
     dia_spmv_il32_kernel(const DiagMeta *__restrict__ meta, int nd, const float *__restrict__ are,
-                         const float *__restrict__ aim, int rows, const float *__restrict__ xr,
-                         const float *__restrict__ xi, const uint32_t *__restrict__ tmask, int64_t mw, Epi epi) {
+                         const float *__restrict__ aim, int rows, const float *xr,
+                         const float *xi, const uint32_t *__restrict__ tmask, int64_t mw, Epi epi) {
     static_assert(G == 4 || G == 8, "4 or 8 states per thread");
     constexpr bool kTile = Epi::kPsiTile;
     __shared__ int4 sq[kMetaChunk];       // off, lo, hi, mask word
@@ -431,33 +434,38 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
     const int r = row0 + (wid / groups) * 32 + lane;
     float accr[G], acci[G];
     bool tile = false;
-    if constexpr (kTile) {
-        tile = epi.reads_psi() && r < rows;
-        if (tile) {
+    // what needs the previous term's results: the fp32(psi) quads, the block's rows of the input states
+    auto begin = [&]() {
+        if constexpr (CHAINED) dependency_wait();
+        if constexpr (kTile) {
+            tile = epi.reads_psi() && r < rows;
+            if (tile) {
 #pragma unroll
-            for (int h = 0; h < G / 4; ++h) {
-                const int64_t i = il_at(r, g * (G / 4) + h, quads);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(&spsi[wid][h][0][lane])),
-                             "l"(epi.fr + i)
-                             : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(&spsi[wid][h][1][lane])),
-                             "l"(epi.fi + i)
-                             : "memory");
+                for (int h = 0; h < G / 4; ++h) {
+                    const int64_t i = il_at(r, g * (G / 4) + h, quads);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(&spsi[wid][h][0][lane])),
+                                 "l"(epi.fr + i)
+                                 : "memory");
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(&spsi[wid][h][1][lane])),
+                                 "l"(epi.fi + i)
+                                 : "memory");
+                }
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    if (threadIdx.x == 0 && row0 < rows) {
-        // the block's own rows of the input states (all quads: one contiguous run per plane),
-        // inside the rows padded to 32
-        const int64_t at = (int64_t)(row0 >> 5) * quads * 128;
-        const int tiles = min(8 / groups, (rows + 31 - row0) >> 5);
-        const uint32_t bytes = (uint32_t)tiles * (uint32_t)quads * 512u;
-        prefetch_l2(xr + at, bytes);
-        prefetch_l2(xi + at, bytes);
-    }
+        if (threadIdx.x == 0 && row0 < rows) {
+            // the block's own rows of the input states (all quads: one contiguous run per plane),
+            // inside the rows padded to 32
+            const int64_t at = (int64_t)(row0 >> 5) * quads * 128;
+            const int tiles = min(8 / groups, (rows + 31 - row0) >> 5);
+            const uint32_t bytes = (uint32_t)tiles * (uint32_t)quads * 512u;
+            prefetch_l2(xr + at, bytes);
+            prefetch_l2(xi + at, bytes);
+        }
+    };
+    if (!CHAINED || nd == 0) begin();
 #pragma unroll
     for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;
     for (int c0 = 0; c0 < nd; c0 += kMetaChunk) {
@@ -480,16 +488,18 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
                                   block_tile_bits((uint32_t)q.w, row0, 8 / groups), row0);
             }
         }
+        if (CHAINED && c0 == 0) begin();
         if (r >= rows) continue;
-        il_accumulate32<G, true, REAL>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+        il_accumulate32<G, true, REAL, CHAINED>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
         if constexpr (REAL) {   // one chunk (the launcher sees to it): not finite -- sum again, in full
             if (il_nonfinite<G>(accr, acci)) {
 #pragma unroll
                 for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;
-                il_accumulate32<G, true, false>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+                il_accumulate32<G, true, false, CHAINED>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
             }
         }
     }
+    if constexpr (CHAINED) dependents_go();
     if constexpr (kTile) asm volatile("cp.async.wait_all;" ::: "memory");
     if (r >= rows) return;
 #pragma unroll
@@ -589,7 +599,7 @@ namespace diaq_gb300 {
 // memory, spmv_tma.cuh; 8 or 4 states per thread as 9; the register kernel of 9 when the matrix
 // has more diagonals than one metadata chunk).
 template <class Epi>
-int launch_il(const EvolvePlan &P, const float *xr, const float *xi, const Epi &e) {
+int launch_il(const EvolvePlan &P, const float *xr, const float *xi, const Epi &e, bool chained) {
     const int v = P.cfg.pipe;
     const bool eight = v >= 9 && P.sp % 8 == 0;
     if (v == 12 && (int64_t)P.n_pad * P.sp < ((int64_t)1 << 31)) {
@@ -603,14 +613,24 @@ int launch_il(const EvolvePlan &P, const float *xr, const float *xi, const Epi &
         const DiagMeta *md = P.Hc->d_meta;
         const int nd = P.Hc->nd, n = (int)P.n;
         const bool real = P.real && nd <= kMetaChunk;
-        if (eight && real)
-            dia_spmv_il32_kernel<Epi, 8, 5, true><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
-        else if (eight)
-            dia_spmv_il32_kernel<Epi, 8, 5, false><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
-        else if (real)
-            dia_spmv_il32_kernel<Epi, 4, 6, true><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
-        else
-            dia_spmv_il32_kernel<Epi, 4, 6, false><<<g, kSpmvThreads, 0, P.s>>>(md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
+        // Terms of few blocks are chained: launch gaps and staging count there (16 qubits, 8 states:
+        // 10.7 -> 10.1 us per term), while many blocks hide them and run better with __ldg (20
+        // qubits: 84 us per term, 88 chained; 19 qubits, 2,048 blocks: 47.0 and 48.0)
+        // (8 states per thread of a complex matrix: 16.6 us per term either way at 15 qubits, not chained.)
+        const bool few = g <= 8u * (unsigned)num_sms() && (real || !eight);
+        auto go = [&](auto kernel) {
+            return launch_chained(few && chained, kernel, g, kSpmvThreads, P.s, md, nd, are, aim, n, xr, xi, P.tmask, mw, e);
+        };
+        if (few) {
+            if (eight) go(dia_spmv_il32_kernel<Epi, 8, 5, true, true>);
+            else if (real) go(dia_spmv_il32_kernel<Epi, 4, 6, true, true>);
+            else go(dia_spmv_il32_kernel<Epi, 4, 6, false, true>);
+        } else {
+            if (eight && real) go(dia_spmv_il32_kernel<Epi, 8, 5, true, false>);
+            else if (eight) go(dia_spmv_il32_kernel<Epi, 8, 5, false, false>);
+            else if (real) go(dia_spmv_il32_kernel<Epi, 4, 6, true, false>);
+            else go(dia_spmv_il32_kernel<Epi, 4, 6, false, false>);
+        }
         DQ_CUDA(cudaGetLastError());
         return DIAQ_OK;
     }
@@ -763,6 +783,7 @@ static int enqueue_step(EvolvePlan &P, double dt, int sl, int m, double *pr, dou
     const int sub = 1 << sl;
     const double tau = dt / (double)sub;
     P.launches_per_step = 0;
+    bool chained = false;   // the last thing enqueued is a term kernel of this step (see launch_chained)
     if (P.mode == DIAQ_EVOLVE_C128) {
         double *w = (double *)P.buf;
         const int64_t L = n;  // work vectors use ld = n
@@ -786,7 +807,8 @@ static int enqueue_step(EvolvePlan &P, double dt, int sl, int m, double *pr, dou
                 e.outi = oth_i;
                 e.ld = L;
                 e.scale = tau / (double)t;
-                DQ_TRY((launch_dia_spmv_rhs_cfg<double, EpiPlain, 2, 1>(*P.H, tin_r, tin_i, L, (int)k, e, P.s, P.cfg, P.tmask)));
+                DQ_TRY((launch_dia_spmv_rhs_cfg<double, EpiPlain, 2, 1>(*P.H, tin_r, tin_i, L, (int)k, e, P.s, P.cfg, P.tmask, chained)));
+                chained = true;
                 ++P.launches_per_step;
                 tin_r = tout_r;
                 tin_i = tout_i;
@@ -821,22 +843,24 @@ static int enqueue_step(EvolvePlan &P, double dt, int sl, int m, double *pr, dou
                 if (P.interleaved()) {
                     if (last) {
                         EpiHornerT<1> e{out_r, out_i, fr, fi, gr, gi, pr, pi, ld, P.sp, (int)k, scale, 1};
-                        DQ_TRY(launch_il(P, in_r, in_i, e));
+                        DQ_TRY(launch_il(P, in_r, in_i, e, chained));
                     } else {
                         EpiHornerT<0> e{out_r, out_i, fr, fi, gr, gi, pr, pi, ld, P.sp, (int)k, scale, 0};
-                        DQ_TRY(launch_il(P, in_r, in_i, e));
+                        DQ_TRY(launch_il(P, in_r, in_i, e, chained));
                     }
                 } else if (last) {
                     EpiHornerP<1> e{out_r, out_i, fr, fi, pr, pi, gr, gi, L, scale, 1};
                     DQ_TRY((launch_dia_spmv_rhs_cfg<float, EpiHornerP<1>, 4, 2, 1>(*P.Hc, in_r, in_i, L, (int)k, e,
-                                                                                P.s, P.cfg, P.tmask)));
+                                                                                P.s, P.cfg, P.tmask, chained)));
                 } else {
                     EpiHornerP<0> e{out_r, out_i, fr, fi, pr, pi, gr, gi, L, scale, 0};
                     DQ_TRY((launch_dia_spmv_rhs_cfg<float, EpiHornerP<0>, 4, 2, 1>(*P.Hc, in_r, in_i, L, (int)k, e,
-                                                                                P.s, P.cfg, P.tmask)));
+                                                                                P.s, P.cfg, P.tmask, chained)));
                 }
+                chained = true;
                 ++P.launches_per_step;
                 if (gr != fr) {
+                    chained = false;
                     DQ_CUDA(cudaMemcpyAsync(fr, gr, sizeof(float) * VL, cudaMemcpyDeviceToDevice, P.s));
                     DQ_CUDA(cudaMemcpyAsync(fi, gi, sizeof(float) * VL, cudaMemcpyDeviceToDevice, P.s));
                 }
@@ -860,7 +884,8 @@ static int enqueue_step(EvolvePlan &P, double dt, int sl, int m, double *pr, dou
             if (P.interleaved()) {
                 EpiMixedIL e{out_r, out_i, hr, hi, lr, li, pr, pi, ld, P.sp, (int)k, (float)(tau / (double)t),
                              t == 1, t == m};
-                DQ_TRY(launch_il(P, in_r, in_i, e));
+                DQ_TRY(launch_il(P, in_r, in_i, e, chained));
+                chained = true;
                 ++P.launches_per_step;
                 std::swap(in_r, out_r);
                 std::swap(in_i, out_i);
@@ -886,7 +911,8 @@ static int enqueue_step(EvolvePlan &P, double dt, int sl, int m, double *pr, dou
                 DQ_TRY(launch_dia_spmv_pipe<EpiMixed>(*P.Hc, in_r, in_i, L, (int)k, e, P.s, P.cfg.kmax,
                                                       &P.launches_per_step));
             } else {
-                DQ_TRY((launch_dia_spmv_rhs_cfg<float, EpiMixed, 4, 2, 1>(*P.Hc, in_r, in_i, L, (int)k, e, P.s, P.cfg, P.tmask)));
+                DQ_TRY((launch_dia_spmv_rhs_cfg<float, EpiMixed, 4, 2, 1>(*P.Hc, in_r, in_i, L, (int)k, e, P.s, P.cfg, P.tmask, chained)));
+                chained = true;
                 ++P.launches_per_step;  // one launch over all states
             }
             std::swap(in_r, out_r);

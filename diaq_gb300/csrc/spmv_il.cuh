@@ -245,10 +245,11 @@ __device__ __forceinline__ void il_term(int64_t c, int g0, int quads, float a, f
 // tile or a diagonal outside its rows together.  REAL: the matrix holds no imaginary part, so half the
 // matrix loads and multiply-adds are left out (choosing per tile, as the planar kernels do, put
 // branches between the loads of successive diagonals and made this loop 10 % slower, not faster).
-template <int G, bool PACKED = false, bool REAL = false>
+// CHAINED: see load_state.
+template <int G, bool PACKED = false, bool REAL = false, bool CHAINED = false>
 __device__ __forceinline__ void il_accumulate32(const int4 *sq, const int64_t *sb, int cn, int r, int g0, int quads,
                                                 const float *__restrict__ are, const float *__restrict__ aim,
-                                                const float *__restrict__ xr, const float *__restrict__ xi,
+                                                const float *xr, const float *xi,
                                                 float (&accr)[G], float (&acci)[G]) {
     const int tbit = (r >> 5) & 31;
     // unrolled by 2: 93.1 us per 8-state Horner term on the 20-qubit chain (1 and 4: 95.0 and 93.9)
@@ -263,8 +264,8 @@ __device__ __forceinline__ void il_accumulate32(const int4 *sq, const int64_t *s
 #pragma unroll
         for (int h = 0; h < G / 4; ++h) {
             const int at = ((((c >> 5) * quads) + g0 + h) << 7) + ((c & 31) << 2);
-            w.x[h] = __ldg(reinterpret_cast<const float4 *>(xr + at));
-            w.y[h] = __ldg(reinterpret_cast<const float4 *>(xi + at));
+            w.x[h] = load_state<CHAINED>(reinterpret_cast<const float4 *>(xr + at));
+            w.y[h] = load_state<CHAINED>(reinterpret_cast<const float4 *>(xi + at));
         }
         il_fma<G, PACKED, true, !REAL>(a, b, w, accr, acci);
     }

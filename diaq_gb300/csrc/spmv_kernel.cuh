@@ -111,6 +111,17 @@ __device__ __forceinline__ void load_vec(T (&dst)[VR], const T *p) {
     unpack<VT, T, VR>(dst, __ldg(reinterpret_cast<const VT *>(p)));
 }
 
+// A state value.  In a chained kernel (see launch_chained) a predecessor may still be writing the
+// vector when the kernel starts, so the load is of the ordinary, coherent kind and the pointers to the
+// vector are not __restrict__; elsewhere it is __ldg, which promises data that nobody writes while the
+// kernel lives and is the faster one under load (24 chains batched: 1,225 us against 1,305; __ldca,
+// opaque to the compiler's scheduling: 1,273).
+template <bool CHAINED, typename T>
+__device__ __forceinline__ T load_state(const T *p) {
+    if constexpr (CHAINED) return *p;
+    else return __ldg(p);
+}
+
 // Matrix values stream once: evict them first from L2, keeping x resident.
 template <typename T, int VR = VecOf<T>::V>
 __device__ __forceinline__ void load_vec_stream(T (&dst)[VR], const T *p) {
@@ -181,9 +192,9 @@ struct BaseIm {
 
 // One diagonal's (q = offset, lo, hi) products with rows r0 .. r0 + V - 1 of up to K states, the real
 // (RE) and the imaginary (IM) plane of the matrix each taken or left out.
-template <typename T, int K, int V, bool RE, bool IM>
+template <typename T, int K, int V, bool RE, bool IM, bool CHAINED>
 __device__ __forceinline__ void dia_mac(const int4 &q, int64_t base, int64_t r0, const T *__restrict__ are,
-                                        const T *__restrict__ aim, const T *__restrict__ xr, const T *__restrict__ xi,
+                                        const T *__restrict__ aim, const T *xr, const T *xi,
                                         int64_t ldx, int kq, T (&accr)[K][V], T (&acci)[K][V]) {
     constexpr int VB = V * (int)sizeof(T);
     const int64_t lo = q.y, hi = q.z;
@@ -204,14 +215,15 @@ __device__ __forceinline__ void dia_mac(const int4 &q, int64_t base, int64_t r0,
         const T *pxi = xi + k * ldx + c;
         T xrv[V], xiv[V];
         if (full && aligned_to<VB>(pxr) && aligned_to<VB>(pxi)) {
-            load_vec<T, V>(xrv, pxr);
-            load_vec<T, V>(xiv, pxi);
+            using VT = typename Vec<T, V>::type;
+            unpack<VT, T, V>(xrv, load_state<CHAINED>(reinterpret_cast<const VT *>(pxr)));
+            unpack<VT, T, V>(xiv, load_state<CHAINED>(reinterpret_cast<const VT *>(pxi)));
         } else {
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const bool ok = (r0 + v >= lo) && (r0 + v < hi);
-                xrv[v] = ok ? __ldg(pxr + v) : (T)0;
-                xiv[v] = ok ? __ldg(pxi + v) : (T)0;
+                xrv[v] = ok ? load_state<CHAINED>(pxr + v) : (T)0;
+                xiv[v] = ok ? load_state<CHAINED>(pxi + v) : (T)0;
             }
         }
 #pragma unroll
@@ -231,8 +243,8 @@ __device__ __forceinline__ void dia_mac(const int4 &q, int64_t base, int64_t r0,
 template <typename T, int K, int VR, class Epi>
 __global__ void __launch_bounds__(kSpmvThreads)
     dia_spmv_kernel(const DiagMeta *__restrict__ meta, int nd, const T *__restrict__ are,
-                    const T *__restrict__ aim, int64_t rows, const T *__restrict__ xr,
-                    const T *__restrict__ xi, int64_t ldx, int nrhs, int nchunk, const uint32_t *__restrict__ tmask,
+                    const T *__restrict__ aim, int64_t rows, const T *xr,
+                    const T *xi, int64_t ldx, int nrhs, int nchunk, const uint32_t *__restrict__ tmask,
                     int64_t mw, Epi epi0) {
     constexpr int V = VR;
     // per diagonal: offset, row range and the real plane's mask word of the block's rows in one
@@ -252,6 +264,7 @@ __global__ void __launch_bounds__(kSpmvThreads)
     const int tbit = (int)((r0 >> 5) & 31);
     T accr[K][V], acci[K][V];
 
+    if (Epi::kChained && nd == 0) dependency_wait();
     for (int pass = 0;; ++pass) {  // a second pass, with both planes, for rows that are not finite
 #pragma unroll
         for (int q = 0; q < K; ++q)
@@ -270,6 +283,7 @@ __global__ void __launch_bounds__(kSpmvThreads)
                     sb[i] = BaseIm{m.base, wi, 0u};
                 }
                 __syncthreads();
+                if constexpr (Epi::kChained) dependency_wait();
             }
             if (r0 >= rows) continue;
 #pragma unroll 2
@@ -285,11 +299,11 @@ __global__ void __launch_bounds__(kSpmvThreads)
                 // (165 us per c128 product on the 20-qubit chain).  float32 takes imaginary-only tiles
                 // as complex ones: a third body cost its complex tiles 4 %
                 if (!im)
-                    dia_mac<T, K, V, true, false>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
+                    dia_mac<T, K, V, true, false, Epi::kChained>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
                 else if (re || sizeof(T) == 4)
-                    dia_mac<T, K, V, true, true>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
+                    dia_mac<T, K, V, true, true, Epi::kChained>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
                 else
-                    dia_mac<T, K, V, false, true>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
+                    dia_mac<T, K, V, false, true, Epi::kChained>(q, b.base, r0, are, aim, xr, xi, ldx, kq, accr, acci);
             }
         }
         if (pass || !tmask) break;
@@ -302,6 +316,7 @@ __global__ void __launch_bounds__(kSpmvThreads)
         const bool again = any_nonfinite<T>(big);
         if (!(nd > kMetaChunk ? __syncthreads_or(again) : again)) break;
     }
+    if constexpr (Epi::kChained) dependents_go();
     if (r0 < rows) epi.template apply<T, K, V>(r0, rows, kq, accr, acci);
 }
 
@@ -322,7 +337,7 @@ constexpr int64_t kRowKernelMax = sizeof(T) == 8 ? 65536 : 262144;
 template <typename T, int K, int NT, int U, class Epi>
 __global__ void __launch_bounds__(NT)
     dia_spmv_row_kernel(const DiagMeta *__restrict__ meta, int nd, const T *__restrict__ are,
-                        const T *__restrict__ aim, int rows, const T *__restrict__ xr, const T *__restrict__ xi,
+                        const T *__restrict__ aim, int rows, const T *xr, const T *xi,
                         int64_t ldx, int nrhs, int nchunk, const uint32_t *__restrict__ tmask, int64_t mw, Epi epi0) {
     __shared__ int4 sq[kMetaChunk];
     __shared__ BaseIm sb[kMetaChunk];
@@ -342,6 +357,7 @@ __global__ void __launch_bounds__(NT)
     xi += r;
     are += r;
     aim += r;
+    if (Epi::kChained && nd == 0) dependency_wait();
     for (int pass = 0;; ++pass) {
 #pragma unroll
         for (int k = 0; k < K; ++k) accr[k][0] = acci[k][0] = (T)0;
@@ -358,6 +374,7 @@ __global__ void __launch_bounds__(NT)
                     sb[i] = BaseIm{m.base, wi, 0u};
                 }
                 __syncthreads();
+                if constexpr (Epi::kChained) dependency_wait();
             }
             for (int i0 = 0; i0 < cn; i0 += 32) {
                 bool re = false, im = false;
@@ -380,8 +397,8 @@ __global__ void __launch_bounds__(NT)
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
                         if (k >= kq) break;
-                        d.x[k] = ok ? __ldg(xr + k * ldx + q.x) : (T)0;
-                        d.y[k] = ok ? __ldg(xi + k * ldx + q.x) : (T)0;
+                        d.x[k] = ok ? load_state<Epi::kChained>(xr + k * ldx + q.x) : (T)0;
+                        d.y[k] = ok ? load_state<Epi::kChained>(xi + k * ldx + q.x) : (T)0;
                     }
                 };
                 auto mac_re = [&](T a, const D &d) {
@@ -469,6 +486,7 @@ __global__ void __launch_bounds__(NT)
         const bool again = any_nonfinite<T>(big);
         if (!(nd > kMetaChunk ? __syncthreads_or(again) : __any_sync(0xffffffffu, again))) break;
     }
+    if constexpr (Epi::kChained) dependents_go();
     if (r < rows) epi.template apply<T, K, 1>(r, rows, kq, accr, acci);
 }
 
@@ -637,9 +655,10 @@ inline bool pf_kernel_fits(const Matrix &A, const float *xr, const float *xi, in
            (reinterpret_cast<uintptr_t>(xi) & 15) == 0;
 }
 
-// Store y = A x.
+// Store y = A x.  (kChained: whether kernels with this epilogue are launched with launch_chained.)
 template <typename T>
 struct EpiStore {
+    static constexpr bool kChained = false;
     T *yr, *yi;
     int64_t ldy;
     template <typename U, int K, int V>
@@ -680,6 +699,7 @@ struct EpiStore {
 // state itself, saving the copy).  Vectors and accumulator of type T.
 template <typename T>
 struct EpiTaylor {
+    static constexpr bool kChained = true;
     T *tr, *ti;      // term out
     T *accr, *acci;  // running sum
     const T *initr, *initi;
@@ -727,10 +747,10 @@ struct SpmvCfg {
 
 template <typename T, int K, class Epi, int VR, int... More>
 void launch_vr(int vr, const Matrix &A, const T *xr, const T *xi, int64_t ldx, int nrhs, int nchunk,
-               const Epi &e, cudaStream_t s, const uint32_t *tmask) {
+               const Epi &e, cudaStream_t s, const uint32_t *tmask, bool chained) {
     if constexpr (sizeof...(More) > 0) {
         if (vr != VR) {
-            launch_vr<T, K, Epi, More...>(vr, A, xr, xi, ldx, nrhs, nchunk, e, s, tmask);
+            launch_vr<T, K, Epi, More...>(vr, A, xr, xi, ldx, nrhs, nchunk, e, s, tmask, chained);
             return;
         }
     }
@@ -738,15 +758,15 @@ void launch_vr(int vr, const Matrix &A, const T *xr, const T *xi, int64_t ldx, i
         constexpr int NT = 64, U = K == 1 ? 4 : 2;
         const int64_t blocks = (A.rows + NT - 1) / NT * nchunk;
         if (A.rows * nchunk <= kRowKernelMax<T>) {
-            dia_spmv_row_kernel<T, K, NT, U, Epi><<<(unsigned)blocks, NT, 0, s>>>(
-                A.d_meta, A.nd, (const T *)A.re, (const T *)A.im, (int)A.rows, xr, xi, ldx, nrhs, nchunk, tmask,
-                tile_mask_words(A.rows), e);
+            launch_chained(chained, dia_spmv_row_kernel<T, K, NT, U, Epi>, (unsigned)blocks, NT, s, A.d_meta, A.nd,
+                           (const T *)A.re, (const T *)A.im, (int)A.rows, xr, xi, ldx, nrhs, nchunk, tmask,
+                           tile_mask_words(A.rows), e);
             return;
         }
     }
-    dia_spmv_kernel<T, K, VR, Epi><<<spmv_blocks(A.rows, VR) * (unsigned)nchunk, kSpmvThreads, 0, s>>>(
-        A.d_meta, A.nd, (const T *)A.re, (const T *)A.im, A.rows, xr, xi, ldx, nrhs, nchunk, tmask,
-        tile_mask_words(A.rows), e);
+    launch_chained(chained, dia_spmv_kernel<T, K, VR, Epi>, spmv_blocks(A.rows, VR) * (unsigned)nchunk, kSpmvThreads, s,
+                   A.d_meta, A.nd, (const T *)A.re, (const T *)A.im, A.rows, xr, xi, ldx, nrhs, nchunk, tmask,
+                   tile_mask_words(A.rows), e);
 }
 
 // One launch over all right-hand sides, in chunks of up to cfg.kmax (<= 8) states per block
@@ -754,10 +774,10 @@ void launch_vr(int vr, const Matrix &A, const T *xr, const T *xi, int64_t ldx, i
 // chunks of a row tile run side by side (see dia_spmv_kernel).  VRs lists the rows-per-thread
 // variants compiled for this epilogue (the first is the default).  Epi must offer
 // `shifted(q0)` on host and device, the same epilogue for right-hand sides q0.. .  tmask: A's
-// zero-tile mask (build_tile_mask), or NULL to visit every tile.
+// zero-tile mask (build_tile_mask), or NULL to visit every tile.  chained: see launch_chained.
 template <typename T, class Epi, int... VRs>
 int launch_dia_spmv_rhs_cfg(const Matrix &A, const T *xr, const T *xi, int64_t ldx, int nrhs, Epi epi,
-                            cudaStream_t s, SpmvCfg cfg, const uint32_t *tmask = nullptr) {
+                            cudaStream_t s, SpmvCfg cfg, const uint32_t *tmask = nullptr, bool chained = false) {
     if (A.rows == 0 || nrhs <= 0) return DIAQ_OK;
     int k = cfg.kmax >= 8 ? 8 : cfg.kmax >= 4 ? 4 : cfg.kmax >= 2 ? 2 : 1;
     while (k > 1 && k / 2 >= nrhs) k /= 2;  // no wider than the states need
@@ -766,13 +786,13 @@ int launch_dia_spmv_rhs_cfg(const Matrix &A, const T *xr, const T *xi, int64_t l
     if ((uint64_t)spmv_blocks(A.rows, vr) * (uint64_t)nchunk > 0x7fffffffull)
         return set_error(DIAQ_ERR_UNSUPPORTED, "spmv: too many row tiles x state chunks for one launch");
     if (k == 8)
-        launch_vr<T, 8, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask);
+        launch_vr<T, 8, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask, chained);
     else if (k == 4)
-        launch_vr<T, 4, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask);
+        launch_vr<T, 4, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask, chained);
     else if (k == 2)
-        launch_vr<T, 2, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask);
+        launch_vr<T, 2, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask, chained);
     else
-        launch_vr<T, 1, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask);
+        launch_vr<T, 1, Epi, VRs...>(vr, A, xr, xi, ldx, nrhs, nchunk, epi, s, tmask, chained);
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
@@ -837,12 +857,12 @@ SpmvCfg default_cfg(int64_t rows, int nrhs) {
 }
 template <typename T, class Epi>
 int launch_dia_spmv_rhs(const Matrix &A, const T *xr, const T *xi, int64_t ldx, int nrhs, Epi epi,
-                        cudaStream_t s, const uint32_t *tmask) {
+                        cudaStream_t s, const uint32_t *tmask, bool chained = false) {
     const SpmvCfg cfg = default_cfg<T>(A.rows, nrhs);
     if constexpr (sizeof(T) == 4)
-        return launch_dia_spmv_rhs_cfg<T, Epi, 4, 1>(A, xr, xi, ldx, nrhs, epi, s, cfg, tmask);
+        return launch_dia_spmv_rhs_cfg<T, Epi, 4, 1>(A, xr, xi, ldx, nrhs, epi, s, cfg, tmask, chained);
     else
-        return launch_dia_spmv_rhs_cfg<T, Epi, 1>(A, xr, xi, ldx, nrhs, epi, s, cfg, tmask);
+        return launch_dia_spmv_rhs_cfg<T, Epi, 1>(A, xr, xi, ldx, nrhs, epi, s, cfg, tmask, chained);
 }
 
 template <typename T>
