@@ -54,6 +54,7 @@ struct Matrix {
     // points; every function that writes values into an existing matrix clears tmask_ok
     mutable uint32_t *tmask = nullptr;
     mutable bool tmask_ok = false;
+    mutable bool real = false;             // C128F2: no imaginary part (known while tmask_ok)
 
     // bytes per stored value and array (C128F2: a hi and a lo float, in two planes)
     size_t elem() const { return prec == DIAQ_C64 ? sizeof(float) : sizeof(double); }
@@ -181,7 +182,8 @@ int num_sms();
 int f2_scatter(Matrix &M, const double *re, const double *im, cudaStream_t s);
 int f2_gather(const Matrix &M, double *re, double *im, cudaStream_t s);
 int f2_convert(const Matrix &src, Matrix &dst, cudaStream_t s);
-int f2_spmv(const Matrix &A, const double *xr, const double *xi, double *yr, double *yi, cudaStream_t s);
+int f2_spmv(const Matrix &A, int nrhs, const double *xr, const double *xi, int64_t ldx, double *yr, double *yi,
+            int64_t ldy, cudaStream_t s);
 
 // Copy of A in precision prec / A without its exact-zero diagonals (new matrices).
 int copy_as(const Matrix &A, int prec, cudaStream_t s, Matrix **out, bool internal = false);

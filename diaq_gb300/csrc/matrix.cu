@@ -194,16 +194,18 @@ int plan_layout(Matrix &M, int64_t rows, int64_t cols, int32_t nd, const int32_t
     return DIAQ_OK;
 }
 
-// The metadata block: DiagMeta records and, behind them, the zero-tile mask's storage, so that SpMV
-// calls never allocate (it is filled on first use).
+// The metadata block: DiagMeta records and, behind them, the zero-tile mask's storage (and a flag: does
+// the matrix hold an imaginary part), so that SpMV calls never allocate (it is filled on first use).
 static size_t meta_bytes(const Matrix &M) { return (sizeof(DiagMeta) * (size_t)M.nd + 255) / 256 * 256; }
+
+static size_t block_bytes(const Matrix &M) { return meta_bytes(M) + tile_mask_bytes(M.nd, M.rows) + sizeof(int); }
 
 // The planes come from the pool.  A caller's matrix has its metadata block from cudaMalloc: freeing
 // that waits for all work on the device (as freeing the planes so would), after which the planes may
 // go back to the pool whatever streams the matrix was used on.
 int allocate(Matrix &M, cudaStream_t s, bool zero) {
     cudaGetDevice(&M.device);
-    const size_t bytes = (size_t)M.capacity * M.elem(), block = meta_bytes(M) + tile_mask_bytes(M.nd, M.rows);
+    const size_t bytes = (size_t)M.capacity * M.elem(), block = block_bytes(M);
     if (M.nd == 0 && !M.internal) {   // no metadata block: plain allocations
         DQ_CUDA(dev_malloc(&M.re, bytes));
         DQ_CUDA(dev_malloc(&M.im, bytes));
@@ -221,6 +223,7 @@ int allocate(Matrix &M, cudaStream_t s, bool zero) {
         else
             DQ_CUDA(dev_malloc(&M.d_meta, block));
         M.tmask = (uint32_t *)((uint8_t *)M.d_meta + meta_bytes(M));
+        DQ_CUDA(cudaMemsetAsync((uint8_t *)M.tmask + tile_mask_bytes(M.nd, M.rows), 0, sizeof(int), s));
         DQ_CUDA(cudaMemcpyAsync(M.d_meta, M.meta.data(), sizeof(DiagMeta) * M.nd, cudaMemcpyHostToDevice, s));
         // the host vector may be reallocated later; finish the copy before returning
         DQ_CUDA(cudaStreamSynchronize(s));
@@ -230,7 +233,7 @@ int allocate(Matrix &M, cudaStream_t s, bool zero) {
 
 int publish(Matrix &M) {
     if (!M.internal) return DIAQ_OK;
-    const size_t block = meta_bytes(M) + tile_mask_bytes(M.nd, M.rows);
+    const size_t block = block_bytes(M);
     DiagMeta *d = nullptr;
     void *re = nullptr, *im = nullptr;
     if (M.nd > 0) {

@@ -12,12 +12,8 @@ int spmv_launch(const Matrix &A, const void *xr, const void *xi, int64_t ldx, vo
     if (!xr || !xi || !yr || !yi) return set_error(DIAQ_ERR_INVALID, "vector pointer is NULL");
     if (nrhs > 1 && (ldx < A.cols || ldy < A.rows))
         return set_error(DIAQ_ERR_INVALID, "leading dimension smaller than the vector length");
-    if (A.prec == DIAQ_C128F2) {  // float64 vectors, float-pair arithmetic; one state per launch
-        for (int q = 0; q < nrhs; ++q)
-            DQ_TRY(f2_spmv(A, (const double *)xr + q * ldx, (const double *)xi + q * ldx, (double *)yr + q * ldy,
-                           (double *)yi + q * ldy, s));
-        return DIAQ_OK;
-    }
+    if (A.prec == DIAQ_C128F2)  // float64 vectors, float-pair arithmetic
+        return f2_spmv(A, nrhs, (const double *)xr, (const double *)xi, ldx, (double *)yr, (double *)yi, ldy, s);
     if (A.prec == DIAQ_C128) {
         EpiStoreRhs<double> e;
         e.yr = (double *)yr;

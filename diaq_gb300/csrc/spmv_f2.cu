@@ -87,11 +87,14 @@ __global__ void f2_gather_kernel(const DiagMeta *__restrict__ meta, int nd, cons
     }
 }
 
-// both float64 vectors of x -> their four hi/lo planes in one launch; vec: x_re and x_im are
-// 16-byte aligned, so pairs of values move as double2 -> float2
-__global__ void f2_split_pair_kernel(const double *__restrict__ xr, const double *__restrict__ xi, int64_t n, int vec,
-                                     float *__restrict__ rh, float *__restrict__ rl, float *__restrict__ ih,
-                                     float *__restrict__ il) {
+// both float64 vectors of state blockIdx.y -> their four hi/lo planes in one launch; vec: every
+// state's x_re and x_im are 16-byte aligned, so pairs of values move as double2 -> float2.  State q reads
+// at q * ldx and writes at q * 4 np (planes re hi, re lo, im hi, im lo of np values).
+__global__ void f2_split_pair_kernel(const double *__restrict__ xr, const double *__restrict__ xi, int64_t n, int64_t ldx,
+                                     int vec, float *__restrict__ planes, int64_t np) {
+    xr += blockIdx.y * ldx;
+    xi += blockIdx.y * ldx;
+    float *rh = planes + blockIdx.y * 4 * np, *rl = rh + np, *ih = rl + np, *il = ih + np;
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
     int64_t done = 0;
     if (vec) {
@@ -147,21 +150,113 @@ __device__ __forceinline__ void f2_mac2(F2P &s, float2 ah, float2 al, float2 xh,
 // planes into L2 a few diagonals ahead measured slower on the 20-qubit XXZ chain, 216 against
 // 194 us, and was dropped.)
 
-template <int MINB>
+// The chunk of diagonals staged in sq / sb added to a thread's four rows (two F2P row pairs per
+// accumulator).  IM = false: the matrix holds no imaginary part, half the loads and half the products.
+template <bool IM>
+__device__ __forceinline__ void f2_accumulate(const int4 *sq, const int64_t *sb, int cn, int64_t r0, int lane,
+                                              const float *__restrict__ are, const float *__restrict__ aim, int64_t cap,
+                                              int64_t rows, const float *__restrict__ xrh,
+                                              const float *__restrict__ xrl, const float *__restrict__ xih,
+                                              const float *__restrict__ xil, F2P (&sr)[2], F2P (&si)[2]) {
+    constexpr int V = 4;
+    const int64_t w0 = r0 - (int64_t)V * lane;
+    const int wbit = (int)((w0 >> 5) & 31);  // the warp's 128 rows: 4 tiles, bits wbit .. wbit + 3
+    for (int k = 0; k < cn; ++k) {
+        const int4 q = sq[k];
+        const int64_t lo = q.y, hi = q.z;
+        const uint32_t mword = (uint32_t)q.w;
+        // the same for the whole warp (the windows below are shuffled across its lanes)
+        if (w0 >= hi || w0 + 32 * V <= lo || !((mword >> wbit) & 0xfu)) continue;
+        const int64_t b = sb[k] + r0, c = r0 + q.x;
+        float arh[V], arl[V], aih[V], ail[V];
+        float xrhv[V], xrlv[V], xihv[V], xilv[V];
+        if (w0 >= lo && w0 + 32 * V <= hi) {
+            // an aligned window needs no shuffle: a lane whose tile is zero drops out alone
+            if ((q.x & 3) == 0 && !((mword >> ((r0 >> 5) & 31)) & 1u)) continue;
+            load_vec_stream<float, V>(arh, are + b);
+            load_vec_stream<float, V>(arl, are + cap + b);
+            if constexpr (IM) {
+                load_vec_stream<float, V>(aih, aim + b);
+                load_vec_stream<float, V>(ail, aim + cap + b);
+            }
+            const int s = (int)(c & 3);
+            const int64_t ca = c - s;
+            shifted_window(xrhv, xrh + ca, s, lane);
+            shifted_window(xrlv, xrl + ca, s, lane);
+            shifted_window(xihv, xih + ca, s, lane);
+            shifted_window(xilv, xil + ca, s, lane);
+        } else {
+            if (r0 >= rows || r0 + V <= lo || r0 >= hi) continue;
+            load_vec_stream<float, V>(arh, are + b);
+            load_vec_stream<float, V>(arl, are + cap + b);
+            if constexpr (IM) {
+                load_vec_stream<float, V>(aih, aim + b);
+                load_vec_stream<float, V>(ail, aim + cap + b);
+            }
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const bool ok = (r0 + v >= lo) && (r0 + v < hi);
+                xrhv[v] = ok ? __ldg(xrh + c + v) : 0.f;
+                xrlv[v] = ok ? __ldg(xrl + c + v) : 0.f;
+                xihv[v] = ok ? __ldg(xih + c + v) : 0.f;
+                xilv[v] = ok ? __ldg(xil + c + v) : 0.f;
+                if (!ok) arh[v] = arl[v] = 0.f;
+                if (IM && !ok) aih[v] = ail[v] = 0.f;
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < V; v += 2) {
+            const float2 rh = make_float2(arh[v], arh[v + 1]), rl = make_float2(arl[v], arl[v + 1]);
+            const float2 xrh2 = make_float2(xrhv[v], xrhv[v + 1]), xrl2 = make_float2(xrlv[v], xrlv[v + 1]);
+            const float2 xih2 = make_float2(xihv[v], xihv[v + 1]), xil2 = make_float2(xilv[v], xilv[v + 1]);
+            if constexpr (IM) {
+                const float2 ih = make_float2(aih[v], aih[v + 1]), il = make_float2(ail[v], ail[v + 1]);
+                f2_mac2(sr[v / 2], rh, rl, xrh2, xrl2);
+                f2_mac2(sr[v / 2], neg2(ih), neg2(il), xih2, xil2);
+                f2_mac2(si[v / 2], rh, rl, xih2, xil2);
+                f2_mac2(si[v / 2], ih, il, xrh2, xrl2);
+            } else {
+                f2_mac2(sr[v / 2], rh, rl, xrh2, xrl2);
+                f2_mac2(si[v / 2], rh, rl, xih2, xil2);
+            }
+        }
+    }
+}
+
+// Whether a thread's sums hold an infinite or NaN part.
+template <int N>
+__device__ __forceinline__ bool f2_nonfinite(const F2P (&a)[N], const F2P (&b)[N]) {
+    uint32_t big = 0u;
+#pragma unroll
+    for (int v = 0; v < N; ++v) {
+        big = max(big, max(max(abs_hi(a[v].h.x), abs_hi(a[v].h.y)), max(abs_hi(a[v].l.x), abs_hi(a[v].l.y))));
+        big = max(big, max(max(abs_hi(b[v].h.x), abs_hi(b[v].h.y)), max(abs_hi(b[v].l.x), abs_hi(b[v].l.y))));
+    }
+    return any_nonfinite<float>(big);
+}
+
+// State blockIdx.y: x planes at y * 4 np, y at y * ldy.  REAL: the matrix holds no imaginary part (and
+// one chunk of metadata), half the loads and products; a warp whose sums are not finite sums again in
+// full, as the products left out would have spread an infinite or NaN x.  20-qubit chain: 100 -> 82 us.
+template <int MINB, bool REAL>
 __global__ void __launch_bounds__(kSpmvThreads, MINB)
     f2_spmv_kernel(const DiagMeta *__restrict__ meta, int nd, const float *__restrict__ are,
-                   const float *__restrict__ aim, int64_t cap, int64_t rows, const float *__restrict__ xrh,
-                   const float *__restrict__ xrl, const float *__restrict__ xih, const float *__restrict__ xil,
-                   double *__restrict__ yr, double *__restrict__ yi, const uint32_t *__restrict__ tmask, int64_t mw) {
+                   const float *__restrict__ aim, int64_t cap, int64_t rows, const float *__restrict__ planes, int64_t np,
+                   double *__restrict__ yr, double *__restrict__ yi, int64_t ldy, const uint32_t *__restrict__ tmask,
+                   int64_t mw) {
     constexpr int V = 4;
     __shared__ int4 sq[kMetaChunk];     // offset, lo, hi, mask word (the block's 1024 rows are one word)
     __shared__ int64_t sb[kMetaChunk];  // value base
     const int lane = threadIdx.x & 31;
     const int64_t r0 = ((int64_t)blockIdx.x * kSpmvThreads + threadIdx.x) * V;
     const int64_t w0 = r0 - (int64_t)V * lane;
+    const float *xrh = planes + blockIdx.y * 4 * np, *xrl = xrh + np, *xih = xrl + np, *xil = xih + np;
     F2P sr[V / 2], si[V / 2];   // rows (0, 1) and (2, 3)
+    auto clear = [&]() {
 #pragma unroll
-    for (int v = 0; v < V / 2; ++v) sr[v] = si[v] = F2P{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        for (int v = 0; v < V / 2; ++v) sr[v] = si[v] = F2P{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    };
+    clear();
     for (int c0 = 0; c0 < nd; c0 += kMetaChunk) {
         const int cn = min(kMetaChunk, nd - c0);
         __syncthreads();
@@ -173,59 +268,16 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
         }
         __syncthreads();
         if (w0 >= rows) continue;
-        const int wbit = (int)((w0 >> 5) & 31);  // the warp's 128 rows: 4 tiles, bits wbit .. wbit + 3
-        for (int k = 0; k < cn; ++k) {
-            const int4 q = sq[k];
-            const int64_t lo = q.y, hi = q.z;
-            const uint32_t mword = (uint32_t)q.w;
-            // the same for the whole warp (the windows below are shuffled across its lanes)
-            if (w0 >= hi || w0 + 32 * V <= lo || !((mword >> wbit) & 0xfu)) continue;
-            const int64_t b = sb[k] + r0, c = r0 + q.x;
-            float arh[V], arl[V], aih[V], ail[V];
-            float xrhv[V], xrlv[V], xihv[V], xilv[V];
-            if (w0 >= lo && w0 + 32 * V <= hi) {
-                // an aligned window needs no shuffle: a lane whose tile is zero drops out alone
-                if ((q.x & 3) == 0 && !((mword >> ((r0 >> 5) & 31)) & 1u)) continue;
-                load_vec_stream<float, V>(arh, are + b);
-                load_vec_stream<float, V>(arl, are + cap + b);
-                load_vec_stream<float, V>(aih, aim + b);
-                load_vec_stream<float, V>(ail, aim + cap + b);
-                const int s = (int)(c & 3);
-                const int64_t ca = c - s;
-                shifted_window(xrhv, xrh + ca, s, lane);
-                shifted_window(xrlv, xrl + ca, s, lane);
-                shifted_window(xihv, xih + ca, s, lane);
-                shifted_window(xilv, xil + ca, s, lane);
-            } else {
-                if (r0 >= rows || r0 + V <= lo || r0 >= hi) continue;
-                load_vec_stream<float, V>(arh, are + b);
-                load_vec_stream<float, V>(arl, are + cap + b);
-                load_vec_stream<float, V>(aih, aim + b);
-                load_vec_stream<float, V>(ail, aim + cap + b);
-#pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    const bool ok = (r0 + v >= lo) && (r0 + v < hi);
-                    xrhv[v] = ok ? __ldg(xrh + c + v) : 0.f;
-                    xrlv[v] = ok ? __ldg(xrl + c + v) : 0.f;
-                    xihv[v] = ok ? __ldg(xih + c + v) : 0.f;
-                    xilv[v] = ok ? __ldg(xil + c + v) : 0.f;
-                    if (!ok) arh[v] = arl[v] = aih[v] = ail[v] = 0.f;
-                }
-            }
-#pragma unroll
-            for (int v = 0; v < V; v += 2) {
-                const float2 rh = make_float2(arh[v], arh[v + 1]), rl = make_float2(arl[v], arl[v + 1]);
-                const float2 ih = make_float2(aih[v], aih[v + 1]), il = make_float2(ail[v], ail[v + 1]);
-                const float2 xrh2 = make_float2(xrhv[v], xrhv[v + 1]), xrl2 = make_float2(xrlv[v], xrlv[v + 1]);
-                const float2 xih2 = make_float2(xihv[v], xihv[v + 1]), xil2 = make_float2(xilv[v], xilv[v + 1]);
-                f2_mac2(sr[v / 2], rh, rl, xrh2, xrl2);
-                f2_mac2(sr[v / 2], neg2(ih), neg2(il), xih2, xil2);
-                f2_mac2(si[v / 2], rh, rl, xih2, xil2);
-                f2_mac2(si[v / 2], ih, il, xrh2, xrl2);
-            }
+        if constexpr (REAL) {
+            f2_accumulate<false>(sq, sb, cn, r0, lane, are, aim, cap, rows, xrh, xrl, xih, xil, sr, si);
+            if (!__any_sync(0xffffffffu, f2_nonfinite(sr, si))) continue;
+            clear();
         }
+        f2_accumulate<true>(sq, sb, cn, r0, lane, are, aim, cap, rows, xrh, xrl, xih, xil, sr, si);
     }
     if (r0 >= rows) return;
+    yr += blockIdx.y * ldy;
+    yi += blockIdx.y * ldy;
 #pragma unroll
     for (int v = 0; v < V; ++v)
         if (r0 + v < rows) {
@@ -233,6 +285,94 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
             yr[r0 + v] = (double)((v & 1) ? a.h.y : a.h.x) + (double)((v & 1) ? a.l.y : a.l.x);
             yi[r0 + v] = (double)((v & 1) ? b.h.y : b.h.x) + (double)((v & 1) ? b.l.y : b.l.x);
         }
+}
+
+// The real and imaginary sum of one row, in the two lanes of packed instructions: the arithmetic (and
+// the bits) of f2_mac2.  (re, im) += (ah, al) * (x, y)
+struct F2Row {
+    float2 h, l;
+};
+__device__ __forceinline__ void f2_mac_row(F2Row &s, float2 ah, float2 al, float2 xh, float2 xl) {
+    F2P t{s.h, s.l};
+    f2_mac2(t, ah, al, xh, xl);
+    s = F2Row{t.h, t.l};
+}
+
+// One row per thread in blocks of 64, for few rows x states (see dia_spmv_row_kernel): ballots find the
+// diagonals that hold a real or an imaginary nonzero in the warp's 32 rows, the loads of U of them are
+// issued together, and a plane that is zero there takes part in no product; a warp whose sums are not
+// finite sums again in full.  Against f2_spmv_kernel, split included: 12-qubit chain 12.3 us (24.3),
+// 16-qubit Pauli sum 25.9 (74.3), 250,007 rows of 37 diagonals 35.9 (54.4), 8 states of 100,001 rows 53.6
+// (61.7); from some 800,000 rows x states on the four rows per thread are the better form (20-qubit
+// chain 93.7 against 81.8).
+constexpr int64_t kF2RowKernelMax = 786432;   // rows x states of a launch
+template <int U>
+__global__ void __launch_bounds__(64)
+    f2_spmv_row_kernel(const DiagMeta *__restrict__ meta, int nd, const float *__restrict__ are,
+                       const float *__restrict__ aim, int64_t cap, int rows, const float *__restrict__ planes, int64_t np,
+                       double *__restrict__ yr, double *__restrict__ yi, int64_t ldy, const uint32_t *__restrict__ tmask,
+                       int64_t mw) {
+    const int lane = (int)threadIdx.x & 31, r = (int)(blockIdx.x * 64 + threadIdx.x), w0 = r - lane;
+    if (w0 >= rows) return;
+    const float *xrh = planes + blockIdx.y * 4 * np + r, *xrl = xrh + np, *xih = xrl + np, *xil = xih + np;
+    const float *arh = are + r, *aih = aim + r;
+    F2Row acc;
+    for (int pass = 0;; ++pass) {
+        acc = F2Row{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        for (int c0 = 0; c0 < nd; c0 += 32) {
+            int off = 0, lo = 0, hi = 0;
+            int64_t base = 0;
+            bool re = false, im = false;
+            if (c0 + lane < nd) {
+                const DiagMeta m = meta[c0 + lane];
+                off = m.off;
+                lo = (int)m.lo;
+                hi = (int)m.hi;
+                base = m.base;
+                if (w0 < hi && w0 + 32 > lo) {
+                    const int64_t at = (int64_t)(c0 + lane) * mw + (w0 >> 10);
+                    re = !tmask || (tmask[nd * mw + at] >> ((w0 >> 5) & 31)) & 1u;
+                    im = !tmask || (tmask[2 * nd * mw + at] >> ((w0 >> 5) & 31)) & 1u;
+                }
+            }
+            uint32_t mr = __ballot_sync(0xffffffffu, re), mi = __ballot_sync(0xffffffffu, im), live = mr | mi;
+            if (pass) mr = mi = live;
+            while (live) {
+                float ah[U], al[U], bh[U], bl[U];
+                float2 xh[U], xl[U];
+                uint32_t bit[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    bit[u] = live & (0u - live);
+                    const int j = live ? __ffs(live) - 1 : 0;
+                    live &= live - 1u;
+                    const int o = __shfl_sync(0xffffffffu, off, j), l = __shfl_sync(0xffffffffu, lo, j),
+                              h = __shfl_sync(0xffffffffu, hi, j);
+                    const int64_t b = __shfl_sync(0xffffffffu, base, j);
+                    const bool in = bit[u] && r >= l && r < h, inr = in && (mr & bit[u]), ini = in && (mi & bit[u]);
+                    ah[u] = inr ? __ldcs(arh + b) : 0.f;
+                    al[u] = inr ? __ldcs(arh + cap + b) : 0.f;
+                    bh[u] = ini ? __ldcs(aih + b) : 0.f;
+                    bl[u] = ini ? __ldcs(aih + cap + b) : 0.f;
+                    xh[u] = make_float2(in ? __ldg(xrh + o) : 0.f, in ? __ldg(xih + o) : 0.f);
+                    xl[u] = make_float2(in ? __ldg(xrl + o) : 0.f, in ? __ldg(xil + o) : 0.f);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (mr & bit[u]) f2_mac_row(acc, make_float2(ah[u], ah[u]), make_float2(al[u], al[u]), xh[u], xl[u]);
+                    if (mi & bit[u])   // re -= b y, im += b x
+                        f2_mac_row(acc, make_float2(-bh[u], bh[u]), make_float2(-bl[u], bl[u]),
+                                   make_float2(xh[u].y, xh[u].x), make_float2(xl[u].y, xl[u].x));
+                }
+            }
+        }
+        if (pass || !tmask) break;
+        const uint32_t big = max(max(abs_hi(acc.h.x), abs_hi(acc.h.y)), max(abs_hi(acc.l.x), abs_hi(acc.l.y)));
+        if (!__any_sync(0xffffffffu, any_nonfinite<float>(big))) break;
+    }
+    if (r >= rows) return;
+    yr[blockIdx.y * ldy + r] = (double)acc.h.x + (double)acc.l.x;
+    yi[blockIdx.y * ldy + r] = (double)acc.h.y + (double)acc.l.y;
 }
 
 __global__ void f2_from_c128_kernel(const DiagMeta *__restrict__ meta, int nd, const double *__restrict__ sre,
@@ -298,23 +438,46 @@ int f2_convert(const Matrix &src, Matrix &dst, cudaStream_t s) {
     return DIAQ_OK;
 }
 
-int f2_spmv(const Matrix &A, const double *xr, const double *xi, double *yr, double *yi, cudaStream_t s) {
-    if (A.rows == 0) return DIAQ_OK;
+int f2_spmv(const Matrix &A, int nrhs, const double *xr, const double *xi, int64_t ldx, double *yr, double *yi,
+            int64_t ldy, cudaStream_t s) {
+    if (A.rows == 0 || nrhs <= 0) return DIAQ_OK;
     const int64_t n = A.cols;
-    const int64_t np = (n + 31) / 32 * 32;  // planes 128-byte aligned: equal alignment for hi and lo
+    const int64_t np = std::max<int64_t>((n + 31) / 32 * 32, 32);  // planes 128-byte aligned: equal alignment for hi and lo
+    // up to 8 states per launch; one, if their planes do not fit
+    int k = std::min(nrhs, 8);
     float *buf = nullptr;
-    DQ_CUDA(dev_malloc_async(&buf, sizeof(float) * 4 * (size_t)std::max<int64_t>(np, 32), s));
-    float *xrh = buf, *xrl = buf + np, *xih = buf + 2 * np, *xil = buf + 3 * np;
-    const int g = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8 * num_sms()));
-    const int vec = ((uintptr_t)xr % 16 == 0) && ((uintptr_t)xi % 16 == 0);
-    f2_split_pair_kernel<<<g, 256, 0, s>>>(xr, xi, n, vec, xrh, xrl, xih, xil);
-    // four blocks per SM (64 registers): 166.8 us on the 20-qubit chain; three (80 registers)
-    // 189 us, five or six spill (252, 339 us)
-    f2_spmv_kernel<4><<<spmv_blocks(A.rows, 4), kSpmvThreads, 0, s>>>(A.d_meta, A.nd, (const float *)A.re,
-                                                                  (const float *)A.im, A.capacity, A.rows, xrh, xrl,
-                                                                  xih, xil, yr, yi, cached_tile_mask(A, s),
-                                                                  tile_mask_words(A.rows));
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = dev_malloc_async(&buf, sizeof(float) * 4 * (size_t)np * (size_t)k, s);
+    if (e == cudaErrorMemoryAllocation && k > 1) {
+        cudaGetLastError();
+        k = 1;
+        e = dev_malloc_async(&buf, sizeof(float) * 4 * (size_t)np, s);
+    }
+    if (e != cudaSuccess) return cuda_status(e, "f2 spmv workspace", __FILE__, __LINE__);
+    const uint32_t *tmask = cached_tile_mask(A, s);
+    const float *are = (const float *)A.re, *aim = (const float *)A.im;
+    const int64_t mw = tile_mask_words(A.rows);
+    for (int q = 0; q < nrhs; q += k) {
+        const int kq = std::min(k, nrhs - q);
+        const double *pr = xr + q * ldx, *pi = xi + q * ldx;
+        double *qr = yr + q * ldy, *qi = yi + q * ldy;
+        const dim3 g((unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8 * num_sms() / kq + 1)), (unsigned)kq);
+        const int vec = ((uintptr_t)pr % 16 == 0) && ((uintptr_t)pi % 16 == 0) && (kq == 1 || ldx % 2 == 0);
+        f2_split_pair_kernel<<<g, 256, 0, s>>>(pr, pi, n, ldx, vec, buf, np);
+        if (A.rows * kq <= kF2RowKernelMax) {
+            f2_spmv_row_kernel<4><<<dim3((unsigned)((A.rows + 63) / 64), (unsigned)kq), 64, 0, s>>>(
+                A.d_meta, A.nd, are, aim, A.capacity, (int)A.rows, buf, np, qr, qi, ldy, tmask, mw);
+        } else {
+            // four blocks per SM (64 registers): 82 us on the 20-qubit chain; three (78 registers) 90, five
+            // and six spill (110, 134)
+            auto go = [&](auto kernel) {
+                kernel<<<dim3(spmv_blocks(A.rows, 4), (unsigned)kq), kSpmvThreads, 0, s>>>(
+                    A.d_meta, A.nd, are, aim, A.capacity, A.rows, buf, np, qr, qi, ldy, tmask, mw);
+            };
+            if (tmask && A.real && A.nd <= kMetaChunk) go(f2_spmv_kernel<4, true>);
+            else go(f2_spmv_kernel<4, false>);
+        }
+    }
+    e = cudaGetLastError();
     cudaFreeAsync(buf, s);
     if (e != cudaSuccess) return cuda_status(e, "f2 spmv", __FILE__, __LINE__);
     return DIAQ_OK;

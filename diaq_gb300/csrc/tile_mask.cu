@@ -137,10 +137,23 @@ const uint32_t *cached_tile_mask(const Matrix &A, cudaStream_t s) {
         return nullptr;
     }
     if (A.tmask_ok) return A.tmask;
-    // (an internal matrix is used on its own stream only)
-    if (build_tile_mask(A, A.tmask, s) != DIAQ_OK || (!A.internal && cudaStreamSynchronize(s) != cudaSuccess)) {
-        cudaGetLastError();
-        return nullptr;
+    // (an internal matrix is used on its own stream only: nobody waits)
+    if (A.prec != DIAQ_C128F2) {
+        if (build_tile_mask(A, A.tmask, s) != DIAQ_OK || (!A.internal && cudaStreamSynchronize(s) != cudaSuccess)) {
+            cudaGetLastError();
+            return nullptr;
+        }
+    } else {
+        // is it real?  The flag sits behind the mask, zero since allocate(); it is only ever set, so
+        // threads that make this call at the same time agree
+        int *flag = (int *)(A.tmask + tile_mask_bytes(A.nd, A.rows) / sizeof(uint32_t)), has_im = 1;
+        if (build_tile_mask(A, A.tmask, s, flag) != DIAQ_OK ||
+            cudaMemcpyAsync(&has_im, flag, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        A.real = has_im == 0;
     }
     A.tmask_ok = true;
     return A.tmask;

@@ -23,16 +23,16 @@ def planes(rows, cols, offsets, seed, scale=0.3):
     return np.array(offsets, dtype=np.int32), np.concatenate(re), np.concatenate(im)
 
 
-def full_product(rows, cols, off, re, im, X):
-    """A x row by row with all four products of every value in a tile that holds a nonzero."""
+def full_product(rows, cols, off, re, im, X, tile=32):
+    """A x row by row with all four products of every value in a tile of rows that holds a nonzero."""
     yr, yi = np.zeros((len(X), rows)), np.zeros((len(X), rows))
     p = 0
     with np.errstate(all="ignore"):
         for d in off:
             lo, L = max(0, -d), min(rows, cols - d) - max(0, -d)
             a, b, p = re[p:p + L], im[p:p + L], p + L
-            t = (lo + np.arange(L)) // 32
-            live = np.zeros((rows + 31) // 32, dtype=bool)
+            t = (lo + np.arange(L)) // tile
+            live = np.zeros((rows + tile - 1) // tile, dtype=bool)
             np.logical_or.at(live, t, (a != 0) | (b != 0))
             keep = live[t]
             r, a, b = (lo + np.arange(L))[keep], a[keep], b[keep]
@@ -233,3 +233,35 @@ def test_real_matrices_in_the_interleaved_kernels(native, offs, k, mode, special
         got.append(np.stack([pr.cpu().numpy(), pi.cpu().numpy()]))
     assert np.array_equal(got[0], got[1], equal_nan=True)
     assert np.array_equal(got[0], want, equal_nan=True)
+
+
+@pytest.mark.parametrize("rows,cols,offs,real", [(3001, 2990, [0, 1, -1, 36, -37, 700, -701, 1501, 64], False),
+                                                 (1100, 1100, MANY, False), (33, 40, [0, 2, -3], True),
+                                                 (800003, 800001, [0, 3, -70001], True),
+                                                 (800003, 800001, [0, 3, -70001], False)])
+@pytest.mark.parametrize("k", [1, 3])
+@pytest.mark.parametrize("special", [False, True])
+def test_float_pair_products_are_the_full_products(native, rows, cols, offs, real, k, special):
+    """Float pairs, both kernels, one and three states: the values, and non-finite results where the
+    full product has them (TwoSum turns an infinity into NaN).  The kernel with four rows per thread
+    takes a zero tile along when its strip of 128 rows is live and the offset is not a multiple of 4:
+    0 * infinity may show in such a strip, and nowhere else."""
+    import torch
+
+    capi, _ = native
+    off, re, im = planes(rows, cols, offs, 13)
+    if real:
+        im[:] = 0
+    M = capi.Matrix.create(rows, cols, off, re, im, precision=capi.C128F2)
+    X = vectors(k, cols, 3, special)
+    xr, xi = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (X.real, X.imag))
+    yr, yi = torch.empty(k, rows, device="cuda", dtype=torch.float64), torch.empty(k, rows, device="cuda", dtype=torch.float64)
+    capi.check(capi.lib().diaq_spmm(M.h, k, xr.data_ptr(), xi.data_ptr(), cols, yr.data_ptr(), yi.data_ptr(), rows, None))
+    strips = full_product(rows, cols, off, re, im, X, tile=128)
+    for got, w, ws in zip((yr, yi), full_product(rows, cols, off, re, im, X), strips):
+        got = got.cpu().numpy()
+        assert not np.isfinite(got[~np.isfinite(w)]).any()
+        assert np.isfinite(got[np.isfinite(ws)]).all()
+        ok = np.isfinite(ws)
+        assert maxrel(got[ok], w[ok]) < 1e-12   # 2^-48 per value, up to 290 of them
+        assert ok.all() != special
