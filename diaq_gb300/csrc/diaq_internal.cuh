@@ -187,7 +187,9 @@ int f2_spmv(const Matrix &A, int nrhs, const double *xr, const double *xi, int64
 
 // Copy of A in precision prec / A without its exact-zero diagonals (new matrices).
 int copy_as(const Matrix &A, int prec, cudaStream_t s, Matrix **out, bool internal = false);
-int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out, bool internal = false);
+int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out);
+// Prunes an internal matrix; the matrix itself when there is nothing to drop.
+int prune_internal(Matrix **M, cudaStream_t s);
 void destroy(Matrix *M);
 
 }  // namespace diaq_gb300

@@ -162,8 +162,9 @@ int plan_layout(Matrix &M, int64_t rows, int64_t cols, int32_t nd, const int32_t
     M.nd = nd;
     M.off.assign(off, off + nd);
     M.meta.resize(nd);
-    std::unordered_set<int32_t> seen;
-    seen.reserve(nd * 2 + 1);
+    const bool ascending = std::adjacent_find(off, off + nd, [](int32_t a, int32_t b) { return a >= b; }) == off + nd;
+    std::unordered_set<int32_t> seen;   // (ascending offsets are distinct)
+    if (!ascending) seen.reserve(nd * 2 + 1);
     int64_t cursor = kAlign, pstart = 0;
     for (int32_t k = 0; k < nd; ++k) {
         const int64_t d = off[k];
@@ -171,7 +172,7 @@ int plan_layout(Matrix &M, int64_t rows, int64_t cols, int32_t nd, const int32_t
             return set_error(DIAQ_ERR_INVALID, "diagonal offset " + std::to_string(d) +
                                                    " lies outside a " + std::to_string(rows) + " x " +
                                                    std::to_string(cols) + " matrix");
-        if (!seen.insert(off[k]).second)
+        if (!ascending && !seen.insert(off[k]).second)
             return set_error(DIAQ_ERR_INVALID, "diagonal offset " + std::to_string(d) + " appears twice");
         const int64_t len = diag_len(rows, cols, d);
         const int64_t lo = d < 0 ? -d : 0;
@@ -492,9 +493,9 @@ int copy_as(const Matrix &A, int prec, cudaStream_t s, Matrix **out, bool intern
     return DIAQ_OK;
 }
 
-int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out, bool internal) {
-    if (A.prec == DIAQ_C128F2) return set_error(DIAQ_ERR_UNSUPPORTED, "prune: convert a c128f2 matrix to c128 first");
-    std::vector<int32_t> flag(A.nd, 1);
+// flag[k]: diagonal k of A holds a value other than exact zero.  Waits for s.
+static int nonzero_diagonals(const Matrix &A, cudaStream_t s, std::vector<int32_t> &flag) {
+    flag.assign((size_t)A.nd, 1);
     if (A.nd > 0) {
         int32_t *d_flag = nullptr;
         DQ_CUDA(dev_malloc_async(&d_flag, sizeof(int32_t) * A.nd, s));
@@ -509,6 +510,30 @@ int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out, bool internal) {
         cudaFreeAsync(d_flag, s);
         if (e != cudaSuccess) return cuda_status(e, "prune flags", __FILE__, __LINE__);
     }
+    return DIAQ_OK;
+}
+
+static int keep_diagonals(const Matrix &A, const std::vector<int32_t> &flag, cudaStream_t s, Matrix **out, bool internal);
+
+int prune_matrix(const Matrix &A, cudaStream_t s, Matrix **out) {
+    if (A.prec == DIAQ_C128F2) return set_error(DIAQ_ERR_UNSUPPORTED, "prune: convert a c128f2 matrix to c128 first");
+    std::vector<int32_t> flag;
+    DQ_TRY(nonzero_diagonals(A, s, flag));
+    return keep_diagonals(A, flag, s, out, false);
+}
+
+int prune_internal(Matrix **M, cudaStream_t s) {
+    std::vector<int32_t> flag;
+    DQ_TRY(nonzero_diagonals(**M, s, flag));
+    if (std::find(flag.begin(), flag.end(), 0) == flag.end()) return DIAQ_OK;   // nothing to drop, nothing to copy
+    Matrix *P = nullptr;
+    DQ_TRY(keep_diagonals(**M, flag, s, &P, true));
+    destroy(*M);
+    *M = P;
+    return DIAQ_OK;
+}
+
+static int keep_diagonals(const Matrix &A, const std::vector<int32_t> &flag, cudaStream_t s, Matrix **out, bool internal) {
     std::vector<int32_t> keep_off, map;
     for (int32_t k = 0; k < A.nd; ++k)
         if (flag[k]) {

@@ -534,14 +534,8 @@ int spgemm(const Matrix &A, const Matrix &B, bool prune, cudaStream_t s, Matrix 
     DQ_TRY(make_zero(A.rows, B.cols, (int32_t)offC.size(), offC.data(), A.prec, s, &C, false, internal || prune));
     int st = spgemm_numeric(A, B, *C, s);
     if (st == DIAQ_OK) st = zero_gaps(*C, s);
-    if (st == DIAQ_OK && prune) {
-        Matrix *P = nullptr;
-        st = prune_matrix(*C, s, &P, internal);
-        if (st == DIAQ_OK) {
-            destroy(C);
-            C = P;
-        }
-    }
+    if (st == DIAQ_OK && prune) st = prune_internal(&C, s);
+    if (st == DIAQ_OK && !internal) st = publish(*C);
     if (st == DIAQ_OK && !internal) {
         const cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) st = cuda_status(e, "spgemm", __FILE__, __LINE__);
