@@ -252,20 +252,24 @@ __device__ __forceinline__ void il_accumulate32(const int4 *sq, const int64_t *s
                                                 const float *xr, const float *xi,
                                                 float (&accr)[G], float (&acci)[G]) {
     const int tbit = (r >> 5) & 31;
-    // unrolled by 2: 93.1 us per 8-state Horner term on the 20-qubit chain (1 and 4: 95.0 and 93.9)
-#pragma unroll 2
+    // the window's quads by float4 index: tile (c / 32) * quads * 32 + c % 32 = (c & ~31) (quads - 1) + c
+    const float4 *px = reinterpret_cast<const float4 *>(xr) + g0 * 32, *py = reinterpret_cast<const float4 *>(xi) + g0 * 32;
+    const int more = quads - 1;
+    // unrolled by 2: 93.1 us per 8-state Horner term on the 20-qubit chain (1 and 4: 95.0 and 93.9), the
+    // chained kernels' 4-state form by 4 (14.5 us per term of 4 states of a 15-qubit Pauli sum; by 2 15.1)
+    constexpr int kUnroll = CHAINED && G == 4 ? 4 : 2;
+#pragma unroll kUnroll
     for (int k = 0; k < cn; ++k) {
         const int4 q = sq[k];
         if (r < q.y || r >= q.z || !(((uint32_t)q.w >> tbit) & 1u)) continue;
         const int64_t vb = sb[k] + r;
         const float a = __ldcs(are + vb), b = REAL ? 0.f : __ldcs(aim + vb);
-        const int c = r + q.x;
+        const int c = r + q.x, at = (c & ~31) * more + c;
         IlWindow<G> w;
 #pragma unroll
         for (int h = 0; h < G / 4; ++h) {
-            const int at = ((((c >> 5) * quads) + g0 + h) << 7) + ((c & 31) << 2);
-            w.x[h] = load_state<CHAINED>(reinterpret_cast<const float4 *>(xr + at));
-            w.y[h] = load_state<CHAINED>(reinterpret_cast<const float4 *>(xi + at));
+            w.x[h] = load_state<CHAINED>(px + at + 32 * h);
+            w.y[h] = load_state<CHAINED>(py + at + 32 * h);
         }
         il_fma<G, PACKED, true, !REAL>(a, b, w, accr, acci);
     }
