@@ -252,14 +252,15 @@ struct __align__(16) CDiag {
     int32_t lo, hi, pad[2];
 };
 
+// (Streaming stores: the products that matter are far larger than L2; 18-qubit H H 1,659 -> 1,597 us.)
 template <typename T, int V>
 __device__ __forceinline__ void store_rows(T *__restrict__ p, int64_t lo, int64_t hi, int64_t r0, const T (&v)[V]) {
     if (r0 >= lo && r0 + V <= hi) {
         using VT = typename Vec<T, V>::type;
         if constexpr (V == 2)
-            *reinterpret_cast<VT *>(p + r0) = VT{v[0], v[1]};
+            __stcs(reinterpret_cast<VT *>(p + r0), VT{v[0], v[1]});
         else
-            *reinterpret_cast<VT *>(p + r0) = VT{v[0], v[1], v[2], v[3]};
+            __stcs(reinterpret_cast<VT *>(p + r0), VT{v[0], v[1], v[2], v[3]});
     } else {
 #pragma unroll
         for (int i = 0; i < V; ++i)
@@ -491,11 +492,11 @@ int spgemm_numeric(const Matrix &A, const Matrix &B, Matrix &C, cudaStream_t s) 
         int64_t maxrows = 1;
         for (const auto &m : C.meta) maxrows = std::max(maxrows, m.hi);
         const int V = A.prec == DIAQ_C128 ? 2 : 4;
-        // runs of C diagonals per block: 64 of them, or more where the rows are few -- some 32 blocks
-        // per SM, as the pairs per diagonal vary (1,024 rows, 2,047 diagonals squared: 8.8 ms; 9.4
-        // with half as many runs, 19.9 with 64)
+        // runs of C diagonals per block: 16 of them (18-qubit H H, whole call: 1,604 us; 32 runs 1,625, 64
+        // 1,659, 128 1,735), or more where the rows are few -- some 32 blocks per SM, as the pairs per
+        // diagonal vary (1,024 rows, 2,047 diagonals squared: 8.8 ms; 9.4 with half as many runs)
         const unsigned gx = spmv_blocks(maxrows, V);
-        const int64_t runs = std::min<int64_t>(C.nd, std::max<int64_t>(64, std::min<int64_t>(65535, 32 * (int64_t)num_sms() / gx)));
+        const int64_t runs = std::min<int64_t>(C.nd, std::max<int64_t>(16, std::min<int64_t>(65535, 32 * (int64_t)num_sms() / gx)));
         const int chunk = (int)((C.nd + runs - 1) / runs);
         const dim3 grid(gx, (unsigned)((C.nd + chunk - 1) / chunk));
         // the operands' masks (both or neither); taken here, outside any graph capture
