@@ -50,7 +50,7 @@ namespace diaq_gb300 {
 // ---- epilogues ---------------------------------------------------------------------------------------
 // Plain term: term = (-i*scale) * (A x); out = base + term, base = init (first term) or `in`.
 struct EpiPlain {
-    static constexpr bool kChained = true;
+    static constexpr bool kChained = true, kSplit = true;
     double *tr, *ti;              // term out (NULL on a sub-step's last term: nobody reads it)
     const double *br, *bi;        // base of the sum
     double *outr, *outi;          // sum out
@@ -95,7 +95,7 @@ struct EpiPlain {
 //   k <  m:  vout = t;
 //   k == m:  psi += (double)hi + (double)lo;  vout = fp32(psi)  (next sub-step's input).
 struct EpiMixed {
-    static constexpr bool kChained = true;
+    static constexpr bool kChained = true, kSplit = false;
     float *vr, *vi;                     // vout
     float *hr, *hi_, *lr, *li;          // compensated sum (hi, lo), re and im
     double *pr, *pi;                    // state
@@ -166,7 +166,7 @@ struct EpiMixed {
 // carry no float64 code); -1: the runtime field `last` decides.
 template <int LAST = -1>
 struct EpiHornerP {
-    static constexpr bool kChained = true;
+    static constexpr bool kChained = true, kSplit = false;
     float *wr, *wi;                 // w out
     const float *fr, *fi;           // fp32(psi)
     double *pr, *pi;                // psi

@@ -490,6 +490,126 @@ __global__ void __launch_bounds__(NT)
     if (r < rows) epi.template apply<T, K, 1>(r, rows, kq, accr, acci);
 }
 
+// One row per lane, the diagonals dealt out to the four warps of a block (warp w takes slots w, w + 4,
+// ...), for the smallest matrices: there one warp per scheduler works through its rows' diagonals alone,
+// an instruction every ten cycles or so.  The warps' partial sums are added in a fixed order, so the rounding
+// differs from the other kernels' in the last bit; epilogues whose results are compared bit by bit across
+// kernels keep to those (Epi::kSplit).  Metadata and masks are read by the lanes, a diagonal each, before
+// dependency_wait.
+//
+// Against dia_spmv_row_kernel: 12-qubit Pauli sum (60 diagonals), c128, 9.2 us against 13.3; 120 terms of
+// the evolution under a 13-qubit one 972 against 1,348, under the 12-qubit Ising chain 580 against 612.  The
+// line (rows x state chunks): float64 is bound by FP64 issue from there on (14-qubit XXZ chain, 120
+// terms: 753 against 624), float32 gains further (5 states of a 13-qubit Pauli sum: 8.7 against 14.4).
+template <typename T>
+constexpr int64_t kSplitKernelMax = sizeof(T) == 8 ? 8192 : 32768;
+
+template <typename T, int K, int U, class Epi>
+__global__ void __launch_bounds__(128)
+    dia_spmv_split_kernel(const DiagMeta *__restrict__ meta, int nd, const T *__restrict__ are,
+                          const T *__restrict__ aim, int rows, const T *xr, const T *xi, int64_t ldx, int nrhs,
+                          int nchunk, const uint32_t *__restrict__ tmask, int64_t mw, Epi epi0) {
+    __shared__ T part[3][2 * K][32];
+    const int chunk = (int)(blockIdx.x % (unsigned)nchunk), tile = blockIdx.x / (unsigned)nchunk;
+    const int q0 = chunk * K, kq = min(K, nrhs - q0);
+    const Epi epi = epi0.shifted(q0);
+    const int lane = (int)threadIdx.x & 31, w = (int)threadIdx.x >> 5;
+    const int r = tile * 32 + lane, w0 = tile * 32;
+    xr += q0 * ldx + r;
+    xi += q0 * ldx + r;
+    are += r;
+    aim += r;
+    T accr[K][1], acci[K][1];
+    for (int pass = 0;; ++pass) {   // a second pass, with both planes, for rows that are not finite
+#pragma unroll
+        for (int k = 0; k < K; ++k) accr[k][0] = acci[k][0] = (T)0;
+        for (int c0 = w; c0 < nd; c0 += 128) {
+            const int d = c0 + 4 * lane;
+            int off = 0, lo = 0, hi = 0;
+            int64_t base = 0;
+            bool re = false, im = false;
+            if (d < nd) {
+                const DiagMeta m = meta[d];
+                off = m.off;
+                lo = (int)m.lo;
+                hi = (int)m.hi;
+                base = m.base;
+                const int64_t at = (int64_t)d * mw + (w0 >> 10);
+                const uint32_t wr = tmask ? tmask[nd * mw + at] : 0xffffffffu, wi = tmask ? tmask[2 * nd * mw + at] : 0xffffffffu;
+                if (w0 < hi && w0 + 32 > lo) {
+                    re = (wr >> ((w0 >> 5) & 31)) & 1u;
+                    im = (wi >> ((w0 >> 5) & 31)) & 1u;
+                }
+            }
+            uint32_t mr = __ballot_sync(0xffffffffu, re), mi = __ballot_sync(0xffffffffu, im), live = mr | mi;
+            if (pass) mr = mi = live;
+            if constexpr (Epi::kChained) dependency_wait();
+            while (live) {
+                T a[U], b[U], x[U][K], y[U][K];
+                uint32_t bit[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    bit[u] = live & (0u - live);
+                    if (!live) continue;
+                    const int j = __ffs(live) - 1;
+                    live &= live - 1u;
+                    const int o = __shfl_sync(0xffffffffu, off, j), l = __shfl_sync(0xffffffffu, lo, j),
+                              h = __shfl_sync(0xffffffffu, hi, j);
+                    const int64_t vb = __shfl_sync(0xffffffffu, base, j);
+                    const bool ok = r >= l && r < h;
+                    a[u] = ok && (mr & bit[u]) ? __ldcs(are + vb) : (T)0;
+                    b[u] = ok && (mi & bit[u]) ? __ldcs(aim + vb) : (T)0;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        if (k >= kq) break;
+                        x[u][k] = ok ? load_state<Epi::kChained>(xr + k * ldx + o) : (T)0;
+                        y[u][k] = ok ? load_state<Epi::kChained>(xi + k * ldx + o) : (T)0;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (mr & bit[u])
+#pragma unroll
+                        for (int k = 0; k < K; ++k) {
+                            if (k >= kq) break;
+                            accr[k][0] = fma(a[u], x[u][k], accr[k][0]);
+                            acci[k][0] = fma(a[u], y[u][k], acci[k][0]);
+                        }
+                    if (mi & bit[u])
+#pragma unroll
+                        for (int k = 0; k < K; ++k) {
+                            if (k >= kq) break;
+                            accr[k][0] = fma(-b[u], y[u][k], accr[k][0]);
+                            acci[k][0] = fma(b[u], x[u][k], acci[k][0]);
+                        }
+                }
+            }
+        }
+        if constexpr (Epi::kChained) dependency_wait();   // (a warp without diagonals has not waited yet)
+        if (w > 0)
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                part[w - 1][2 * k][lane] = accr[k][0];
+                part[w - 1][2 * k + 1][lane] = acci[k][0];
+            }
+        __syncthreads();
+        bool again = false;
+        if (w == 0) {
+            uint32_t big = 0u;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                accr[k][0] = (accr[k][0] + part[0][2 * k][lane]) + (part[1][2 * k][lane] + part[2][2 * k][lane]);
+                acci[k][0] = (acci[k][0] + part[0][2 * k + 1][lane]) + (part[1][2 * k + 1][lane] + part[2][2 * k + 1][lane]);
+                big = max(big, max(abs_hi(accr[k][0]), abs_hi(acci[k][0])));
+            }
+            again = any_nonfinite<T>(big);
+        }
+        if (pass || !tmask || !__syncthreads_or(again)) break;
+    }
+    if constexpr (Epi::kChained) dependents_go();
+    if (w == 0 && r < rows) epi.template apply<T, K, 1>(r, rows, kq, accr, acci);
+}
+
 // ---- float variant with L2 prefetch of the matrix and shuffled state windows ----------------------
 //
 // The register kernel above waits, on every diagonal, for the HBM latency of its matrix vector:
@@ -655,10 +775,11 @@ inline bool pf_kernel_fits(const Matrix &A, const float *xr, const float *xi, in
            (reinterpret_cast<uintptr_t>(xi) & 15) == 0;
 }
 
-// Store y = A x.  (kChained: whether kernels with this epilogue are launched with launch_chained.)
+// Store y = A x.  (kChained: whether kernels with this epilogue are launched with launch_chained; kSplit:
+// whether dia_spmv_split_kernel may run them.)
 template <typename T>
 struct EpiStore {
-    static constexpr bool kChained = false;
+    static constexpr bool kChained = false, kSplit = true;
     T *yr, *yi;
     int64_t ldy;
     template <typename U, int K, int V>
@@ -699,7 +820,7 @@ struct EpiStore {
 // state itself, saving the copy).  Vectors and accumulator of type T.
 template <typename T>
 struct EpiTaylor {
-    static constexpr bool kChained = true;
+    static constexpr bool kChained = true, kSplit = true;
     T *tr, *ti;      // term out
     T *accr, *acci;  // running sum
     const T *initr, *initi;
@@ -757,6 +878,14 @@ void launch_vr(int vr, const Matrix &A, const T *xr, const T *xi, int64_t ldx, i
     if constexpr (VR == 1 && K <= 2) {
         constexpr int NT = 64, U = K == 1 ? 4 : 2;
         const int64_t blocks = (A.rows + NT - 1) / NT * nchunk;
+        if constexpr (Epi::kSplit) {
+            if (A.rows * nchunk <= kSplitKernelMax<T>) {
+                launch_chained(chained, dia_spmv_split_kernel<T, K, U, Epi>, (unsigned)((A.rows + 31) / 32 * nchunk), 128, s,
+                               A.d_meta, A.nd, (const T *)A.re, (const T *)A.im, (int)A.rows, xr, xi, ldx, nrhs, nchunk,
+                               tmask, tile_mask_words(A.rows), e);
+                return;
+            }
+        }
         if (A.rows * nchunk <= kRowKernelMax<T>) {
             launch_chained(chained, dia_spmv_row_kernel<T, K, NT, U, Epi>, (unsigned)blocks, NT, s, A.d_meta, A.nd,
                            (const T *)A.re, (const T *)A.im, (int)A.rows, xr, xi, ldx, nrhs, nchunk, tmask,

@@ -90,6 +90,15 @@ def test_products_are_the_full_products(native, rows, cols, offs, prec, k, speci
             assert not ok.all()
 
 
+@pytest.mark.parametrize("rows,cols,offs", [(9001, 9005, [0, 1, -1, 36, -37, 700, -701, 1501, 64]), (70003, 70001, [0, 3, -64]),
+                                            (270011, 270011, [0, -7, 1024])])
+@pytest.mark.parametrize("prec,k", [(0, 1), (0, 3), (1, 1), (1, 5)])
+@pytest.mark.parametrize("special", [False, True])
+def test_larger_products_are_the_full_products(native, rows, cols, offs, prec, k, special):
+    """The same through the kernels for more rows."""
+    test_products_are_the_full_products(native, rows, cols, offs, prec, k, special)
+
+
 def _evolve(capi, H, N, X, mode, cfg):
     import torch
 
