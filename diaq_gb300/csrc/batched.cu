@@ -79,7 +79,9 @@ __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, 
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 
 // phase < 0: initialise v_a = T(psi) for every item.
-template <typename T, int K, int VR>
+// CHAINED: launched with launch_chained; every block waits for its predecessor before it touches a
+// vector, and before it ends.
+template <typename T, int K, int VR, bool CHAINED>
 __global__ void __launch_bounds__(kSpmvThreads)
     batched_phase_kernel(const BatchInst *__restrict__ insts, const BatchItem *__restrict__ items, int n_items,
                          int phase) {
@@ -101,6 +103,7 @@ __global__ void __launch_bounds__(kSpmvThreads)
             const bool init = phase < 0;
             const bool copy = !init && phase == I.sub * I.m && (I.phases > I.sub * I.m);
             if (!init && !copy) continue;
+            if constexpr (CHAINED) dependency_wait();
             for (int q = 0; q < kq; ++q)
                 for (int v = 0; v < VR; ++v) {
                     const int64_t r = r0 + v;
@@ -157,6 +160,7 @@ __global__ void __launch_bounds__(kSpmvThreads)
                         sb[j] = m.base;
                     }
                     __syncthreads();
+                    if constexpr (CHAINED) dependency_wait();
                 }
                 if (r0 >= I.rows) continue;
                 const int tbit = (int)((r0 >> 5) & 31);
@@ -165,9 +169,9 @@ __global__ void __launch_bounds__(kSpmvThreads)
                     const int64_t lo = q.y, hi = q.z;
                     if (r0 + VR <= lo || r0 >= hi || !(((uint32_t)q.w >> tbit) & 1u)) continue;
                     if (real)
-                        dia_mac<T, K, VR, true, false, false>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
+                        dia_mac<T, K, VR, true, false, CHAINED>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
                     else
-                        dia_mac<T, K, VR, true, true, false>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
+                        dia_mac<T, K, VR, true, true, CHAINED>(q, sb[j], r0, are, aim, xr, xi, ld, kq, accr, acci);
                 }
             }
             if (!real) break;
@@ -247,12 +251,13 @@ __global__ void __launch_bounds__(kSpmvThreads)
             }
         }
     }
+    if constexpr (CHAINED) dependency_wait();
 }
 
 // One item of an interleaved instance: row block `tile` (32 * 8 / (sp / G) rows) and all sp
 // states.  Phases as in batched_phase_kernel; the initialisation and copy phases move the item's
 // rows of every state, which are one contiguous range of the tiled vectors.
-template <int G, bool HORNER>
+template <int G, bool HORNER, bool CHAINED>
 __device__ __forceinline__ void batched_il_item(const BatchInst &I, int4 *sq, int64_t *sb, int64_t tile,
                                                 int phase) {
     const int quads = I.sp >> 2, groups = I.sp / G;
@@ -262,6 +267,7 @@ __device__ __forceinline__ void batched_il_item(const BatchInst &I, int4 *sq, in
     if (phase < 0 || phase >= I.sub * I.m) {
         const bool init = phase < 0;
         const bool copy = !init && phase == I.sub * I.m && (I.phases > I.sub * I.m);
+        if constexpr (CHAINED) dependency_wait();
         if (!init && !copy) return;
         const int64_t e1 = min(r0 + rpb, I.n_pad) * I.sp;
         for (int64_t e = r0 * I.sp + threadIdx.x; e < e1; e += blockDim.x) {
@@ -325,14 +331,19 @@ __device__ __forceinline__ void batched_il_item(const BatchInst &I, int4 *sq, in
                                   block_tile_bits((uint32_t)q.w, r0, 8 / groups), r0);
             }
         }
+        if constexpr (CHAINED) dependency_wait();
         if (r >= I.rows) continue;
         if (real) {
-            il_accumulate32<G, false, true>(sq, sb, cn, (int)r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+            il_accumulate32<G, false, true, CHAINED>(sq, sb, cn, (int)r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
             if (!il_nonfinite<G>(accr, acci)) continue;
 #pragma unroll
             for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;   // not finite: sum again, in full
         }
-        il_accumulate32<G>(sq, sb, cn, (int)r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+        il_accumulate32<G, false, false, CHAINED>(sq, sb, cn, (int)r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
+    }
+    if constexpr (CHAINED) {
+        if (I.nd == 0) dependency_wait();
+        dependents_go();
     }
     if (r >= I.rows) return;
     if constexpr (HORNER) {  // the last step reads w_1, not fp32(psi): refreshing v_a there is safe
@@ -362,7 +373,7 @@ __device__ __forceinline__ void batched_il_item(const BatchInst &I, int4 *sq, in
 // 5,904 at four, 5,543 at eight, whose spills cost more than the occupancy gains), the
 // compensated form at five (5,759; 5,637 at six); with the compact metadata loop
 // (il_accumulate32) 7,571 and 6,091.
-template <int G, bool HORNER>
+template <int G, bool HORNER, bool CHAINED>
 __global__ void __launch_bounds__(kSpmvThreads, HORNER ? 6 : 5)
     batched_il_kernel(const BatchInst *__restrict__ insts, const BatchItem *__restrict__ items, int phase) {
     __shared__ int4 sq[kMetaChunk];
@@ -371,7 +382,7 @@ __global__ void __launch_bounds__(kSpmvThreads, HORNER ? 6 : 5)
     const BatchItem item = items[blockIdx.x];
     if (threadIdx.x == 0) si = insts[item.inst];
     __syncthreads();
-    batched_il_item<G, HORNER>(si, sq, sb, item.tile, phase);
+    batched_il_item<G, HORNER, CHAINED>(si, sq, sb, item.tile, phase);
 }
 
 struct Batch {
@@ -479,59 +490,76 @@ static int build_items(Batch &B) {
     return DIAQ_OK;
 }
 
+// Chained kernels (coherent state loads) are for batches that leave the GPU room, as in the plans: 3
+// chains of 8 qubits, 2 steps of 8 terms: 170 -> 142 us; 28 of 8-12 qubits: 222 -> 207; 24 of 10-17 qubits
+// (2,830 blocks a phase) would lose: 1,225 -> 1,321.
+static bool few_blocks(const Batch &B) { return B.n_items + B.n_il_items <= 8 * num_sms(); }
+
 template <typename T, int K, int VR>
-static int launch_phase_t(const Batch &B, int phase, cudaStream_t s) {
+static int launch_phase_t(const Batch &B, int phase, cudaStream_t s, bool chained) {
     if (B.n_items == 0) return DIAQ_OK;
     static int blocks_per_sm = 0;
     if (blocks_per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, batched_phase_kernel<T, K, VR>, kSpmvThreads, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, batched_phase_kernel<T, K, VR, false>, kSpmvThreads, 0);
         if (blocks_per_sm < 1) blocks_per_sm = 1;
     }
     const int grid = std::max(1, std::min(B.n_items, blocks_per_sm * num_sms()));
-    batched_phase_kernel<T, K, VR><<<grid, kSpmvThreads, 0, s>>>(B.d_inst, B.d_items, B.n_items, phase);
+    if (few_blocks(B))
+        launch_chained(chained, batched_phase_kernel<T, K, VR, true>, (unsigned)grid, kSpmvThreads, s, B.d_inst, B.d_items,
+                       B.n_items, phase);
+    else
+        batched_phase_kernel<T, K, VR, false><<<grid, kSpmvThreads, 0, s>>>(B.d_inst, B.d_items, B.n_items, phase);
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
 
 template <typename T, int K>
-static int launch_phase_k(const Batch &B, int phase, cudaStream_t s) {
+static int launch_phase_k(const Batch &B, int phase, cudaStream_t s, bool chained) {
     switch (vr_of(B)) {
-        case 1: return launch_phase_t<T, K, 1>(B, phase, s);
-        case 2: return launch_phase_t<T, K, 2>(B, phase, s);
+        case 1: return launch_phase_t<T, K, 1>(B, phase, s, chained);
+        case 2: return launch_phase_t<T, K, 2>(B, phase, s, chained);
         default:
-            if constexpr (sizeof(T) == 4) return launch_phase_t<T, K, 4>(B, phase, s);
-            return launch_phase_t<T, K, 2>(B, phase, s);
+            if constexpr (sizeof(T) == 4) return launch_phase_t<T, K, 4>(B, phase, s, chained);
+            return launch_phase_t<T, K, 2>(B, phase, s, chained);
     }
 }
 
 template <typename T>
-static int launch_phase(const Batch &B, int phase, cudaStream_t s) {
+static int launch_phase(const Batch &B, int phase, cudaStream_t s, bool chained) {
     switch (B.cfg.kmax) {
-        case 1: return launch_phase_k<T, 1>(B, phase, s);
-        case 2: return launch_phase_k<T, 2>(B, phase, s);
-        case 4: return launch_phase_k<T, 4>(B, phase, s);
-        default: return launch_phase_k<T, 8>(B, phase, s);
+        case 1: return launch_phase_k<T, 1>(B, phase, s, chained);
+        case 2: return launch_phase_k<T, 2>(B, phase, s, chained);
+        case 4: return launch_phase_k<T, 4>(B, phase, s, chained);
+        default: return launch_phase_k<T, 8>(B, phase, s, chained);
     }
+}
+
+template <int G, bool HORNER>
+static void launch_il(const Batch &B, const BatchItem *it, int n, int phase, cudaStream_t s, bool chained) {
+    if (few_blocks(B))
+        launch_chained(chained, batched_il_kernel<G, HORNER, true>, (unsigned)n, kSpmvThreads, s, B.d_inst, it, phase);
+    else
+        batched_il_kernel<G, HORNER, false><<<n, kSpmvThreads, 0, s>>>(B.d_inst, it, phase);
 }
 
 // The kernels of one phase: 0 the planar instances, 1 .. 4 the segments of the interleaved ones.
 constexpr int kChains = 5;
 static bool chain_empty(const Batch &B, int c) { return c == 0 ? B.n_items == 0 : B.il_seg[c] == B.il_seg[c - 1]; }
-static int phase_chain(const Batch &B, int c, int p, cudaStream_t s) {
+static int phase_chain(const Batch &B, int c, int p, cudaStream_t s, bool chained) {
     if (chain_empty(B, c)) return DIAQ_OK;
-    if (c == 0) return B.prec == DIAQ_C64 ? launch_phase<float>(B, p, s) : launch_phase<double>(B, p, s);
+    if (c == 0) return B.prec == DIAQ_C64 ? launch_phase<float>(B, p, s, chained) : launch_phase<double>(B, p, s, chained);
     const BatchItem *it = B.d_il_items + B.il_seg[c - 1];
     const int n = B.il_seg[c] - B.il_seg[c - 1];
-    if (c == 1) batched_il_kernel<8, true><<<n, kSpmvThreads, 0, s>>>(B.d_inst, it, p);
-    else if (c == 2) batched_il_kernel<8, false><<<n, kSpmvThreads, 0, s>>>(B.d_inst, it, p);
-    else if (c == 3) batched_il_kernel<4, true><<<n, kSpmvThreads, 0, s>>>(B.d_inst, it, p);
-    else batched_il_kernel<4, false><<<n, kSpmvThreads, 0, s>>>(B.d_inst, it, p);
+    if (c == 1) launch_il<8, true>(B, it, n, p, s, chained);
+    else if (c == 2) launch_il<8, false>(B, it, n, p, s, chained);
+    else if (c == 3) launch_il<4, true>(B, it, n, p, s, chained);
+    else launch_il<4, false>(B, it, n, p, s, chained);
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
 
 static int phase(const Batch &B, int p, cudaStream_t s) {
-    for (int c = 0; c < kChains; ++c) DQ_TRY(phase_chain(B, c, p, s));
+    for (int c = 0; c < kChains; ++c) DQ_TRY(phase_chain(B, c, p, s, false));
     return DIAQ_OK;
 }
 
@@ -573,7 +601,7 @@ static int record_step(Batch &B) {
         if (chain_empty(B, c)) continue;
         cudaStream_t s = c == lead ? B.s : B.side[c];
         if (c != lead) DQ_CUDA(cudaStreamWaitEvent(s, B.fork, 0));
-        for (int p = 0; p < B.max_phases; ++p) DQ_TRY(phase_chain(B, c, p, s));
+        for (int p = 0; p < B.max_phases; ++p) DQ_TRY(phase_chain(B, c, p, s, p > 0));
         if (c != lead) DQ_CUDA(cudaEventRecord(B.join[c], s));
     }
     for (int c = 0; c < kChains; ++c)
