@@ -38,8 +38,8 @@ struct Mlp {
 // of W3, a strip of W1, a bias) and written once per block; mlp_reduce_kernel then sums the blocks'
 // parts.  The sum over the batch is split over up to 2 blocks per SM this way: one thread per weight
 // walking the whole batch left a chain of B dependent loads on 34 blocks: a training step of 1,024
-// rows took 544 us that way (450 of them in those launches) and takes 26 us now.  What bounds it now
-// is latency: two dependent launches with one round of 8 rows per block.
+// rows took 544 us that way (450 of them in those launches) and takes 21 us now.  What bounds it now
+// is latency: two dependent launches (chained, 26 -> 21 us) with one round of 8 rows per block.
 constexpr int kRows = 8;                       // rows per block and round: one per warp in the softmax
 constexpr int kMlpThreads = 256;
 constexpr int kLd2 = kH2 + 1;                  // W2 rows padded: read along both indices, conflict-free
@@ -50,7 +50,7 @@ struct MlpShared {  // 45 KB
     alignas(16) float x[kRows][kIn], a1[kRows][kH1], a2[kRows][kH2], lg[kRows][kOutPad], d2[kRows][kH2], d1[kRows][kH1];
 };
 
-__device__ __forceinline__ void mlp_load_weights(MlpShared &S, const float *__restrict__ p) {
+__device__ __forceinline__ void mlp_load_weights(MlpShared &S, const float *p) {
     const int t = threadIdx.x;
     for (int i = t; i < kIn * kH1; i += kMlpThreads) S.w1[i] = p[oW1 + i];
     for (int i = t; i < kH1 * kH2; i += kMlpThreads) S.w2[(i / kH2) * kLd2 + i % kH2] = p[oW2 + i];
@@ -62,7 +62,7 @@ __device__ __forceinline__ void mlp_load_weights(MlpShared &S, const float *__re
 
 // Logits of rows row0 .. row0 + kRows - 1 into S.lg (rows past B read as zeros).  Thread t works on
 // unit t % 64 of rows t / 64 and t / 64 + 4; each unit's sum runs over its inputs in order.
-__device__ __forceinline__ void mlp_forward_rows(MlpShared &S, const float *__restrict__ X, int64_t row0, int B) {
+__device__ __forceinline__ void mlp_forward_rows(MlpShared &S, const float *X, int64_t row0, int B) {
     const int t = threadIdx.x, j = t & 63, q = t >> 6;
     if (t < kRows * kIn) {
         const int64_t b = row0 + t / kIn;
@@ -158,9 +158,9 @@ __device__ __forceinline__ void outer4(float (&acc)[4][4], const float4 &u, cons
 // Per-row losses (loss may be NULL) and, per block, the gradient of the mean loss over the block's
 // rows: part[block][kParams].
 __global__ void __launch_bounds__(kMlpThreads)
-    mlp_grad_kernel(const float *__restrict__ p, const float *__restrict__ X, const int32_t *__restrict__ ys,
-                    const int32_t *__restrict__ ym, int B, float *__restrict__ loss, float *__restrict__ part) {
+    mlp_grad_kernel(const float *p, const float *X, const int32_t *ys, const int32_t *ym, int B, float *loss, float *part) {
     __shared__ MlpShared S;
+    dependency_wait();   // launched while the previous step's reduction drains
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
     mlp_load_weights(S, p);
     const int i4 = (t >> 4) * 4, j4 = (t & 15) * 4;       // tile of W2 (and of W3, j4 < 52); column strip of W1
@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(kMlpThreads)
     if (t < kH1) o[oB1 + t] = gb;
     else if (t < kH1 + kH2) o[oB2 + t - kH1] = gb;
     else if (t < kH1 + kH2 + kOut) o[oB3 + t - kH1 - kH2] = gb;
+    dependents_go();
 }
 
 // Sums the blocks' parts per parameter in a fixed order (8 slices of the blocks, then the slices),
@@ -238,8 +239,9 @@ struct AdamStep {
 };
 constexpr int kSlices = 8;
 __global__ void __launch_bounds__(32 * kSlices)
-    mlp_reduce_kernel(const float *__restrict__ part, int nblk, float *__restrict__ g, int adam, AdamStep A) {
+    mlp_reduce_kernel(const float *part, int nblk, float *g, int adam, AdamStep A) {
     __shared__ float red[kSlices][32];
+    dependency_wait();   // launched while the gradient kernel drains
     const int lane = threadIdx.x & 31, sl = threadIdx.x >> 5;
     const int i = blockIdx.x * 32 + lane;
     float s = 0.f;
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(32 * kSlices)
         for (int b = sl; b < nblk; b += kSlices) s += part[(int64_t)b * kParams + i];
     }
     red[sl][lane] = s;
+    dependents_go();
     __syncthreads();
     if (sl != 0 || i >= kParams) return;
     float gi = red[0][lane];
@@ -286,8 +289,9 @@ static int gradient(Mlp &M, const float *X, const int32_t *ys, const int32_t *ym
                     const AdamStep *adam, cudaStream_t s) {
     const int nblk = grad_blocks(B);
     DQ_TRY(ensure_work(M, nblk));
-    mlp_grad_kernel<<<nblk, kMlpThreads, 0, s>>>(M.p, X, ys, ym, B, loss, M.work);
-    mlp_reduce_kernel<<<(kParams + 31) / 32, 32 * kSlices, 0, s>>>(M.work, nblk, g, adam ? 1 : 0, adam ? *adam : AdamStep{});
+    launch_chained(true, mlp_grad_kernel, (unsigned)nblk, kMlpThreads, s, M.p, X, ys, ym, B, loss, M.work);
+    launch_chained(true, mlp_reduce_kernel, (kParams + 31) / 32, 32 * kSlices, s, M.work, nblk, g, adam ? 1 : 0,
+                   adam ? *adam : AdamStep{});
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
