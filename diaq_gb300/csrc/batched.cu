@@ -175,12 +175,15 @@ __global__ void __launch_bounds__(kSpmvThreads)
                 }
             }
             if (!real) break;
-            uint32_t big = 0u;
+            uint32_t big = 0u, small = ~0u;
 #pragma unroll
             for (int q = 0; q < K; ++q)
 #pragma unroll
-                for (int v = 0; v < VR; ++v) big = max(big, max(abs_hi(accr[q][v]), abs_hi(acci[q][v])));
-            if (!any_nonfinite<T>(big)) break;
+                for (int v = 0; v < VR; ++v) {
+                    big = max(big, max(abs_hi(accr[q][v]), abs_hi(acci[q][v])));
+                    small = min(small, min(abs_hi(accr[q][v]), abs_hi(acci[q][v])));
+                }
+            if (!unsettled<T>(big, small)) break;
         }
         if (r0 >= I.rows) continue;
         if (I.horner) {
@@ -335,7 +338,7 @@ __device__ __forceinline__ void batched_il_item(const BatchInst &I, int4 *sq, in
         if (r >= I.rows) continue;
         if (real) {
             il_accumulate32<G, false, true, CHAINED>(sq, sb, cn, (int)r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
-            if (!il_nonfinite<G>(accr, acci)) continue;
+            if (!il_unsettled<G>(accr, acci)) continue;
 #pragma unroll
             for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;   // not finite: sum again, in full
         }

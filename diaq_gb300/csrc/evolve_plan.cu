@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
         if (r >= rows) continue;
         il_accumulate32<G, true, REAL, CHAINED>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);
         if constexpr (REAL) {   // one chunk (the launcher sees to it): not finite -- sum again, in full
-            if (il_nonfinite<G>(accr, acci)) {
+            if (il_unsettled<G>(accr, acci)) {
 #pragma unroll
                 for (int q = 0; q < G; ++q) accr[q] = acci[q] = 0.f;
                 il_accumulate32<G, true, false, CHAINED>(sq, sb, cn, r, g * (G / 4), quads, are, aim, xr, xi, accr, acci);

@@ -402,10 +402,13 @@ __global__ void __launch_bounds__(kSpmvThreads, 4)
         auto finish = [&]() {
             const CDiag q = cd[c];
             if (w0 < q.hi && w0 + 32 * V > q.lo) {
-                uint32_t big = 0u;
+                uint32_t big = 0u, small = ~0u;
 #pragma unroll
-                for (int v = 0; v < V; ++v) big = max(big, max(abs_hi(accr[v]), abs_hi(acci[v])));
-                if (maskA && __any_sync(0xffffffffu, any_nonfinite<T>(big))) {
+                for (int v = 0; v < V; ++v) {
+                    big = max(big, max(abs_hi(accr[v]), abs_hi(acci[v])));
+                    small = min(small, min(abs_hi(accr[v]), abs_hi(acci[v])));
+                }
+                if (maskA && __any_sync(0xffffffffu, unsettled<T>(big, small))) {
 #pragma unroll
                     for (int v = 0; v < V; ++v) accr[v] = acci[v] = (T)0;
                     const int64_t p1 = cd[c + 1].pstart;

@@ -223,16 +223,22 @@ __device__ __forceinline__ void f2_accumulate(const int4 *sq, const int64_t *sb,
     }
 }
 
-// Whether a thread's sums hold an infinite or NaN part.
+// Whether a thread's sums have to be taken again in full (see unsettled; a NaN high part makes its low
+// part NaN).
 template <int N>
-__device__ __forceinline__ bool f2_nonfinite(const F2P (&a)[N], const F2P (&b)[N]) {
-    uint32_t big = 0u;
+__device__ __forceinline__ bool f2_unsettled(const F2P (&a)[N], const F2P (&b)[N]) {
+    uint32_t big = 0u, small = ~0u;
 #pragma unroll
     for (int v = 0; v < N; ++v) {
-        big = max(big, max(max(abs_hi(a[v].h.x), abs_hi(a[v].h.y)), max(abs_hi(a[v].l.x), abs_hi(a[v].l.y))));
-        big = max(big, max(max(abs_hi(b[v].h.x), abs_hi(b[v].h.y)), max(abs_hi(b[v].l.x), abs_hi(b[v].l.y))));
+        const uint32_t h[4] = {abs_hi(a[v].h.x), abs_hi(a[v].h.y), abs_hi(b[v].h.x), abs_hi(b[v].h.y)};
+        const uint32_t l[4] = {abs_hi(a[v].l.x), abs_hi(a[v].l.y), abs_hi(b[v].l.x), abs_hi(b[v].l.y)};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            big = max(big, max(h[i], l[i]));
+            small = min(small, h[i]);
+        }
     }
-    return any_nonfinite<float>(big);
+    return unsettled<float>(big, small);
 }
 
 // State blockIdx.y: x planes at y * 4 np, y at y * ldy.  REAL: the matrix holds no imaginary part (and
@@ -270,7 +276,7 @@ __global__ void __launch_bounds__(kSpmvThreads, MINB)
         if (w0 >= rows) continue;
         if constexpr (REAL) {
             f2_accumulate<false>(sq, sb, cn, r0, lane, are, aim, cap, rows, xrh, xrl, xih, xil, sr, si);
-            if (!__any_sync(0xffffffffu, f2_nonfinite(sr, si))) continue;
+            if (!__any_sync(0xffffffffu, f2_unsettled(sr, si))) continue;
             clear();
         }
         f2_accumulate<true>(sq, sb, cn, r0, lane, are, aim, cap, rows, xrh, xrl, xih, xil, sr, si);
@@ -368,7 +374,8 @@ __global__ void __launch_bounds__(64)
         }
         if (pass || !tmask) break;
         const uint32_t big = max(max(abs_hi(acc.h.x), abs_hi(acc.h.y)), max(abs_hi(acc.l.x), abs_hi(acc.l.y)));
-        if (!__any_sync(0xffffffffu, any_nonfinite<float>(big))) break;
+        const uint32_t small = min(abs_hi(acc.h.x), abs_hi(acc.h.y));
+        if (!__any_sync(0xffffffffu, unsettled<float>(big, small))) break;
     }
     if (r >= rows) return;
     yr[blockIdx.y * ldy + r] = (double)acc.h.x + (double)acc.l.x;

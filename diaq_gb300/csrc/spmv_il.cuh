@@ -275,13 +275,16 @@ __device__ __forceinline__ void il_accumulate32(const int4 *sq, const int64_t *s
     }
 }
 
-// Whether any of a thread's sums is infinite or NaN.
+// Whether a thread's sums have to be taken again in full (see unsettled).
 template <int G>
-__device__ __forceinline__ bool il_nonfinite(const float (&accr)[G], const float (&acci)[G]) {
-    uint32_t big = 0u;
+__device__ __forceinline__ bool il_unsettled(const float (&accr)[G], const float (&acci)[G]) {
+    uint32_t big = 0u, small = ~0u;
 #pragma unroll
-    for (int q = 0; q < G; ++q) big = max(big, max(abs_hi(accr[q]), abs_hi(acci[q])));
-    return any_nonfinite<float>(big);
+    for (int q = 0; q < G; ++q) {
+        big = max(big, max(abs_hi(accr[q]), abs_hi(acci[q])));
+        small = min(small, min(abs_hi(accr[q]), abs_hi(acci[q])));
+    }
+    return unsettled<float>(big, small);
 }
 
 }  // namespace diaq_gb300

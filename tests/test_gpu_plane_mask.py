@@ -99,6 +99,33 @@ def test_larger_products_are_the_full_products(native, rows, cols, offs, prec, k
     test_products_are_the_full_products(native, rows, cols, offs, prec, k, special)
 
 
+@pytest.mark.parametrize("rows", [70, 9001, 70003, 270011])
+@pytest.mark.parametrize("prec,k", [(0, 1), (0, 3), (1, 1)])
+def test_products_of_nan_vectors(native, rows, prec, k):
+    """Sums that are NaN in both parts are not taken twice: vectors that hold NaN in both parts, in
+    one, and infinities, in blocks (a product over several diagonals meets all mixtures)."""
+    import torch
+
+    capi, _ = native
+    off, re, im = planes(rows, rows, [0, 1, -1, 33, -37], 17)
+    dt = torch.float64 if prec != 1 else torch.float32
+    if prec == 1:
+        re, im = re.astype(np.float32).astype(float), im.astype(np.float32).astype(float)
+    M = capi.Matrix.create(rows, rows, off, re, im, precision=prec)
+    bad = np.array([complex(np.nan, np.nan), complex(np.nan, 1), complex(2, np.nan), complex(np.inf, 1), complex(1, -np.inf), 1 + 1j])
+    rng = np.random.default_rng(8)
+    X = bad[np.repeat(np.minimum(rng.integers(0, 15, (k, rows // 23 + 1)), 5), 23, axis=1)[:, :rows]]
+    xr, xi = (torch.from_numpy(np.ascontiguousarray(v)).to("cuda", dt) for v in (X.real, X.imag))
+    yr, yi = torch.empty(k, rows, device="cuda", dtype=dt), torch.empty(k, rows, device="cuda", dtype=dt)
+    capi.check(capi.lib().diaq_spmm(M.h, k, xr.data_ptr(), xi.data_ptr(), rows, yr.data_ptr(), yi.data_ptr(), rows, None))
+    for got, w in zip((yr, yi), full_product(rows, rows, off, re, im, X)):
+        got = got.double().cpu().numpy()
+        assert np.array_equal(np.isnan(got), np.isnan(w))
+        assert np.array_equal(got[np.isinf(w)], w[np.isinf(w)])
+        ok = np.isfinite(w)
+        assert ok.any() and maxrel(got[ok], w[ok]) < (1e-13 if prec == 0 else 1e-5)
+
+
 def _evolve(capi, H, N, X, mode, cfg):
     import torch
 
