@@ -36,8 +36,8 @@ METRIC = "expm(-iHt)·ψ states·steps/s"
 # ncu captures (profiles/), keyed by (qubits, states, form, states per block, rows per thread,
 # variant): for variant 12 the mean over the 12 launches of one time step (first, middle and last
 # terms, as roofline.achieved averages them); for variant 9 one middle term.  The kernels skip
-# all-zero 32-row tiles.
-TRAFFIC_PER_LAUNCH = {(20, 8, "horner", 4, 1, 9): 390.6e6, (20, 8, "horner", 4, 1, 12): 378.3e6}
+# all-zero 32-row tiles.  Variant 12: the real plane alone (the chain holds nothing else).
+TRAFFIC_PER_LAUNCH = {(20, 8, "horner", 4, 1, 9): 390.6e6, (20, 8, "horner", 4, 1, 12): 293.5e6}
 
 
 def peaks():
@@ -308,7 +308,8 @@ def run_spmv_only(args):
     psi = ham.random_state(N, 0)
     sp = torch.cuda.current_stream().cuda_stream
     live = tile_live_values(N, off, re, im)
-    out = {"stored_values": int(re.size), "live_tile_values": live}
+    planes = value_planes(im)
+    out = {"stored_values": int(re.size), "live_tile_values": live, "value_planes": planes}
     for name, M, dt, fn in (("c128", H, torch.float64, L.diaq_spmv_z), ("c64", Hc, torch.float32, L.diaq_spmv_c),
                             ("c128f2", Hf, torch.float64, L.diaq_spmv_z)):
         xr = torch.from_numpy(psi.real.copy()).to("cuda", dt)
@@ -325,12 +326,12 @@ def run_spmv_only(args):
         us = 1e3 * _timed(torch.cuda.current_stream(), loop) / args.spmv_reps
         # algorithmic bytes: the values of the live tiles (the kernels skip the all-zero ones), x, y
         w = 8 if name == "c64" else 16
-        by = w * live + 2 * w * N
+        by = w // 2 * planes * live + 2 * w * N
         peak, _ = peaks()
         out[name] = {"us": us, "gbs": by / us / 1e3, "frac": by / us / 1e3 / peak, "bytes": by,
                      "effective_gbs": (w * int(re.size) + 2 * w * N) / us / 1e3}
         if name == "c128":
-            out[name]["dfma_per_s"] = 4 * live / (us * 1e-6)
+            out[name]["dfma_per_s"] = 2 * planes * live / (us * 1e-6)
         if name == "c128f2":   # error of the float-pair product against the float64 one
             y64r, y64i = torch.empty_like(xr), torch.empty_like(xi)
             capi.check(L.diaq_spmv_z(H.h, xr.data_ptr(), xi.data_ptr(), y64r.data_ptr(), y64i.data_ptr(), sp))
@@ -509,6 +510,7 @@ def _ops_xxz(args, out, L, peak, peak_kind, dfma_peak, cpu, gpu_wall, cpu_wall):
     H = capi.Matrix.create(N, N, off, re, im)
     res, macs = _spgemm_counts(N, [int(d) for d in off], [int(d) for d in off])
     live_macs = _live_macs(N, off, re, im)
+    dfma = value_planes(im) ** 2 * live_macs
     offs = np.empty(len(off) * len(off), dtype=np.int32)
     cnt = ctypes.c_int32()
 
@@ -554,10 +556,10 @@ def _ops_xxz(args, out, L, peak, peak_kind, dfma_peak, cpu, gpu_wall, cpu_wall):
                        "complex_macs": int(macs), "complex_macs_live_tiles": int(live_macs),
                        "algorithmic_bytes": int(algo_bytes),
                        "gbs": algo_bytes / t_full / 1e9, "frac_hbm": algo_bytes / t_full / 1e9 / peak,
-                       "dfma_per_s": 4 * live_macs / t_full, "frac_fp64": 4 * live_macs / t_full / dfma_peak,
+                       "dfma_per_s": dfma / t_full, "frac_fp64": dfma / t_full / dfma_peak,
                        "note": "includes the device allocation and zeroing of C and the dry-run; products "
                                "with a factor in an all-zero 32-row tile are skipped, so the FP64 rate counts "
-                               "complex_macs_live_tiles (4 DFMA each); parity: the pruned product's offsets "
+                               "complex_macs_live_tiles (1 DFMA each: the chain is real); parity: the pruned product's offsets "
                                "and Frobenius norm against the CPU product"}}
     out["peak_hbm_gbs"] = peak
     out["peak_kind"] = peak_kind
@@ -845,6 +847,13 @@ def run_batched(args):
         print(json.dumps(out), flush=True)
 
 
+def value_planes(im):
+    """Planes of a matrix that the kernels read: the real one alone where no imaginary part is stored
+    (the float32 term kernels and the float-pair SpMV decide per matrix, the float64 kernels per tile;
+    the chains measured here are real throughout)."""
+    return 2 if np.any(im) else 1
+
+
 def tile_live_values(N, off, re, im):
     """Stored values of a square DiaQ matrix (packed re/im) that lie in 32-row tiles holding a
     nonzero -- what the term kernels read; they skip the all-zero tiles of every diagonal."""
@@ -934,8 +943,9 @@ def measure_precision(n: int = 24, states: int = 8, ref_states: int = 2, peak: f
                        "rel_err_max": float(err.max()), "fidelity_min": float(fid.min()),
                        "norm_drift_max": float(drift.max()), "launches_per_step": lps}
         if name == "horner":
-            # bytes of one step: the live c64 matrix once per launch, (24 m + 16) N per state and sub-step
-            step_bytes = (1 << s_c) * m_c * 8 * live + S * (1 << s_c) * (24 * m_c + 16) * N
+            # bytes of one step: the live c64 matrix once per launch (its real plane: the chain holds
+            # nothing else), (24 m + 16) N per state and sub-step
+            step_bytes = (1 << s_c) * m_c * 4 * live + S * (1 << s_c) * (24 * m_c + 16) * N
             ach = step_bytes / (ms / steps * 1e-3) / 1e9
             forms[name]["roofline"] = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                                        "frac": ach / peak, "bytes_per_step": step_bytes,
@@ -1099,15 +1109,16 @@ def run_ours(args, rank, world):
 
     peak, peak_kind = peaks()
     # algorithmic bytes of one chosen time step.  Every Taylor term is one launch over all S
-    # states and reads the c64 matrix once (8 B per stored value) -- the values of the 32-row
-    # tiles that hold a nonzero, the only ones the term kernels visit.  Per state, Horner form: the
-    # first term reads fp32(psi) (8N; its window and its epilogue read the same vector) and writes
+    # states and reads the c64 matrix once (4 B per stored value and plane that holds anything) -- the
+    # values of the 32-row tiles that hold a nonzero, the only ones the term kernels visit.  Per state,
+    # Horner form: the first term reads fp32(psi) (8N; its window and its epilogue read the same vector) and writes
     # w (8N); a middle term reads w and fp32(psi) and writes the next w (24N); the last reads w,
     # read-modify-writes psi in float64 and writes fp32(psi) (8N + 32N + 8N) -- (24 m + 16) N per
     # sub-step for m >= 2.
     per_state_step = (1 << s_c) * (24 * m_c + 16) * N
     live = tile_live_values(N, off, re, im)
-    step_bytes = (1 << s_c) * m_c * 8 * live + S * per_state_step
+    planes = value_planes(im)
+    step_bytes = (1 << s_c) * m_c * 4 * planes * live + S * per_state_step
     achieved = step_bytes / (ms / K * 1e-3) / 1e9
     k_launch, v_launch = chosen.config()
     variant = chosen.pipelined()
@@ -1116,7 +1127,7 @@ def run_ours(args, rank, world):
                 8: "dia_spmv_il_kernel<EpiHornerT<0/1>,8,4>", 9: "dia_spmv_il_kernel<EpiHornerT<0/1>,0,8>",
                 10: "dia_spmv_tma_kernel<EpiHornerT<0/1>,8,true,4>",
                 11: "dia_spmv_tma_kernel<EpiHornerT<0/1>,8,false,8>",
-                12: "dia_spmv_il32_kernel<EpiHornerT<0/1>,8,5>"}
+                12: f"dia_spmv_il32_kernel<EpiHornerT<0/1>,8,5,{'real' if planes == 1 else 'complex'}>"}
     kernel = (il_names.get(variant) if variant >= 6 else
               f"dia_spmv_kernel<float,{k_launch},{v_launch},EpiHornerP<0/1>>" if variant == 0 else
               f"variant {variant}, {k_launch} states x {v_launch} rows per thread")
@@ -1130,7 +1141,7 @@ def run_ours(args, rank, world):
         "ms_per_step": ms / K, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
         "dtype": "f32 terms + f64 state", "data": "synthetic (seeded XXZ couplings and states, built in-process)",
         "config": {"workload": f"xxz{args.n}_periodic_evolve", "form": "chosen", "evaluation": "horner", "n_qubits": args.n, "rows": N,
-                   "ndiag": len(off), "stored_values": total, "live_tile_values": live, "dt": DT,
+                   "ndiag": len(off), "stored_values": total, "live_tile_values": live, "value_planes": planes, "dt": DT,
                    "states_per_gpu": S,
                    "substeps": 1 << s_c, "taylor_terms": m_c, "selection": selection,
                    "launch_shape": {"states_per_block": chosen.config()[0], "rows_per_thread": chosen.config()[1],
@@ -1151,14 +1162,14 @@ def run_ours(args, rank, world):
                      "note": "achieved = algorithmic bytes per launch / mean launch time (CUDA events over the "
                              "timed steps; every launch of a step is this kernel: its middle-term and its "
                              "last-term instantiation)"},
-        "spmv_c128": {"us": spmv_us, "gbs": (16 * live + 32 * N) / spmv_us / 1e3,
-                      "frac": (16 * live + 32 * N) / spmv_us / 1e3 / peak,
-                      "dfma_per_launch": 4 * live, "reps": args.spmv_reps,
+        "spmv_c128": {"us": spmv_us, "gbs": (8 * planes * live + 32 * N) / spmv_us / 1e3,
+                      "frac": (8 * planes * live + 32 * N) / spmv_us / 1e3 / peak,
+                      "dfma_per_launch": 2 * planes * live, "reps": args.spmv_reps,
                       "effective_gbs": (16 * total + 32 * N) / spmv_us / 1e3,
-                      "note": "gbs, frac: bytes of the live 32-row tiles (all-zero tiles skipped); effective_gbs: "
+                      "note": "gbs, frac: bytes of the live 32-row tiles (all-zero tiles and planes skipped); effective_gbs: "
                               "all stored values (w Σlen + 2 w N) per time, the dense-diagonal figure"},
-        "spmv_c128f2": {"us": spmv_f2_us, "gbs": (16 * live + 32 * N) / spmv_f2_us / 1e3,
-                        "frac": (16 * live + 32 * N) / spmv_f2_us / 1e3 / peak,
+        "spmv_c128f2": {"us": spmv_f2_us, "gbs": (8 * planes * live + 32 * N) / spmv_f2_us / 1e3,
+                        "frac": (8 * planes * live + 32 * N) / spmv_f2_us / 1e3 / peak,
                         "effective_gbs": (16 * total + 32 * N) / spmv_f2_us / 1e3,
                         "maxrel_vs_c128": f2_err, "reps": args.spmv_reps,
                         "note": "same matrix as float pairs (DIAQ_C128F2), float64 vectors; includes the split of x"},
