@@ -332,6 +332,127 @@ __global__ void __launch_bounds__(kSpmvThreads)
     if (r0 < rows) epi.template apply<T, K, V>(r0, rows, kq, accr, acci);
 }
 
+// dia_spmv_kernel for float32, several states and windows off the 16-byte boundaries: a thread's V rows
+// are 32 apart (row of lane l: strip + 32 v + l), so that a warp's loads are runs of 128 bytes whatever
+// the offset of the diagonal and the alignment of the vectors, and the tiles of its strip are live or
+// not for the whole warp.  With vectors of 4 rows an unaligned window falls apart into single loads 16
+// bytes apart.  The sums are those of dia_spmv_kernel, in its order.  250,007-row band, 37 diagonals, 5
+// states: 33.5 us against 39.9 (6 states of 300,000 rows, 30 diagonals: 31.1 against 41.5).  Bound by
+// latency: three states (64 registers, 4 blocks per SM) read the matrix fewer times than two and leave
+// a fuller last wave; two 37, four 51, five 61 us; 48 registers spill, 59.
+constexpr int kStripStates = 3, kStripRows = 4;
+template <int K, int V, class Epi>
+__global__ void __launch_bounds__(kSpmvThreads)
+    dia_spmv_strip_kernel(const DiagMeta *__restrict__ meta, int nd, const float *__restrict__ are,
+                          const float *__restrict__ aim, int64_t rows, const float *__restrict__ xr, const float *__restrict__ xi, int64_t ldx,
+                          int nrhs, int nchunk, const uint32_t *__restrict__ tmask, int64_t mw, Epi epi0) {
+    static_assert(!Epi::kChained, "waits for no predecessor");
+    __shared__ int4 sq[kMetaChunk];
+    __shared__ BaseIm sb[kMetaChunk];
+    const int chunk = (int)(blockIdx.x % (unsigned)nchunk);
+    const int64_t tile = blockIdx.x / (unsigned)nchunk;
+    const int q0 = chunk * K;
+    const int kq = min(K, nrhs - q0);
+    xr += q0 * ldx;
+    xi += q0 * ldx;
+    const Epi epi = epi0.shifted(q0);
+    const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+    const int64_t w0 = (tile * kSpmvThreads + warp * 32) * V;   // the warp's rows: w0 .. w0 + 32 V - 1
+    const int64_t mword = (tile * kSpmvThreads * V) >> 10;      // a block's rows lie in one mask word (V | 4)
+    const int shift = (int)(w0 >> 5) & 31;
+    const int64_t r0 = w0 + lane;
+    float accr[K][V], acci[K][V];
+
+    // the products of one diagonal with the tiles of `live`
+    auto mac = [&](auto im_c, const int4 &q, int64_t base, uint32_t live) {
+        constexpr bool IM = decltype(im_c)::value;
+        const bool full = w0 >= q.y && w0 + 32 * V <= q.z;
+        const float *pa = are + base + r0, *pb = aim + base + r0;
+        const int64_t c = r0 + q.x;
+        float a[V], b[V];
+        bool ok[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            ok[v] = ((live >> v) & 1u) && (full || (r0 + 32 * v >= q.y && r0 + 32 * v < q.z));
+            a[v] = ok[v] ? __ldcs(pa + 32 * v) : 0.f;
+            if constexpr (IM) b[v] = ok[v] ? __ldcs(pb + 32 * v) : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (k >= kq) break;
+            const float *px = xr + k * ldx + c, *py = xi + k * ldx + c;
+            float x[V], y[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                x[v] = ok[v] ? __ldg(px + 32 * v) : 0.f;
+                y[v] = ok[v] ? __ldg(py + 32 * v) : 0.f;
+            }
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                accr[k][v] = fma(a[v], x[v], accr[k][v]);
+                if constexpr (IM) accr[k][v] = fma(-b[v], y[v], accr[k][v]);
+                acci[k][v] = fma(a[v], y[v], acci[k][v]);
+                if constexpr (IM) acci[k][v] = fma(b[v], x[v], acci[k][v]);
+            }
+        }
+    };
+
+    for (int pass = 0;; ++pass) {  // a second pass, with both planes, for rows that are not finite
+#pragma unroll
+        for (int q = 0; q < K; ++q)
+#pragma unroll
+            for (int v = 0; v < V; ++v) accr[q][v] = acci[q][v] = 0.f;
+        for (int c0 = 0; c0 < nd; c0 += kMetaChunk) {
+            const int cn = min(kMetaChunk, nd - c0);
+            if (pass == 0 || nd > kMetaChunk) {
+                __syncthreads();
+                for (int i = threadIdx.x; i < cn; i += kSpmvThreads) {
+                    const DiagMeta m = meta[c0 + i];
+                    const int64_t w = (int64_t)(c0 + i) * mw + mword;
+                    const uint32_t wr = tmask ? tmask[nd * mw + w] : 0xffffffffu;
+                    const uint32_t wi = tmask ? tmask[2 * nd * mw + w] : 0xffffffffu;
+                    sq[i] = make_int4(m.off, (int)m.lo, (int)m.hi, (int)wr);
+                    sb[i] = BaseIm{m.base, wi, 0u};
+                }
+                __syncthreads();
+            }
+            if (w0 >= rows) continue;
+            for (int k = 0; k < cn; ++k) {
+                const int4 q = sq[k];
+                const BaseIm b = sb[k];
+                const uint32_t im = (b.im >> shift) & ((1u << V) - 1u);
+                const uint32_t live = (((uint32_t)q.w >> shift) & ((1u << V) - 1u)) | im;
+                if (w0 + 32 * V <= q.y || w0 >= q.z || !live) continue;
+                if (im || pass)
+                    mac(std::true_type{}, q, b.base, live);
+                else
+                    mac(std::false_type{}, q, b.base, live);
+            }
+        }
+        if (pass || !tmask) break;
+        uint32_t big = 0u, small = ~0u;
+#pragma unroll
+        for (int q = 0; q < K; ++q)
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                big = max(big, max(abs_hi(accr[q][v]), abs_hi(acci[q][v])));
+                small = min(small, min(abs_hi(accr[q][v]), abs_hi(acci[q][v])));
+            }
+        const bool again = unsettled<float>(big, small);
+        if (!(nd > kMetaChunk ? __syncthreads_or(again) : __any_sync(0xffffffffu, again))) break;
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        float sr[K][1], si[K][1];
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+            sr[q][0] = accr[q][v];
+            si[q][0] = acci[q][v];
+        }
+        if (r0 + 32 * v < rows) epi.template apply<float, K, 1>(r0 + 32 * v, rows, kq, sr, si);
+    }
+}
+
 // One row per thread in blocks of NT threads, for matrices of few rows.  With only a few warps per SM
 // nothing hides the chain of one diagonal after the other, so each warp finds the diagonals that hold
 // a nonzero in its 32 rows 32 at a time (one per lane, ballots for the two planes) and issues the loads
@@ -993,17 +1114,48 @@ int launch_dia_spmv_pf(const Matrix &A, const float *xr, const float *xi, int64_
 // band, where unaligned windows fall apart into single loads) and for few rows (the row kernel);
 // 16-byte vectors of 4 rows for float32 above that (35 us against 62 on the 20-qubit chain).  Two
 // states per block rather than eight: 38 against 79 us for 11 float32 states of 65,536 rows, 40 against
-// 46 for 5 of 250,007.
+// 46 for 5 of 250,007 (before dia_spmv_strip_kernel took the latter).
 template <typename T>
 SpmvCfg default_cfg(int64_t rows, int nrhs) {
     const int k = nrhs == 1 ? 1 : 2;
     const bool few = rows * ((nrhs + k - 1) / k) <= kRowKernelMax<T>;
     return SpmvCfg{k, sizeof(T) == 8 || few ? 1 : 4, 0};
 }
+
+// Whether dia_spmv_strip_kernel takes a product whose default is the kernel of two states and four rows:
+// it needs fewer passes over the matrix (3 states, or 5 and more); the two-state shape's blocks are more
+// than run at a time (four per SM), so that its last wave is mostly empty (33 diagonals: 200,001
+// rows, 5 states, 587 blocks 26 us against 29; 220,001 rows, 645 blocks, 34 against 27); and at least
+// half of the windows are not on 16-byte boundaries (18-qubit chain, 8 states: 41 us against 45).
+inline bool strips_pay(const Matrix &A, const float *xr, const float *xi, int64_t ldx, int nrhs) {
+    if ((nrhs + 2) / 3 >= (nrhs + 1) / 2) return false;
+    if (A.rows > 0x7fffffffll * 1024 / nrhs) return false;
+    if ((int64_t)spmv_blocks(A.rows, kStripRows) * ((nrhs + 1) / 2) <= 4 * (int64_t)num_sms()) return false;
+    if (ldx % 4 || ((reinterpret_cast<uintptr_t>(xr) | reinterpret_cast<uintptr_t>(xi)) & 15u)) return true;
+    int32_t odd = 0;
+    for (int32_t d : A.off) odd += (d & 3) != 0;
+    return 2 * (int64_t)odd >= A.nd;
+}
+
+template <class Epi>
+int launch_dia_spmv_strips(const Matrix &A, const float *xr, const float *xi, int64_t ldx, int nrhs, Epi epi,
+                           cudaStream_t s, const uint32_t *tmask) {
+    const int nchunk = (nrhs + kStripStates - 1) / kStripStates;
+    dia_spmv_strip_kernel<kStripStates, kStripRows, Epi>
+        <<<spmv_blocks(A.rows, kStripRows) * (unsigned)nchunk, kSpmvThreads, 0, s>>>(
+            A.d_meta, A.nd, (const float *)A.re, (const float *)A.im, A.rows, xr, xi, ldx, nrhs, nchunk, tmask,
+            tile_mask_words(A.rows), epi);
+    DQ_CUDA(cudaGetLastError());
+    return DIAQ_OK;
+}
+
 template <typename T, class Epi>
 int launch_dia_spmv_rhs(const Matrix &A, const T *xr, const T *xi, int64_t ldx, int nrhs, Epi epi,
                         cudaStream_t s, const uint32_t *tmask, bool chained = false) {
     const SpmvCfg cfg = default_cfg<T>(A.rows, nrhs);
+    if constexpr (sizeof(T) == 4 && !Epi::kChained)
+        if (cfg.vr == kStripRows && strips_pay(A, xr, xi, ldx, nrhs))
+            return launch_dia_spmv_strips(A, xr, xi, ldx, nrhs, epi, s, tmask);
     if constexpr (sizeof(T) == 4)
         return launch_dia_spmv_rhs_cfg<T, Epi, 4, 1>(A, xr, xi, ldx, nrhs, epi, s, cfg, tmask, chained);
     else

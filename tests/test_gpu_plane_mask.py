@@ -99,6 +99,18 @@ def test_larger_products_are_the_full_products(native, rows, cols, offs, prec, k
     test_products_are_the_full_products(native, rows, cols, offs, prec, k, special)
 
 
+@pytest.mark.parametrize("rows,cols,offs,k", [(208003, 208005, [0, 1, -1, 36, -37, 701, -207990, 208000], 5),
+                                              (312007, 312001, [0, 3, -66, 1022], 3),
+                                              (125004, 125004, [1, -3, 30, -1025, 2048], 9),
+                                              (208005, 208011, MANY, 5)])
+@pytest.mark.parametrize("special", [False, True])
+def test_strip_products_are_the_full_products(native, rows, cols, offs, k, special):
+    """3, 5 and 9 complex64 states at sizes where strips of 128 rows and 3 states take over: rows and
+    columns off the tile sizes, diagonals of a few rows, more than one chunk of metadata, an incomplete
+    chunk of states, aligned vectors with unaligned offsets."""
+    test_products_are_the_full_products(native, rows, cols, offs, 1, k, special)
+
+
 @pytest.mark.parametrize("rows", [70, 9001, 70003, 270011])
 @pytest.mark.parametrize("prec,k", [(0, 1), (0, 3), (1, 1)])
 def test_products_of_nan_vectors(native, rows, prec, k):
