@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(kSpmvThreads)
 
         T accr[K][VR], acci[K][VR];
         const T *are = (const T *)I.are, *aim = (const T *)I.aim;
+        if (CHAINED && I.nd == 0) dependency_wait();   // (the others wait once their metadata is staged)
         // float64, no imaginary part in the matrix: half the loads and multiply-adds (one chunk of
         // metadata only), and rows that are not finite once more in full (20 chains of 10-14 qubits:
         // 2,546 -> 1,609 us for 2 steps; float32, bound by latency here, lost 5 %)
