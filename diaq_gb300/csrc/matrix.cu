@@ -280,11 +280,18 @@ void release(Matrix &M) {
         if (M.im) cudaFreeAsync(M.im, M.stream);
         if (M.d_meta) cudaFreeAsync(M.d_meta, M.stream);
     } else if (M.nd > 0) {
+        // The planes go back only after a wait that succeeded: given back without one, the next
+        // allocation could take them from under kernels still queued.  A cudaFree that is refused
+        // (while a stream is being captured in global mode) has waited for nothing; the planes then
+        // stay allocated, as the block itself does.
         // (a matrix whose allocation failed half-way was used by nothing but its own stream's fills)
-        if (M.d_meta) cudaFree(M.d_meta);
-        else cudaStreamSynchronize(M.stream);
-        pool_free_idle(M.re, M.device);
-        pool_free_idle(M.im, M.device);
+        const cudaError_t e = M.d_meta ? cudaFree(M.d_meta) : cudaStreamSynchronize(M.stream);
+        if (e == cudaSuccess) {
+            pool_free_idle(M.re, M.device);
+            pool_free_idle(M.im, M.device);
+        } else {
+            cudaGetLastError();   // not the next launch's
+        }
     } else {
         cudaFree(M.re);
         cudaFree(M.im);
