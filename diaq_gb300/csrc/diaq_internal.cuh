@@ -90,11 +90,16 @@ int cuda_status(cudaError_t e, const char *what, const char *file, int line);
 //
 // dev_malloc_async takes memory from the library's own pool on the current device (freed with
 // cudaFreeAsync): mapping and unmapping device memory takes about a millisecond per GB, and every
-// cudaMalloc and cudaFree synchronises.  The pool keeps at most kPoolKeep bytes of freed memory, gives
-// them back when the last matrix on the device goes or when an allocation fails (alloc_failed), and is
-// the driver's stream-ordered allocator: safe for any number of threads and streams.  H H of the
-// 18-qubit chain (2.4 GB): 3.9 -> 1.7 ms; exp(-i t H) of a 10-qubit chain: 33.0 -> 20.3 ms.
+// cudaMalloc and cudaFree synchronises.  The pool is the driver's stream-ordered allocator, safe for any
+// number of threads and streams; large value arrays of matrices are kept beside it (array_malloc in
+// matrix.cu).  Together they keep at most kPoolKeep bytes of freed memory, and give them back when the
+// last matrix on the device goes (all but kPoolRest) or when an allocation fails (alloc_failed).
+// H H of the 18-qubit chain (2.4 GB): 3.9 -> 1.7 ms; exp(-i t H) of a 10-qubit chain: 33.0 -> 20.3 ms.
 constexpr uint64_t kPoolKeep = 4ull << 30;
+constexpr uint64_t kBlockKeep = 3ull << 30;    // of it, value arrays kept one by one
+constexpr size_t kBlockMin = 32u << 20;        // a value array from this size on is
+constexpr size_t kBlockGrain = 2u << 20;       // the granularity of the driver's mappings
+constexpr uint64_t kPoolRest = 16u << 20;
 size_t alloc_limit();
 cudaError_t pool_malloc(void **p, size_t bytes, cudaStream_t s);
 // Frees a pool allocation no work on the device uses any more.
