@@ -16,6 +16,7 @@
 // much as the entries inside when offsets spread over the whole range: 65,536 x 16, 33 diagonals, complex
 // 224 us that way, 123 now (97 % of the FP64 rate); real 63.5 and 37.9.
 #include <algorithm>
+#include <type_traits>
 
 #include "diaq_internal.cuh"
 
@@ -42,7 +43,14 @@ struct Cplx {
     }
 };
 
-template <class T>
+// I: the type of element, row and column numbers: with few diagonals the division by n_right and the
+// shuffles are most of a warp's instructions.  And a grid-stride loop over some waves of blocks, as
+// starting a block per 256 elements costs as much there.  10^6 x 64 complex elements, 1, 2 and 3
+// diagonals: 700, 1,086 and 1,448 us with 64-bit numbers and a block per 256 elements, 539, 891 and 1,282 this way (every
+// diagonal visited, no ballots: 554, 917, 1,329); real, 3 diagonals 706, 617 (885).  Blocks per SM: 64, which
+// holds 100,000 x 20 in one wave of the loop (8 diagonals 61 us; 63 with 16); 16 for one or two diagonals
+// (3 10^6 x 1 complex, 2 diagonals 51.5 us; 55 with 64).
+template <class T, class I>
 __global__ void __launch_bounds__(kSpmmThreads)
     spmm_dia_kernel(const int64_t *__restrict__ offsets, int nd, const typename T::V *__restrict__ vals,
                     int64_t M, int64_t K, const typename T::V *__restrict__ B, int64_t R,
@@ -52,8 +60,8 @@ __global__ void __launch_bounds__(kSpmmThreads)
     const int64_t total = M * R;
     const int64_t stride = (int64_t)gridDim.x * kSpmmThreads;
     for (int64_t e0 = (int64_t)blockIdx.x * kSpmmThreads + (threadIdx.x - lane); e0 < total; e0 += stride) {
-        const int64_t e = e0 + lane, r = min(e, total - 1) / R;   // (lanes past the end load nothing)
-        const int64_t r0 = __shfl_sync(0xffffffffu, r, 0), r1 = __shfl_sync(0xffffffffu, r, 31);
+        const I e = (I)e0 + lane, r = min(e, (I)(total - 1)) / (I)R;   // (lanes past the end load nothing)
+        const I r0 = __shfl_sync(0xffffffffu, r, 0), r1 = __shfl_sync(0xffffffffu, r, 31);
         V acc = T::zero();
         for (int c0 = 0; c0 < nd; c0 += 32) {
             const int64_t own = c0 + lane < nd ? offsets[c0 + lane] : 0;
@@ -62,10 +70,10 @@ __global__ void __launch_bounds__(kSpmmThreads)
             auto load = [&](V &a, V &b) {
                 const int j = __ffs(live) - 1;
                 live &= live - 1u;
-                const int64_t o = __shfl_sync(0xffffffffu, own, j), c = r + o;
-                const bool ok = e < total && c >= 0 && c < K;
+                const I o = __shfl_sync(0xffffffffu, (I)own, j), c = r + o;   // (that of a live diagonal fits)
+                const bool ok = e < (I)total && c >= 0 && c < (I)K;
                 a = ok ? vals[(int64_t)(c0 + j) * M + r] : T::zero();
-                b = ok ? __ldg(B + e + o * R) : T::zero();
+                b = ok ? __ldg(B + e + (int64_t)o * R) : T::zero();
             };
             while (__popc(live) >= kUnroll) {
                 V a[kUnroll], b[kUnroll];
@@ -80,7 +88,7 @@ __global__ void __launch_bounds__(kSpmmThreads)
                 acc = T::mac(acc, a, b);
             }
         }
-        if (e < total) C[e] = acc;
+        if (e < (I)total) C[e] = acc;
     }
 }
 
@@ -100,14 +108,17 @@ extern "C" int diaq_spmm_dia_device(const int64_t *offsets, const void *vals, in
         return set_error(DIAQ_ERR_INVALID, "spmm_dia_device: NULL array");
     const int64_t total = n_rows * n_right;
     const int64_t want = (total + kSpmmThreads - 1) / kSpmmThreads;
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, 0x7fffffffll));
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, (n_diags <= 2 ? 16 : 64) * (int64_t)num_sms()));
     const cudaStream_t s = (cudaStream_t)stream;
-    if (is_complex)
-        spmm_dia_kernel<Cplx><<<grid, kSpmmThreads, 0, s>>>(offsets, n_diags, (const double2 *)vals, n_rows, n_cols,
-                                                            (const double2 *)B, n_right, (double2 *)C);
-    else
-        spmm_dia_kernel<Real><<<grid, kSpmmThreads, 0, s>>>(offsets, n_diags, (const double *)vals, n_rows, n_cols,
-                                                           (const double *)B, n_right, (double *)C);
+    auto go = [&](auto kernel, auto *c) {
+        using V = std::remove_pointer_t<decltype(c)>;
+        kernel<<<grid, kSpmmThreads, 0, s>>>(offsets, n_diags, (const V *)vals, n_rows, n_cols, (const V *)B, n_right, c);
+    };
+    // 32 bits hold every element, row and column number, and a row plus the offset of a diagonal that
+    // reaches it
+    const bool narrow = total <= 0x7fffffffll && n_cols <= 0x7fffffffll - n_rows;
+    if (is_complex) narrow ? go(spmm_dia_kernel<Cplx, int>, (double2 *)C) : go(spmm_dia_kernel<Cplx, int64_t>, (double2 *)C);
+    else narrow ? go(spmm_dia_kernel<Real, int>, (double *)C) : go(spmm_dia_kernel<Real, int64_t>, (double *)C);
     DQ_CUDA(cudaGetLastError());
     return DIAQ_OK;
 }
