@@ -1040,10 +1040,12 @@ static std::string tune_key(const EvolvePlan &P, int sl, int m) {
     for (auto &ch : name)
         if (ch == '"' || ch == ' ') ch = '_';
     char buf[256];
-    // (v2: the kernels changed since the first keys were written; their times say nothing any more)
-    std::snprintf(buf, sizeof(buf), "%s|v2|%s|n=%lld|nd=%d|k=%d|s=%d|m=%d", name.c_str(),
+    // (v2: the kernels changed since the first keys were written; their times say nothing any more.  A
+    // matrix without an imaginary part has its own interleaved kernels, so it does not share a shape with a
+    // complex one of the same size; complex128 kernels decide by tile.)
+    std::snprintf(buf, sizeof(buf), "%s|v2|%s%s|n=%lld|nd=%d|k=%d|s=%d|m=%d", name.c_str(),
                   P.mode == DIAQ_EVOLVE_MIXED ? "mixed" : P.mode == DIAQ_EVOLVE_HORNER ? "horner" : "c128",
-                  (long long)P.n, P.H->nd, P.nrhs, sl, m);
+                  P.real ? "|real" : "", (long long)P.n, P.H->nd, P.nrhs, sl, m);
     return buf;
 }
 
