@@ -639,6 +639,10 @@ __global__ void __launch_bounds__(NT)
 // terms: 753 against 624), float32 gains further (5 states of a 13-qubit Pauli sum: 8.7 against 14.4).
 template <typename T>
 constexpr int64_t kSplitKernelMax = sizeof(T) == 8 ? 8192 : 32768;
+template <typename T>
+inline bool split_kernel_fits(int64_t rows, int nchunk) {
+    return rows * nchunk <= kSplitKernelMax<T>;
+}
 
 template <typename T, int K, int U, class Epi>
 __global__ void __launch_bounds__(128)
@@ -1016,7 +1020,7 @@ void launch_vr(int vr, const Matrix &A, const T *xr, const T *xi, int64_t ldx, i
         constexpr int NT = 64, U = K == 1 ? 4 : 2;
         const int64_t blocks = (A.rows + NT - 1) / NT * nchunk;
         if constexpr (Epi::kSplit) {
-            if (A.rows * nchunk <= kSplitKernelMax<T>) {
+            if (split_kernel_fits<T>(A.rows, nchunk)) {
                 launch_chained(chained, dia_spmv_split_kernel<T, K, U, Epi>, (unsigned)((A.rows + 31) / 32 * nchunk), 128, s,
                                A.d_meta, A.nd, (const T *)A.re, (const T *)A.im, (int)A.rows, xr, xi, ldx, nrhs, nchunk,
                                tmask, tile_mask_words(A.rows), e);

@@ -43,3 +43,24 @@ def test_real_and_complex_matrices_are_tuned_apart(native, mode, tmp_path, monke
         assert set(json.loads(f.read_text())) == both
         seen.append(both)
     assert seen[0] == seen[1]
+
+
+SHAPES = [(8, 1, 0), (8, 2, 0), (4, 2, 0), (2, 2, 0), (1, 2, 0), (2, 1, 0), (1, 1, 0)]
+
+
+@pytest.mark.parametrize("n,k", [(6, 3), (10, 8), (12, 2), (12, 4), (13, 2), (12, 5), (13, 3), (14, 2), (12, 9)])
+def test_complex128_results_do_not_depend_on_what_was_timed(native, n, k, tmp_path, monkeypatch):
+    """Whatever shape another process's timing left in the file, the evolved states are the same bits: on
+    both sides of the line up to which four warps share a row's diagonals (8,192 rows x state pairs)."""
+    capi, _ = native
+    N, off, re, im = ham.xxz(n)
+    H = capi.Matrix.create(N, N, off, re, 0.3 * re)
+    P = ham.random_state(N, n, k=k)
+    f = tmp_path / "tune.json"
+    monkeypatch.setenv("DIAQ_AUTOTUNE_CACHE", str(f))
+    want = _run(capi, H, P, capi.EVOLVE_C128)
+    keys = list(json.loads(f.read_text())) if f.exists() else []
+    for shape in SHAPES:
+        if keys:
+            f.write_text(json.dumps({key: list(shape) for key in keys}))
+        assert np.array_equal(_run(capi, H, P, capi.EVOLVE_C128), want), shape
