@@ -309,7 +309,8 @@ int diaq_evolve_set_wait_limit(diaq_evolve_t E, int64_t wait_ns);
  * 0 states = choose automatically: on the first run the autotuner times the candidate shapes on
  * two steps of scratch copies of the states and keeps the fastest, caching the choice in a JSON
  * file (DIAQ_AUTOTUNE_CACHE, else $HOME/.cache/diaq_gb300/autotune.json).  The candidates' results
- * agree bit for bit.  Shapes of 1 or 2 states and 1 row per thread that a caller sets add in another order in complex128 plans
+ * agree bit for bit; a complex128 plan of one state has one candidate, which is not timed.  Shapes
+ * of 1 or 2 states and 1 row per thread that a caller sets add in another order in complex128 plans
  * of up to 8192 rows x state groups, as the automatic choice does there.  Setting a shape drops
  * the recorded graphs.  pipelined may be NULL in diaq_evolve_config. */
 int diaq_evolve_set_config(diaq_evolve_t E, int states_per_block, int rows_per_thread, int pipelined);

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from diaq_gb300 import hamiltonians as ham
+from oracle import oracle as orc
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +65,25 @@ def test_complex128_results_do_not_depend_on_what_was_timed(native, n, k, tmp_pa
         if keys:
             f.write_text(json.dumps({key: list(shape) for key in keys}))
         assert np.array_equal(_run(capi, H, P, capi.EVOLVE_C128), want), shape
+
+
+@pytest.mark.parametrize("n", [6, 12, 15])
+def test_one_complex128_state_is_not_tuned(native, n, tmp_path, monkeypatch):
+    """A plan of one state has one shape: its first run copies no states (it works with every further
+    allocation refused) and writes no file."""
+    capi, _ = native
+    import torch
+
+    f = tmp_path / "tune.json"
+    monkeypatch.setenv("DIAQ_AUTOTUNE_CACHE", str(f))
+    N, off, re, im = ham.tfim(n)
+    H = capi.Matrix.create(N, N, off, re, im)
+    E = capi.Evolve(H, 1, capi.EVOLVE_C128)
+    x = ham.random_state(N, 2)
+    pr, pi = (torch.from_numpy(np.ascontiguousarray(v)).cuda() for v in (x.real, x.imag))
+    monkeypatch.setenv("DIAQ_DEVICE_ALLOC_LIMIT", "1")
+    E.run(pr, pi, N, 0.05, 2, 0, 8)
+    torch.cuda.synchronize()
+    assert not f.exists()
+    want = orc.ham_sim(orc.OMatrix(N, N, off, re, im), x, 0.1, 2, 8)
+    assert np.linalg.norm((pr + 1j * pi).cpu().numpy() - want) / np.linalg.norm(want) < 1e-12
