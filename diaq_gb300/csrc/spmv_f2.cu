@@ -308,10 +308,20 @@ __device__ __forceinline__ void f2_mac_row(F2Row &s, float2 ah, float2 al, float
 // diagonals that hold a real or an imaginary nonzero in the warp's 32 rows, the loads of U of them are
 // issued together, and a plane that is zero there takes part in no product; a warp whose sums are not
 // finite sums again in full.  Against f2_spmv_kernel, split included: 12-qubit chain 12.3 us (24.3),
-// 16-qubit Pauli sum 25.9 (74.3), 250,007 rows of 37 diagonals 35.9 (54.4), 8 states of 100,001 rows 53.6
-// (61.7); from some 800,000 rows x states on the four rows per thread are the better form (20-qubit
-// chain 93.7 against 81.8).
-constexpr int64_t kF2RowKernelMax = 786432;   // rows x states of a launch
+// 16-qubit Pauli sum 25.9 (74.3), 250,007 rows of 37 diagonals 35.9 (54.4), 8 states of 100,001 rows 51.3
+// (57.7).  The lines, in rows x states of a launch: a matrix without an imaginary part costs the other
+// kernel half, so from some 360,000 on four rows per thread are the better form (16-qubit chain, 5
+// states, 327,680: 32.8 us against 34.9; 17 qubits, 3 states, 393,216: Ising 45.2 against 42.0, XXZ 36.9 and
+// 37.0; 524,288: 50 against 46) -- but where its blocks are a little more than run at a time (four per SM)
+// their last wave is mostly empty (655,360: Ising 69 against 73) -- a complex one from some 900,000 on
+// (Pauli sum, 786,432: 144 against 162; 917,504: 159 against 150; bands of 850,000 57 against 66, of
+// 1,040,000 68 against 71).
+constexpr int64_t kF2RowKernelMax = 900000, kF2RowKernelMaxReal = 360000;
+inline bool f2_row_kernel_pays(int64_t rows, int states, bool real) {
+    if (!real) return rows * states <= kF2RowKernelMax;
+    const int64_t blocks = spmv_blocks(rows, 4) * (int64_t)states, wave = 4 * (int64_t)num_sms();
+    return rows * states <= kF2RowKernelMaxReal || (blocks > wave && 5 * blocks < 6 * wave);
+}
 template <int U>
 __global__ void __launch_bounds__(64)
     f2_spmv_row_kernel(const DiagMeta *__restrict__ meta, int nd, const float *__restrict__ are,
@@ -463,6 +473,7 @@ int f2_spmv(const Matrix &A, int nrhs, const double *xr, const double *xi, int64
     const uint32_t *tmask = cached_tile_mask(A, s);
     const float *are = (const float *)A.re, *aim = (const float *)A.im;
     const int64_t mw = tile_mask_words(A.rows);
+    const bool real = tmask && A.real && A.nd <= kMetaChunk;
     for (int q = 0; q < nrhs; q += k) {
         const int kq = std::min(k, nrhs - q);
         const double *pr = xr + q * ldx, *pi = xi + q * ldx;
@@ -470,7 +481,7 @@ int f2_spmv(const Matrix &A, int nrhs, const double *xr, const double *xi, int64
         const dim3 g((unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8 * num_sms() / kq + 1)), (unsigned)kq);
         const int vec = ((uintptr_t)pr % 16 == 0) && ((uintptr_t)pi % 16 == 0) && (kq == 1 || ldx % 2 == 0);
         f2_split_pair_kernel<<<g, 256, 0, s>>>(pr, pi, n, ldx, vec, buf, np);
-        if (A.rows * kq <= kF2RowKernelMax) {
+        if (f2_row_kernel_pays(A.rows, kq, real)) {
             f2_spmv_row_kernel<4><<<dim3((unsigned)((A.rows + 63) / 64), (unsigned)kq), 64, 0, s>>>(
                 A.d_meta, A.nd, are, aim, A.capacity, (int)A.rows, buf, np, qr, qi, ldy, tmask, mw);
         } else {
@@ -480,7 +491,7 @@ int f2_spmv(const Matrix &A, int nrhs, const double *xr, const double *xi, int64
                 kernel<<<dim3(spmv_blocks(A.rows, 4), (unsigned)kq), kSpmvThreads, 0, s>>>(
                     A.d_meta, A.nd, are, aim, A.capacity, A.rows, buf, np, qr, qi, ldy, tmask, mw);
             };
-            if (tmask && A.real && A.nd <= kMetaChunk) go(f2_spmv_kernel<4, true>);
+            if (real) go(f2_spmv_kernel<4, true>);
             else go(f2_spmv_kernel<4, false>);
         }
     }
