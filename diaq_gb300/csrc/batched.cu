@@ -80,7 +80,11 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 
 // phase < 0: initialise v_a = T(psi) for every item.
 // CHAINED: launched with launch_chained; every block waits for its predecessor before it touches a
-// vector, and before it ends.
+// vector, and before it ends.  The blocks of the next phase come in as this one's end (2-15 % for
+// batches that fit the GPU at once: 8 chains of 10 qubits, 2 states, float32, 2 steps of 8 terms 175 us
+// unchained, 155 chained; complex128 210 and 198).  Letting them in earlier, after a block's last sums, took
+// that to 136 and 178 but 4 chains of 14 qubits in complex128 from 281 to 296 (compensated 330 to 388):
+// they wait where the working blocks need the registers.
 template <typename T, int K, int VR, bool CHAINED>
 __global__ void __launch_bounds__(kSpmvThreads)
     batched_phase_kernel(const BatchInst *__restrict__ insts, const BatchItem *__restrict__ items, int n_items,
@@ -496,7 +500,8 @@ static int build_items(Batch &B) {
 
 // Chained kernels (coherent state loads) are for batches that leave the GPU room, as in the plans: 3
 // chains of 8 qubits, 2 steps of 8 terms: 170 -> 142 us; 28 of 8-12 qubits: 222 -> 207; 24 of 10-17 qubits
-// (2,830 blocks a phase) would lose: 1,225 -> 1,321.
+// (2,830 blocks a phase) would lose: 1,225 -> 1,321.  (The interleaved kernels let their successor in
+// after the sums, the planar one as its blocks end.)
 static bool few_blocks(const Batch &B) { return B.n_items + B.n_il_items <= 8 * num_sms(); }
 
 template <typename T, int K, int VR>

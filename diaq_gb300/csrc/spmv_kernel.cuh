@@ -1,16 +1,18 @@
 // The diagonal-sparse SpMV kernel (y = A x for up to K right-hand sides at once), shared by the
 // plain SpMV entry points and the fused time-evolution terms, which differ only in the epilogue.
 //
-// Work split: thread t of block b owns the V consecutive rows r0 = (b*256 + t)*V .. r0+V-1
-// (V = 2 doubles or 4 floats = one 16-byte vector).  For every diagonal (metadata staged in
-// shared memory in chunks), the thread loads the V matrix values of its rows as one aligned
-// 16-byte vector per array (the row-phase aligned layout makes base + r0 a multiple of V), so a
-// warp streams 512 contiguous bytes per array per diagonal: fully coalesced.  x is read at
+// Work split: thread t of block b owns the V consecutive rows r0 = (b*256 + t)*V .. r0+V-1: by default
+// one row in float64, whose products are bound by FP64 issue, and 4 rows, one 16-byte vector, in float32
+// (default_cfg); the evolution plans' launch shapes choose among 1, 2 and 4.  For every diagonal
+// (metadata staged in shared memory in chunks), the thread loads the V matrix values of its rows as one
+// aligned vector per array (the row-phase aligned layout makes base + r0 a multiple of V), so a warp
+// streams 256 or 512 contiguous bytes per array per diagonal: fully coalesced.  x is read at
 // columns r0+d .. r0+d+V-1 -- as one vector when d is a multiple of V, else element by element --
 // through L1/L2, where the reuse across diagonals and neighbouring blocks lives (the state
 // vector of a 2^20-row problem is 16 MB, L2-resident on GB300).  Each row's sum runs over the
 // diagonals in slot order with fused multiply-adds; the epilogue functor gets the V sums per
-// right-hand side.
+// right-hand side.  Variants for few rows (dia_spmv_row_kernel, dia_spmv_split_kernel) and for several
+// float32 states off the 16-byte boundaries (dia_spmv_strip_kernel) follow it.
 #pragma once
 
 #include "diaq_internal.cuh"
@@ -637,6 +639,7 @@ __global__ void __launch_bounds__(NT)
 // the evolution under a 13-qubit one 972 against 1,348, under the 12-qubit Ising chain 580 against 612.  The
 // line (rows x state chunks): float64 is bound by FP64 issue from there on (14-qubit XXZ chain, 120
 // terms: 753 against 624), float32 gains further (5 states of a 13-qubit Pauli sum: 8.7 against 14.4).
+// The line goes by the call's rows and states alone, so the bits of a result do too.
 template <typename T>
 constexpr int64_t kSplitKernelMax = sizeof(T) == 8 ? 8192 : 32768;
 template <typename T>
@@ -1118,7 +1121,10 @@ int launch_dia_spmv_pf(const Matrix &A, const float *xr, const float *xi, int64_
 // band, where unaligned windows fall apart into single loads) and for few rows (the row kernel);
 // 16-byte vectors of 4 rows for float32 above that (35 us against 62 on the 20-qubit chain).  Two
 // states per block rather than eight: 38 against 79 us for 11 float32 states of 65,536 rows, 40 against
-// 46 for 5 of 250,007 (before dia_spmv_strip_kernel took the latter).
+// 46 for 5 of 250,007 (before dia_spmv_strip_kernel took the latter).  Where the matrix no longer fits in
+// L2 beside the chunks it holds as well: 1,000,001 rows of 41 complex diagonals, 8 / 32 states, 173 /
+// 817 us in float32 (eight states per block, before the choice of planes: 273 / 1,150), float64
+// 1,098 / 4,347 (1,158 / 4,543); 20-qubit chain, 16 states, float32 277 (358).
 template <typename T>
 SpmvCfg default_cfg(int64_t rows, int nrhs) {
     const int k = nrhs == 1 ? 1 : 2;

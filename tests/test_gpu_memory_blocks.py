@@ -80,3 +80,32 @@ def test_products_reuse_arrays_on_streams_of_their_own(native):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("n", [6, 14, 18])
+def test_destroying_a_matrix_waits_for_its_readers(native, n):
+    """The arrays of a caller's matrix are reused only because freeing the matrix waits for the work queued
+    on every stream: a product behind a sleeping stream has run when destroy returns."""
+    import torch
+
+    capi, _ = native
+    N, off, re, im = ham.tfim(n)
+    keep = capi.Matrix.create(64, 64, [0])
+    A = capi.Matrix.create(N, N, off, re, im)
+    x, y = torch.ones(2, N, device="cuda", dtype=torch.float64), torch.empty(2, N, device="cuda", dtype=torch.float64)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def product():
+        capi.check(capi.lib().diaq_spmv_z(A.h, x[0].data_ptr(), x[1].data_ptr(), y[0].data_ptr(), y[1].data_ptr(),
+                                          s.cuda_stream))
+
+    product()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(100_000_000)
+    product()
+    assert not s.query()
+    del A
+    assert s.query()
+    del keep
