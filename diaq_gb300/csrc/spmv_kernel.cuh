@@ -1116,18 +1116,32 @@ int launch_dia_spmv_pf(const Matrix &A, const float *xr, const float *xi, int64_
     return DIAQ_OK;
 }
 
-// The default shape, two states per block.  One row per thread for float64 (bound by FP64 issue or by
-// latency: 76 us against 83 with two rows on the 20-qubit chain, 43 against 53 on a 250,007-row
-// band, where unaligned windows fall apart into single loads) and for few rows (the row kernel);
-// 16-byte vectors of 4 rows for float32 above that (35 us against 62 on the 20-qubit chain).  Two
-// states per block rather than eight: 38 against 79 us for 11 float32 states of 65,536 rows, 40 against
-// 46 for 5 of 250,007 (before dia_spmv_strip_kernel took the latter).  Where the matrix no longer fits in
-// L2 beside the chunks it holds as well: 1,000,001 rows of 41 complex diagonals, 8 / 32 states, 173 /
-// 817 us in float32 (eight states per block, before the choice of planes: 273 / 1,150), float64
+// The default shape.  One row per thread for float64 (bound by FP64 issue or by latency: 76 us against
+// 83 with two rows on the 20-qubit chain, 43 against 53 on a 250,007-row band, where unaligned windows
+// fall apart into single loads) and for few rows (the row kernel); 16-byte vectors of 4 rows for float32
+// above that (35 us against 62 on the 20-qubit chain).
+//
+// Two states per block rather than eight: 38 against 79 us for 11 float32 states of 65,536 rows, 40
+// against 46 for 5 of 250,007 (before dia_spmv_strip_kernel took the latter).  Where the matrix no longer
+// fits in L2 beside the chunks it holds as well: 1,000,001 rows of 41 complex diagonals, 8 / 32 states,
+// 173 / 817 us in float32 (eight states per block, before the choice of planes: 273 / 1,150), float64
 // 1,098 / 4,347 (1,158 / 4,543); 20-qubit chain, 16 states, float32 277 (358).
+//
+// One state per block for an odd number of them in float64, where the last block's empty slot takes as
+// long as a state: 150,001-row band, 20 / 45 diagonals, 3 states 39 / 80 us against 51 / 102; 16-qubit
+// chain, 5 states 25.6 against 28.8.  Not where that takes the call past the line of a kernel for fewer
+// rows (12-qubit Pauli sum, 3 states, 10.9 against 8.4; 5 states of 20,001 rows 26.9 against 25.3) -- but
+// for 3 states at the second line (15-qubit Ising chain 12.9 against 16.9).
 template <typename T>
 SpmvCfg default_cfg(int64_t rows, int nrhs) {
-    const int k = nrhs == 1 ? 1 : 2;
+    int k = nrhs == 1 ? 1 : 2;
+    if (sizeof(T) == 8 && nrhs % 2) {
+        auto kernel = [&](int groups) {
+            return split_kernel_fits<T>(rows, groups) ? 0 : rows * groups <= kRowKernelMax<T> ? 1 : 2;
+        };
+        const int pairs = kernel((nrhs + 1) / 2);
+        if (pairs == kernel(nrhs) || (nrhs == 3 && pairs == 1)) k = 1;
+    }
     const bool few = rows * ((nrhs + k - 1) / k) <= kRowKernelMax<T>;
     return SpmvCfg{k, sizeof(T) == 8 || few ? 1 : 4, 0};
 }

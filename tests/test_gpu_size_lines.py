@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 # rows x groups of states at which kernels change: c128 8,192 and 65,536 (one or two states a group), c64
 # 32,768 and 262,144, float pairs 360,000 (no imaginary part; again from 622,592 to 747,110) and 900,000 rows x
 # states
-CASES = [("c128", 8192, 1), ("c128", 8193, 1), ("c128", 4096, 4), ("c128", 4097, 3), ("c128", 32768, 4), ("c128", 32769, 4),
+CASES = [("c128", 8192, 1), ("c128", 8193, 1), ("c128", 4096, 4), ("c128", 4097, 3), ("c128", 32768, 4), ("c128", 32769, 4), ("c128", 2730, 3), ("c128", 2731, 3), ("c128", 13107, 5), ("c128", 13108, 5),
+         ("c128", 21845, 5), ("c128", 21846, 5), ("c128", 32769, 3),
          ("c64", 32768, 2), ("c64", 32769, 2), ("c64", 16384, 3), ("c64", 16385, 4), ("c64", 131072, 3), ("c64", 131073, 3),
          ("c128f2", 120000, 3), ("c128f2", 120001, 3), ("c128f2", 218000, 3), ("c128f2", 250000, 3), ("c128f2", 300000, 3), ("c128f2", 300001, 3)]
 # sums of 9 complex products: 18 roundings of 2^-53 (2^-24, 2^-46) relative to sums of |a||x|
