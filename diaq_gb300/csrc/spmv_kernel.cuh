@@ -251,8 +251,16 @@ __device__ __forceinline__ void dia_mac(const int4 &q, int64_t base, int64_t r0,
 // b % nchunk of row tile b / nchunk: the blocks of one row tile are neighbours in launch order and
 // run at the same time, so the matrix tile they all read comes from HBM once and from L2 for the
 // other chunks -- the matrix traffic of one launch over all states, with the registers of K.
+//
+// Four float32 rows a thread with two and four states are held to the registers of four and three blocks
+// per SM.  Left alone, the choice of planes took the plans' instances past them (66-70 and 90
+// registers): two Horner steps of 24 terms on two 19-qubit Ising states 2,338 us, 1,441 with 58 registers;
+// 20 qubits 3,650 and 2,767.  The other shapes do best as the compiler has them.
+template <typename T, int K, int VR>
+constexpr int kSpmvMinBlocks = sizeof(T) == 4 && VR == 4 ? (K == 2 ? 4 : K == 4 ? 3 : 0) : 0;
+
 template <typename T, int K, int VR, class Epi>
-__global__ void __launch_bounds__(kSpmvThreads)
+__global__ void __launch_bounds__(kSpmvThreads, kSpmvMinBlocks<T, K, VR>)
     dia_spmv_kernel(const DiagMeta *__restrict__ meta, int nd, const T *__restrict__ are,
                     const T *__restrict__ aim, int64_t rows, const T *xr,
                     const T *xi, int64_t ldx, int nrhs, int nchunk, const uint32_t *__restrict__ tmask,
