@@ -96,7 +96,7 @@ int cuda_status(cudaError_t e, const char *what, const char *file, int line);
 // last matrix on the device goes (all but kPoolRest) or when an allocation fails (alloc_failed).
 // H H of the 18-qubit chain (2.4 GB): 3.9 -> 1.7 ms; exp(-i t H) of a 10-qubit chain: 33.0 -> 20.3 ms.
 constexpr uint64_t kPoolKeep = 4ull << 30;
-constexpr uint64_t kBlockKeep = 3ull << 30;    // of it, value arrays kept one by one
+constexpr uint64_t kBlockKeep = 3ull << 30;    // of it, at most, value arrays kept one by one
 constexpr size_t kBlockMin = 32u << 20;        // a value array from this size on is
 constexpr size_t kBlockGrain = 2u << 20;       // the granularity of the driver's mappings
 constexpr uint64_t kPoolRest = 16u << 20;

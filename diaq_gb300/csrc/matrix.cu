@@ -72,7 +72,7 @@ static cudaError_t pool_of(int dev, DevicePool **out) {   // g_pool_mu held, dev
     cudaMemPool_t pool = nullptr;
     cudaError_t e = cudaMemPoolCreate(&pool, &props);
     if (e != cudaSuccess) return e;
-    uint64_t keep = kPoolKeep - kBlockKeep;
+    uint64_t keep = kPoolKeep - P.block_bytes;
     e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e == cudaSuccess && !P.s) e = cudaStreamCreateWithFlags(&P.s, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
@@ -118,6 +118,13 @@ void pool_free_idle(void *p, int device) {
 // And cudaFree gives a kept array back at once, whatever still reads it.
 static size_t block_size(size_t bytes) { return (bytes + kBlockGrain - 1) / kBlockGrain * kBlockGrain; }
 
+// `by` bytes more kept as blocks (g_pool_mu held): the driver's pool may keep the rest of kPoolKeep.
+static void count_block(DevicePool &P, int64_t by) {
+    P.block_bytes += by;
+    uint64_t keep = kPoolKeep - P.block_bytes;
+    if (P.pool) cudaMemPoolSetAttribute(P.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
 static void free_blocks(std::vector<Block> &v) {
     for (const Block &b : v) {
         if (cudaFree(b.p) != cudaSuccess) cudaGetLastError();   // (refused during a capture: stays allocated)
@@ -139,7 +146,7 @@ static cudaError_t array_malloc(void **p, size_t bytes, int device, cudaStream_t
             if (P.blocks[i].bytes == size) {
                 got = P.blocks[i];
                 P.blocks.erase(P.blocks.begin() + i);
-                P.block_bytes -= size;
+                count_block(P, -(int64_t)size);
                 break;
             }
     }
@@ -179,13 +186,13 @@ static void array_free(void *p, size_t bytes, int device, cudaStream_t s, bool i
     if (keep) {
         std::lock_guard<std::mutex> lock(g_pool_mu);
         DevicePool &P = g_pools[device];
-        P.blocks.push_back(b);
-        P.block_bytes += b.bytes;
-        while (P.block_bytes > kBlockKeep) {
+        while (P.block_bytes + b.bytes > kBlockKeep) {
             out.push_back(P.blocks.front());
-            P.block_bytes -= P.blocks.front().bytes;
+            count_block(P, -(int64_t)P.blocks.front().bytes);
             P.blocks.erase(P.blocks.begin());
         }
+        P.blocks.push_back(b);
+        count_block(P, (int64_t)b.bytes);
     } else {
         out.push_back(b);
     }
@@ -201,7 +208,7 @@ bool alloc_failed(cudaError_t e) {
         for (auto &P : g_pools) {
             out.insert(out.end(), P.blocks.begin(), P.blocks.end());
             P.blocks.clear();
-            P.block_bytes = 0;
+            count_block(P, -(int64_t)P.block_bytes);
         }
     }
     bool any = !out.empty();
@@ -228,7 +235,7 @@ static void count_matrix(int device, int by) {
         P.matrices += by;
         if (P.matrices != 0) return;
         out.swap(P.blocks);
-        P.block_bytes = 0;
+        count_block(P, -(int64_t)P.block_bytes);
         uint64_t kept = 0;
         if (P.pool && cudaMemPoolGetAttribute(P.pool, cudaMemPoolAttrReservedMemCurrent, &kept) == cudaSuccess &&
             kept > kPoolRest) {

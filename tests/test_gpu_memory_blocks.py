@@ -109,3 +109,35 @@ def test_destroying_a_matrix_waits_for_its_readers(native, n):
     del A
     assert s.query()
     del keep
+
+
+BOUND = """
+import torch, numpy as np
+from diaq_gb300 import capi
+L = capi.lib()
+N, rows, cols, k = 1 << 20, 64, 1 << 26, 3
+keep = capi.Matrix.create(64, 64, [0])
+F = capi.Matrix.create(rows, cols, [0], np.ones(rows), np.ones(rows), precision=capi.C128F2)
+x, y = torch.ones(2, k, cols, device="cuda", dtype=torch.float64), torch.empty(2, k, rows, device="cuda", dtype=torch.float64)
+def product():   # 3 GiB of scratch
+    capi.check(L.diaq_spmm(F.h, k, x[0].data_ptr(), x[1].data_ptr(), cols, y[0].data_ptr(), y[1].data_ptr(), rows, None))
+    torch.cuda.synchronize()
+torch.cuda.synchronize()
+free0 = torch.cuda.mem_get_info()[0]
+kept = lambda: free0 - torch.cuda.mem_get_info()[0]
+slack = 96 << 20
+product()
+assert 3 << 30 <= kept() <= (4 << 30) + slack, kept()
+for _ in range(2):
+    big = capi.Matrix.create(N, N, list(range(180)))              # 2 x 1.4 GiB
+    del big
+    product()
+    assert kept() <= (4 << 30) + slack, kept()
+"""
+
+
+def test_kept_memory_is_bounded_together(native):
+    """What the driver's pool keeps of scratch and the arrays kept beside it stay below 4 GiB in all."""
+    r = subprocess.run([sys.executable, "-c", BOUND], cwd=ROOT, capture_output=True, text=True,
+                       env=dict(os.environ, PYTHONPATH=ROOT), timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
