@@ -50,6 +50,7 @@ struct Matrix {
     // library's memory pool and goes back in stream order.  publish() makes it a caller's matrix.
     bool internal = false;
     cudaStream_t stream = nullptr;         // internal: that stream
+    bool pooled = false;                   // the value arrays come from the driver's pool (see matrix.cu)
     // zero-tile mask of the values (see spmv_kernel.cuh), built on first use by the SpMV entry
     // points; every function that writes values into an existing matrix clears tmask_ok
     mutable uint32_t *tmask = nullptr;

@@ -112,8 +112,7 @@ void pool_free_idle(void *p, int device) {
 // per GB where cudaMalloc and cudaFree take 0.25 and 0.6, so whatever it had not kept cost more than with
 // plain allocations.  With cudaMalloc alone, with the pool alone, and this way: making and destroying a
 // 20-qubit chain, the only matrix, 0.9, 1.7 and 0.8 ms; chain, H H of 18 qubits and both destroyed 5.7, 7.6
-// and 4.9 ms; pruned H H of 20 qubits (12 GB) 32, 44 and 28 ms; unpruned 14.5, 8.3 (the pool goes beyond
-// its bound until something synchronises) and 10.9 ms; H H of 18 qubits again and again 4.2, 1.6 and
+// and 4.9 ms; pruned H H of 20 qubits (12 GB) 32, 44 and 28 ms; H H of 18 qubits again and again 4.2, 1.6 and
 // 1.6 ms.  Below kBlockMin the pool's cheap suballocation counts for more (small products and exponentials).
 // And cudaFree gives a kept array back at once, whatever still reads it.
 static size_t block_size(size_t bytes) { return (bytes + kBlockGrain - 1) / kBlockGrain * kBlockGrain; }
@@ -133,9 +132,18 @@ static void free_blocks(std::vector<Block> &v) {
     v.clear();
 }
 
+// Whether value arrays of this size come from the driver's pool.  result: those of a product that goes to
+// the caller as it is.  Programs make these again and again, and where they are too large to be kept here
+// the pool holds on to them until something synchronises (unpruned H H of 20 qubits, 11 GB: 8.4 ms a
+// product, 11.0 from cudaMalloc; the first one, with its matrix made and destroyed, 34 and 18).
+static bool array_pooled(size_t bytes, int device, bool result) {
+    if (bytes < kBlockMin || device < 0 || device >= kMaxDevices) return true;
+    return result && bytes > kBlockKeep / 2;   // (a matrix has two arrays)
+}
+
 // A value array on the current device; work on s may use it.
-static cudaError_t array_malloc(void **p, size_t bytes, int device, cudaStream_t s) {
-    if (bytes < kBlockMin || device < 0 || device >= kMaxDevices) return dev_malloc_async(p, bytes, s);
+static cudaError_t array_malloc(void **p, size_t bytes, int device, cudaStream_t s, bool pooled) {
+    if (pooled) return dev_malloc_async(p, bytes, s);
     if (bytes > alloc_limit()) return cudaErrorMemoryAllocation;
     const size_t size = block_size(bytes);
     Block got{nullptr, 0, nullptr};
@@ -168,16 +176,16 @@ static cudaError_t array_malloc(void **p, size_t bytes, int device, cudaStream_t
 }
 
 // Gives back a value array of the device.  idle: nothing uses it any more; else work on s may.
-static void array_free(void *p, size_t bytes, int device, cudaStream_t s, bool idle) {
+static void array_free(void *p, size_t bytes, int device, cudaStream_t s, bool idle, bool pooled) {
     if (!p) return;
-    if (bytes < kBlockMin || device < 0 || device >= kMaxDevices) {
+    if (pooled) {
         if (idle) pool_free_idle(p, device);
         else cudaFreeAsync(p, s);
         return;
     }
     Block b{p, block_size(bytes), nullptr};
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    bool keep = b.bytes <= kBlockKeep;
+    bool keep = b.bytes <= kBlockKeep / 2;
     if (keep && !idle)   // an event of a stream being captured marks no work
         keep = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
                cudaEventCreateWithFlags(&b.last, cudaEventDisableTiming) == cudaSuccess &&
@@ -330,8 +338,9 @@ int allocate(Matrix &M, cudaStream_t s, bool zero) {
         DQ_CUDA(dev_malloc(&M.re, bytes));
         DQ_CUDA(dev_malloc(&M.im, bytes));
     } else {
-        DQ_CUDA(array_malloc(&M.re, bytes, M.device, s));
-        DQ_CUDA(array_malloc(&M.im, bytes, M.device, s));
+        M.pooled = array_pooled(bytes, M.device, !zero && !M.internal);
+        DQ_CUDA(array_malloc(&M.re, bytes, M.device, s, M.pooled));
+        DQ_CUDA(array_malloc(&M.im, bytes, M.device, s, M.pooled));
     }
     if (zero) {
         DQ_CUDA(cudaMemsetAsync(M.re, 0, bytes, s));
@@ -384,8 +393,8 @@ int publish(Matrix &M) {
         M.d_meta = d;
         M.tmask = (uint32_t *)((uint8_t *)d + meta_bytes(M));
     } else {
-        array_free(M.re, (size_t)M.capacity * M.elem(), M.device, M.stream, false);
-        array_free(M.im, (size_t)M.capacity * M.elem(), M.device, M.stream, false);
+        array_free(M.re, (size_t)M.capacity * M.elem(), M.device, M.stream, false, M.pooled);
+        array_free(M.im, (size_t)M.capacity * M.elem(), M.device, M.stream, false, M.pooled);
         M.re = re;
         M.im = im;
     }
@@ -396,8 +405,8 @@ int publish(Matrix &M) {
 void release(Matrix &M) {
     const size_t bytes = (size_t)M.capacity * M.elem();
     if (M.internal) {
-        array_free(M.re, bytes, M.device, M.stream, false);
-        array_free(M.im, bytes, M.device, M.stream, false);
+        array_free(M.re, bytes, M.device, M.stream, false, M.pooled);
+        array_free(M.im, bytes, M.device, M.stream, false, M.pooled);
         if (M.d_meta) cudaFreeAsync(M.d_meta, M.stream);
     } else if (M.nd > 0) {
         // The planes go back only after a wait that succeeded: given back without one, the next
@@ -407,8 +416,8 @@ void release(Matrix &M) {
         // (a matrix whose allocation failed half-way was used by nothing but its own stream's fills)
         const cudaError_t e = M.d_meta ? cudaFree(M.d_meta) : cudaStreamSynchronize(M.stream);
         if (e == cudaSuccess) {
-            array_free(M.re, bytes, M.device, nullptr, true);
-            array_free(M.im, bytes, M.device, nullptr, true);
+            array_free(M.re, bytes, M.device, nullptr, true, M.pooled);
+            array_free(M.im, bytes, M.device, nullptr, true, M.pooled);
         } else {
             cudaGetLastError();   // not the next launch's
         }
